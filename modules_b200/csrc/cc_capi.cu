@@ -10,6 +10,7 @@
 #include "cc_internal.h"
 #include "cc_kernels.cuh"
 #include "cc_lbfgs.cuh"
+#include "cc_lines.cuh"
 #include "cc_multi_launch.h"
 #include "cc_nufft.cuh"
 #include "cc_plan.h"
@@ -90,20 +91,67 @@ int cci::get_splits(DevKSet &k, int want, const DevSplits **out)
 }
 
 
+// The plan's arrays (and the line plan's) go up in one copy into one allocation, followed by what the kernels write,
+// zeroed: slots without a mode are read (with weight 0) but never written on the line path, and the ticket starts at 0.
 int cci::upload_kset(DevKSet &k, const cc::Plan &plan)
 {
 	k.release();
 	k.plan = plan;
-	int rc;
+	k.lplan = cc::build_line_plan(plan);
+	const cc::LinePlan &L = k.lplan;
+	std::vector<unsigned char> up;
+	auto room = [](size_t bytes) { return (bytes + 255) / 256 * 256; };
+	auto put = [&](const void *p, size_t bytes) {
+		const size_t at = up.size();
+		up.resize(at + room(bytes));
+		if (bytes)
+			std::memcpy(up.data() + at, p, bytes);
+		return at;
+	};
+#define CC_PUT(v) put((v).data(), (v).size() * sizeof((v)[0]))
+	const size_t o_segs = CC_PUT(plan.segs), o_bstart = CC_PUT(plan.bstart), o_bspec = CC_PUT(plan.bspec),
+	             o_slotV = CC_PUT(plan.slotV), o_mode = CC_PUT(plan.mode_slot);
+	const size_t o_rows = CC_PUT(L.rows), o_lines = CC_PUT(L.lines), o_tlines = CC_PUT(L.tlines), o_cells = CC_PUT(L.cells),
+	             o_cellV = CC_PUT(L.cellV), o_groups = CC_PUT(L.groups), o_phases = CC_PUT(L.phases),
+	             o_tasks = CC_PUT(L.tasks);
+#undef CC_PUT
 	const size_t nslot = plan.slotV.size(), M = plan.mode_slot.size();
-	const size_t nred = (nslot + 31) / 32;
-	if ((rc = upload(&k.segs, plan.segs)) || (rc = upload(&k.rspec, plan.rspec)) || (rc = upload(&k.slotV, plan.slotV)) ||
-	    (rc = upload(&k.bstart, plan.bstart)) || (rc = upload(&k.bspec, plan.bspec)) ||
-	    (rc = upload(&k.mode_slot, plan.mode_slot)) || (rc = dev_alloc(&k.rho_slot, nslot)) ||
-	    (rc = dev_alloc(&k.u_slot, nslot)) || (rc = dev_alloc(&k.rho_mode, M)) || (rc = dev_alloc(&k.eblock, nred)) ||
-	    (rc = dev_alloc(&k.ticket, 1)))
+	const size_t nred = (nslot + 31) / 32, nlred = (size_t)L.nunit * (64 / cc::kLineRedCells);
+	size_t end = up.size();
+	auto take = [&](size_t bytes) {
+		const size_t at = end;
+		end += room(std::max<size_t>(bytes, 1));
+		return at;
+	};
+	const size_t o_ticket = take(sizeof(unsigned)), o_rho = take(nslot * sizeof(double2)),
+	             o_u = take(nslot * sizeof(double2)), o_rhom = take(M * sizeof(double2)), o_eb = take(nred * sizeof(double)),
+	             o_w = take((size_t)L.nunit * 8 * 32 * sizeof(double2)), o_leb = take(nlred * sizeof(double));
+	if (int rc = dev_alloc(&k.blob, end))
 		return rc;
-	CC_CUDA(cudaMemset(k.ticket, 0, sizeof(unsigned)));
+	if (!up.empty())
+		CC_CUDA(cudaMemcpy(k.blob, up.data(), up.size(), cudaMemcpyHostToDevice));
+	CC_CUDA(cudaMemset(k.blob + up.size(), 0, end - up.size()));
+	unsigned char *b = k.blob;
+	k.segs = reinterpret_cast<cc::Seg *>(b + o_segs);
+	k.bstart = reinterpret_cast<int *>(b + o_bstart);
+	k.bspec = reinterpret_cast<cc::TabSpec *>(b + o_bspec);
+	k.slotV = reinterpret_cast<double *>(b + o_slotV);
+	k.mode_slot = reinterpret_cast<int *>(b + o_mode);
+	k.ticket = reinterpret_cast<unsigned *>(b + o_ticket);
+	k.rho_slot = reinterpret_cast<double2 *>(b + o_rho);
+	k.u_slot = reinterpret_cast<double2 *>(b + o_u);
+	k.rho_mode = reinterpret_cast<double2 *>(b + o_rhom);
+	k.eblock = reinterpret_cast<double *>(b + o_eb);
+	k.line.rows = reinterpret_cast<cc::LineRow *>(b + o_rows);
+	k.line.lines = reinterpret_cast<cc::LineIdx *>(b + o_lines);
+	k.line.tlines = reinterpret_cast<cc::LineIdx *>(b + o_tlines);
+	k.line.cells = reinterpret_cast<cc::LineCell *>(b + o_cells);
+	k.line.cellV = reinterpret_cast<double2 *>(b + o_cellV);
+	k.line.groups = reinterpret_cast<cc::LineTabs *>(b + o_groups);
+	k.line.phases = reinterpret_cast<cc::LineTabs *>(b + o_phases);
+	k.line.tasks = reinterpret_cast<cc::LineTask *>(b + o_tasks);
+	k.line.weights = reinterpret_cast<double2 *>(b + o_w);
+	k.line.eblock = reinterpret_cast<double *>(b + o_leb);
 	return CC_OK;
 }
 
@@ -112,12 +160,6 @@ namespace {
 // ---------------------------------------------------------------------------------------------------------------
 // launch configuration
 // ---------------------------------------------------------------------------------------------------------------
-struct Launch {
-	int nsplit, per_split, csize, chunk;   // rho: particle splits (a multiple of the cluster size)
-	int want_force;                       // force: requested number of segment splits
-};
-
-
 // Record a timing event; inside a stream capture it must be an external record node to carry a timestamp.
 cudaError_t record_timing(cudaEvent_t e, cudaStream_t st)
 {
@@ -143,9 +185,78 @@ double grid_cost(int64_t blocks, int wave, double pairs, double fixed_pairs)
 	return (double)waves * (1.0 + pairs / (double)blocks / fixed_pairs);
 }
 
-Launch choose_launch(const cc::Plan &p, int64_t N, bool mixed)
+// The line kernels' grids (B200, CUDA graphs of evaluations, sweeps over 2D and 3D sets of N = 300 to 100000).
+// rho: particle splits (multiples of 8 particles) with the least estimated time: whole waves of blocks, a block's fixed cost
+// (loads, the tables' latency) and its matrix work at 70 % of the pipe, plus the partial rows, which cross L2 twice: 3D
+// N=2000 chi=0.45 takes 6.9 us with 84 splits of 24 particles, 7.9 with 125 of 16 and 8.0 with 42 of 48; 2D N=7001
+// chi=0.37 13.8 with 146 of 48 (one wave), 17.7 with 219 of 32.
+// force: tiles of 8 particles per block and warps per block, by whole waves of what one wave measured (3D, 67 units: 9.4,
+// 15.2, 20.6 and 28.7 us for 1 to 4 tiles with 8 warps, two blocks to an SM; 9.0, 11.8 and 16.8 for 2 to 4 tiles with 16).
+constexpr double kLineFixedUs = 1.5, kLinePipe = 0.7, kLineL2BytesPerUs = 3e6;
+
+Launch choose_line_launch(const cc::LinePlan &p, int d, int64_t N)
 {
-	Launch l;
+	Launch l = {};
+	l.line = true;
+	l.csize = 1;
+	const int sms = sm_count();
+	const int64_t G = std::max<int64_t>(1, (int64_t)p.groups.size());
+	const int per_sm = p.ntask <= cc::kLineTasks ? 2 : 1;
+	const double particle_us = p.group_cycles / (kLinePipe * 1965.0);
+	double best = 1e300;
+	l.nsplit = 1;
+	l.per_split = 8;
+	const int64_t maxns = std::max<int64_t>(1, std::min<int64_t>((N + 7) / 8, 4096));
+	for (int64_t ns = 1; ns <= maxns; ns++) {
+		const int64_t per = std::max<int64_t>(8, ((N + ns - 1) / ns + 7) / 8 * 8), real = std::max<int64_t>(1, (N + per - 1) / per);
+		const int64_t wave = (int64_t)per_sm * sms, full = G * real / wave, rest = G * real - full * wave;
+		const double us = (double)per * particle_us, last = rest == 0 ? 0.0 : rest <= sms ? us : per_sm * us;
+		const double c = (double)(full + (rest > 0)) * kLineFixedUs + (double)full * per_sm * us + last +
+		                 (double)real * (double)p.nunit * 4096.0 / kLineL2BytesPerUs;
+		if (c < best) {
+			best = c;
+			l.nsplit = (int)real;
+			l.per_split = (int)per;
+		}
+		if (G * real > 8LL * sms)
+			break;
+	}
+	// chunks: a power of two that holds a split, or as many particles as fit (and have a thread per coordinate)
+	const size_t row = (size_t)p.group_row * sizeof(double2);
+	const size_t room = (per_sm == 2 ? 100 : 204) * 1024;
+	const int most = std::min(cc::kLineMaxChunk, p.ntask * 32 / d);
+	l.chunk = 8;
+	while (l.chunk < l.per_split && 2 * l.chunk <= most && 2 * l.chunk * row <= room)
+		l.chunk *= 2;
+	// force
+	static const struct {
+		int mt, warps;
+		double unit_us;   // per unit and wave
+	} opt[] = {{1, 8, 0.117}, {2, 8, 0.205}, {3, 8, 0.285}, {4, 8, 0.406}, {2, 16, 0.112}, {3, 16, 0.154}, {4, 16, 0.228}};
+	best = 1e300;
+	l.mt = 1;
+	l.fwarps = 8;
+	for (const auto &o : opt) {
+		const double waves = (double)((N + 8 * o.mt - 1) / (8 * o.mt)) / ((o.warps == 8 ? 2.0 : 1.0) * sms);
+		// few waves: whole ones; many: the blocks of a new wave start as those of the last one end
+		const double c = (waves < 4.0 ? std::ceil(waves) : waves + 0.5) * (kLineFixedUs + o.unit_us * p.nunit);
+		if (c < best) {
+			best = c;
+			l.mt = o.mt;
+			l.fwarps = o.warps;
+		}
+	}
+	return l;
+}
+
+// FP64 evaluations take the line kernels where the k-set has a line plan; mixed precision and the other sets (1D, sparse
+// lines) the segment kernels.
+Launch find_launch(const DevKSet &k, int64_t N, bool mixed)
+{
+	const cc::Plan &p = k.plan;
+	if (!mixed && k.lplan.ok)
+		return choose_line_launch(k.lplan, p.d, N);
+	Launch l = {};
 	const size_t esz = mixed ? sizeof(float2) : sizeof(double2);
 	l.chunk = (int)std::max<size_t>(8, std::min<size_t>(64, kRhoTabBudget / (esz * std::max(1, p.block_max_row | 1))));
 	const double pairs = (double)std::max<int64_t>(N, 1) * (double)std::max<int64_t>(p.real_segs, 1) * p.L;
@@ -194,6 +305,19 @@ Launch choose_launch(const cc::Plan &p, int64_t N, bool mixed)
 			break;
 	}
 	return l;
+}
+
+// A k-set keeps its last few choices: a program evaluates few particle counts with one handle, and searching the grids
+// takes longer on the host than launching them.
+Launch choose_launch(const DevKSet &k, int64_t N, bool mixed)
+{
+	for (const DevKSet::Chosen &c : k.chosen)
+		if (c.N == N && c.mixed == mixed)
+			return c.l;
+	if (k.chosen.size() >= 8)
+		k.chosen.erase(k.chosen.begin());
+	k.chosen.push_back({N, mixed, find_launch(k, N, mixed)});
+	return k.chosen.back().l;
 }
 
 // ---------------------------------------------------------------------------------------------------------------
@@ -373,6 +497,43 @@ int launch_force(int d, const cc::ForceArgs &a, bool mixed, int64_t N, int row, 
 	}
 }
 
+constexpr int kLineSmemMax = 106 * 1024;   // two blocks per SM
+
+template <int D> int launch_line_rho_t(const cc::LineRhoArgs &a, int nsplit, size_t smem, cudaStream_t st)
+{
+	static cudaError_t e = cudaFuncSetAttribute(cc::cc_line_rho_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+	                                            2 * kLineSmemMax);
+	if (e)
+		return fail(CC_ERR_CUDA, std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e));
+	CC_CUDA(launch_pdl(cc::cc_line_rho_kernel<D>, dim3(a.ngroup, nsplit), dim3(32 * a.ntask), smem, st, a));
+	return CC_OK;
+}
+
+template <int D, int MT, int W> int launch_line_force_t(const cc::LineForceArgs &a, int row, cudaStream_t st)
+{
+	static cudaError_t e = cudaFuncSetAttribute(cc::cc_line_force_kernel<D, MT, W>,
+	                                            cudaFuncAttributeMaxDynamicSharedMemorySize, kLineSmemMax);
+	if (e)
+		return fail(CC_ERR_CUDA, std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e));
+	const unsigned blocks = (unsigned)((a.N + 8 * MT - 1) / (8 * MT)) + (a.E_out ? 1u : 0u);
+	CC_CUDA(launch_pdl(cc::cc_line_force_kernel<D, MT, W>, dim3(blocks), dim3(32 * W),
+	                   cc::line_force_smem(row, MT, W, D), st, a));
+	return CC_OK;
+}
+
+template <int D> int launch_line_force_d(const cc::LineForceArgs &a, int mt, int warps, int row, cudaStream_t st)
+{
+	switch (mt * 100 + warps) {
+	case 108: return launch_line_force_t<D, 1, 8>(a, row, st);
+	case 208: return launch_line_force_t<D, 2, 8>(a, row, st);
+	case 308: return launch_line_force_t<D, 3, 8>(a, row, st);
+	case 408: return launch_line_force_t<D, 4, 8>(a, row, st);
+	case 216: return launch_line_force_t<D, 2, 16>(a, row, st);
+	case 316: return launch_line_force_t<D, 3, 16>(a, row, st);
+	default: return launch_line_force_t<D, 4, 16>(a, row, st);
+	}
+}
+
 // force splits for `want`, uploaded once and cached on the k-set
 
 // ---------------------------------------------------------------------------------------------------------------
@@ -526,6 +687,62 @@ int run_rho(cc_handle *h, DevKSet &k, int64_t N, const double *d_frac, double *d
 		CC_CUDA(cudaGetLastError());
 		return CC_OK;
 	}
+	if (l.line) {
+		const int nsplit = N > 0 ? l.nsplit : 1;
+		const cc::LinePlan &L = k.lplan;
+		if (int rc = ensure_partial(k, (size_t)nsplit * L.nunit * 128))
+			return rc;
+		cc::LineRhoArgs a = {};
+		a.frac = d_frac;
+		a.N = (int)N;
+		a.per_split = N > 0 ? l.per_split : 0;
+		a.chunk = l.chunk;
+		a.log2chunk = __builtin_ctz((unsigned)l.chunk);
+		a.ngroup = (int)L.groups.size();
+		a.nunit = L.nunit;
+		a.ntask = L.ntask;
+		a.groups = k.line.groups;
+		a.tasks = k.line.tasks;
+		a.tlines = k.line.tlines;
+		a.partial = k.partial;
+		a.skip = h->d_skip;
+		a.frac_copy = (&k == &h->main) ? h->rho_copy : nullptr;
+		a.early = (h->early_call && &k == &h->main && !a.skip && !a.frac_copy) ? 1 : 0;
+		const size_t smem = cc::line_rho_smem(L.group_row, l.chunk, h->d);
+		if (int rc = h->d == 2 ? launch_line_rho_t<2>(a, nsplit, smem, st) : launch_line_rho_t<3>(a, nsplit, smem, st))
+			return rc;
+		if (after_rho)
+			CC_CUDA(record_timing(after_rho, st));
+		cc::LineReduceArgs r = {};
+		r.partial = k.partial;
+		r.nsplit = nsplit;
+		r.nunit = L.nunit;
+		r.cells = k.line.cells;
+		r.cellV = k.line.cellV;
+		r.rho_offset = h->rho_offset;
+		r.rho_slot = rho_out ? rho_out : k.rho_slot;
+		r.weights = rho_out ? nullptr : k.line.weights;
+		r.eblock = k.line.eblock;
+		r.ticket = k.ticket;
+		r.inv_vol = 1.0 / h->volume;
+		r.shift = h->shift;
+		r.E_out = d_E;
+		r.finalize = energy_in_force ? 0 : 1;
+		r.skip = h->d_skip;
+		if (!rho_out && h->d_cellS0 && &k == &h->main) {
+			r.cellS0 = h->d_cellS0;
+			r.npart = (double)N;
+			r.inv_vol = 1.0;
+		}
+		CC_CUDA(launch_pdl(cc::cc_line_reduce_kernel, dim3(L.nunit * (64 / cc::kLineRedCells)),
+		                   dim3(cc::kLineRedThreads), 0, st, r));
+		if (want_rho_mode && !p.mode_slot.empty()) {
+			const int M = (int)p.mode_slot.size();
+			cc::cc_gather_rho_kernel<<<(M + 255) / 256, 256, 0, st>>>(k.rho_slot, k.mode_slot, M, k.rho_mode);
+			CC_CUDA(cudaGetLastError());
+		}
+		return CC_OK;
+	}
 	const int nsplit = N > 0 ? l.nsplit : 1;
 	const int csize = N > 0 ? l.csize : 1;
 	const int rows = nsplit / csize;
@@ -597,6 +814,36 @@ int run_force(cc_handle *h, int64_t N, const double *d_frac, double *d_F, double
 		if (d_gfrac)
 			CC_CUDA(cudaMemsetAsync(d_gfrac, 0, sizeof(double) * N * h->d, st));
 		return CC_OK;
+	}
+	if (l.line) {
+		const cc::LinePlan &L = h->main.lplan;
+		const DevLines &k = h->main.line;
+		if (u_in) {
+			const int ncell = L.nunit * 64;
+			cc::cc_line_weights_kernel<<<(4 * ncell + 255) / 256, 256, 0, st>>>(k.cells, u_in, ncell, k.weights);
+			CC_CUDA(cudaGetLastError());
+		}
+		cc::LineForceArgs a = {};
+		a.frac = d_frac;
+		a.N = (int)N;
+		a.nphase = (int)L.phases.size();
+		a.phases = k.phases;
+		a.rows = k.rows;
+		a.lines = k.lines;
+		a.weights = k.weights;
+		for (int i = 0; i < 9; i++)
+			a.recip[i] = h->recip[i];
+		a.fscale = u_in ? fscale_in : h->d_slotS0 ? 4.0 / (double)N : 2.0 / h->volume;
+		a.F_out = d_F;
+		a.gfrac_out = d_gfrac;
+		a.eblock = k.eblock;
+		a.neblock = L.nunit * (64 / cc::kLineRedCells);
+		a.inv_vol = h->d_slotS0 ? 1.0 : 1.0 / h->volume;
+		a.shift = h->shift;
+		a.E_out = d_E;
+		a.skip = h->d_skip;
+		return h->d == 2 ? launch_line_force_d<2>(a, l.mt, l.fwarps, L.phase_row, st)
+		                 : launch_line_force_d<3>(a, l.mt, l.fwarps, L.phase_row, st);
 	}
 	const DevSplits *f = nullptr;
 	if (int rc = get_splits(h->main, l.want_force, &f))
@@ -1009,12 +1256,16 @@ int eval_multiconfig(cc_handle *h, int64_t N, const double *d_frac, double *d_E,
 	}
 	const size_t slab = (size_t)nsub * p.nslot;
 	const int nb = (p.nslot + cc::kS2mThreads - 1) / cc::kS2mThreads;
-	if (int rc = grow(&h->d_msub, h->msub_cap, 2 * slab))
-		return rc;
+	if (2 * slab > h->msub_cap) {
+		if (int rc = grow(&h->d_msub, h->msub_cap, 2 * slab))
+			return rc;
+		// slots without a mode are read (with weight 0) but not written on the line path
+		CC_CUDA(cudaMemsetAsync(h->d_msub, 0, 2 * slab * sizeof(double2), st));
+	}
 	if (int rc = grow(&h->d_mpart, h->mpart_cap, (size_t)nb + 1))
 		return rc;
 	double2 *rho = h->d_msub, *u = h->d_msub + slab;
-	const Launch l = choose_launch(p, Np, false);
+	const Launch l = choose_launch(k, Np, false);
 	double *copy = h->rho_copy;   // graph path: the rho passes store the positions for the force passes
 	for (int c = 0; c < nsub; c++) {
 		h->rho_copy = copy ? copy + (size_t)c * Np * d : nullptr;
@@ -1056,7 +1307,7 @@ int eval_device(cc_handle *h, int64_t N, const double *d_frac, double *d_E, doub
 		return eval_multiconfig(h, N, d_frac, d_E, d_F, d_gfrac, st);
 	}
 	const bool mixed = precision == CC_PREC_MIXED && !h->d_slotS0;   // the S2 form evaluates in FP64
-	const Launch l = choose_launch(h->main.plan, N, mixed);
+	const Launch l = choose_launch(h->main, N, mixed);
 	cudaEvent_t e0 = nullptr, e1 = nullptr, e2 = nullptr, e3 = nullptr;
 	if (h->timing && h->ev_used + 4 <= 4 * 100000) {
 		e0 = next_event(h);
@@ -1305,7 +1556,15 @@ int cc_create_s2(int d, const double *basis, int64_t M, const int32_t *modes, co
 		extra += vs02[q] - W * slotS0[q] * slotS0[q];
 	}
 	h->shift += extra;
-	if (int rc = upload(&h->d_slotS0, slotS0)) {
+	std::vector<double2> cellS0(h->main.lplan.cells.size(), make_double2(0.0, 0.0));
+	for (size_t c = 0; c < cellS0.size(); c++) {
+		const cc::LineCell &x = h->main.lplan.cells[c];
+		cellS0[c] = make_double2(x.sp >= 0 ? slotS0[(size_t)x.sp] : 0.0, x.sm >= 0 ? slotS0[(size_t)x.sm] : 0.0);
+	}
+	int rc = upload(&h->d_slotS0, slotS0);
+	if (!rc && h->main.lplan.ok)
+		rc = upload(&h->d_cellS0, cellS0);
+	if (rc) {
 		cc_destroy(h);
 		return rc;
 	}
@@ -1366,6 +1625,7 @@ int cc_destroy(cc_handle *h)
 	cudaFree(h->d_fcounters);
 	cudaFree(h->d_E);
 	cudaFree(h->d_slotS0);
+	cudaFree(h->d_cellS0);
 	cudaFree(h->d_msub);
 	cudaFree(h->d_mpart);
 	cudaFreeHost(h->h_pin);
@@ -1671,7 +1931,7 @@ int cc_rho(cc_handle *h, double *re, double *im, int precision)
 		if (int rc = run_nufft(h, N, h->d_frac, h->d_E, nullptr, nullptr, true, h->stream))
 			return rc;
 	} else {
-		const Launch l = choose_launch(h->main.plan, N, precision == CC_PREC_MIXED);
+		const Launch l = choose_launch(h->main, N, precision == CC_PREC_MIXED);
 		if (int rc = run_rho(h, h->main, N, h->d_frac, h->d_E, true, precision == CC_PREC_MIXED, l, h->stream))
 			return rc;
 	}
@@ -1736,7 +1996,7 @@ int cc_structure_factor(cc_handle *h, int64_t K, const int32_t *modes, double *S
 	}
 	if (int rc = flush_upload(h))
 		return rc;
-	const Launch l = choose_launch(h->sk.plan, N, precision == CC_PREC_MIXED);
+	const Launch l = choose_launch(h->sk, N, precision == CC_PREC_MIXED);
 	const double save_off = h->rho_offset;
 	h->rho_offset = 0.0;   // S(k) of the particles themselves (StructureFactor has no fixed-particle offset)
 	int rc = run_rho(h, h->sk, N, h->d_frac, h->d_E + 1, true, precision == CC_PREC_MIXED, l, h->stream);
@@ -1819,7 +2079,7 @@ int cc_mc_try_move(cc_handle *h, const double *s_prev, const double *s_after, do
 		// rho of the bound positions in mode order (FP64), as the cached RhoReal / RhoImag of the reference
 		if (int rc = flush_upload(h))
 			return rc;
-		const Launch l = choose_launch(h->main.plan, h->N, false);
+		const Launch l = choose_launch(h->main, h->N, false);
 		if (int rc = run_rho(h, h->main, h->N, h->d_frac, h->d_E, true, false, l, h->stream))
 			return rc;
 		CC_CUDA(cudaMemcpyAsync(h->d_rho_cur, h->main.rho_mode, sizeof(double2) * M, cudaMemcpyDeviceToDevice,
@@ -1924,7 +2184,7 @@ int cc_plan_info(const cc_handle *h, int64_t N, int *L, int64_t *nseg, int *nspl
 {
 	if (int rc = check_handle(h))
 		return rc;
-	const Launch l = choose_launch(h->main.plan, N, false);
+	const Launch l = choose_launch(h->main, N, false);
 	if (L)
 		*L = h->main.plan.L;
 	if (nseg)
@@ -1932,7 +2192,7 @@ int cc_plan_info(const cc_handle *h, int64_t N, int *L, int64_t *nseg, int *nspl
 	if (nsplit)
 		*nsplit = l.nsplit;
 	if (nksplit)
-		*nksplit = (int)cc::force_splits(h->main.plan, l.want_force).count();
+		*nksplit = l.line ? 1 : (int)cc::force_splits(h->main.plan, l.want_force).count();
 	return CC_OK;
 }
 

@@ -4,6 +4,7 @@
 #include "../../include/cc_gpu.h"
 #include "cc_kernels.cuh"
 #include "cc_lbfgs.cuh"
+#include "cc_lines.cuh"
 #include "cc_nufft.cuh"
 #include "cc_plan.h"
 
@@ -38,10 +39,32 @@ struct DevSplits {
 	cc::TabSpec *kspec = nullptr;
 };
 
+// Launch configuration of an evaluation.
+struct Launch {
+	int nsplit, per_split, csize, chunk;   // rho: particle splits (a multiple of the cluster size)
+	int want_force;                       // force: requested number of segment splits
+	bool line;                            // FP64 on the line kernels (cc_lines.cuh): nsplit, per_split, chunk as above
+	int mt, fwarps;                       // line force: tiles of 8 particles per block, warps per block
+};
+
+// A line plan (cc_plan.h) on the device.
+struct DevLines {
+	const cc::LineRow *rows = nullptr;
+	const cc::LineIdx *lines = nullptr, *tlines = nullptr;
+	const cc::LineCell *cells = nullptr;
+	const double2 *cellV = nullptr;
+	const cc::LineTabs *groups = nullptr, *phases = nullptr;
+	const cc::LineTask *tasks = nullptr;
+	double2 *weights = nullptr;     // nunit * 256
+	double *eblock = nullptr;       // one per reduce block
+};
+
 struct DevKSet {
 	cc::Plan plan;
+	cc::LinePlan lplan;
+	DevLines line;
+	unsigned char *blob = nullptr;  // one allocation for the arrays below (and the line plan's) but `partial`
 	cc::Seg *segs = nullptr;
-	cc::TabSpec *rspec = nullptr;
 	int *bstart = nullptr;
 	cc::TabSpec *bspec = nullptr;
 	double *slotV = nullptr;
@@ -54,20 +77,16 @@ struct DevKSet {
 	double2 *partial = nullptr;     // partial rows * nslot
 	size_t partial_cap = 0;         // in double2 elements
 	std::vector<DevSplits> splits;  // force splits per requested count
+	struct Chosen {
+		int64_t N;
+		bool mixed;
+		Launch l;
+	};
+	mutable std::vector<Chosen> chosen;   // launch configurations of the last few particle counts
 
 	void release()
 	{
-		cudaFree(segs);
-		cudaFree(rspec);
-		cudaFree(bstart);
-		cudaFree(bspec);
-		cudaFree(slotV);
-		cudaFree(mode_slot);
-		cudaFree(rho_slot);
-		cudaFree(u_slot);
-		cudaFree(rho_mode);
-		cudaFree(eblock);
-		cudaFree(ticket);
+		cudaFree(blob);
 		cudaFree(partial);
 		for (DevSplits &f : splits) {
 			cudaFree(f.kstart);
@@ -235,6 +254,7 @@ struct cc_handle {
 	unsigned long long last_gen = 0;
 	// S2 form (cc_create_s2): per-slot targets S0, E = sum V (|rho|^2 / N - S0)^2 + shift; split path only
 	double *d_slotS0 = nullptr;
+	double2 *d_cellS0 = nullptr;    // the same per cell of the line plan
 	// S2 over nsub sub-configurations (cc_create_s2_multiconfig): rho and u per sub-configuration, block partials
 	int nsub = 1;
 	double2 *d_msub = nullptr;      // [2][nsub][nslot]: rho, then u

@@ -237,6 +237,265 @@ ForceSplits force_splits(const Plan &p, int want)
 	return f;
 }
 
+namespace {
+
+struct Line {
+	LineIdx ix;
+	int hmax;        // cells 0 .. hmax
+	int a, b;        // first and last last index
+	int s0, s1;      // segments [s0, s1) of the plan (padding segments among them)
+};
+
+struct Span {
+	int lo = 0, hi = -1;
+	void add(int v)
+	{
+		if (hi < lo) {
+			lo = hi = v;
+		} else {
+			lo = std::min(lo, v);
+			hi = std::max(hi, v);
+		}
+	}
+	int n() const { return hi - lo + 1; }
+};
+
+// Table layout for prefix spans a (axis 0), b (axis 1), centres c and cells [hlo, hlo + nh). The entries per particle are
+// padded to `mod` modulo 8, the row stride with which the kernels' fragment loads meet no bank twice.
+LineTabs line_tabs(int d, bool centres, const Span &a, const Span &b, const Span &c, int hlo, int nh, int mod)
+{
+	LineTabs t = {};
+	const Span *s[3] = {&a, &b, &c};
+	const bool use[3] = {true, d == 3, centres};
+	int off = 0;
+	for (int e = 0; e < 3; e++) {
+		t.lo[e] = use[e] ? s[e]->lo : 0;
+		t.n[e] = use[e] ? s[e]->n() : 0;
+		t.off[e] = off;
+		off += t.n[e];
+		t.items += (t.n[e] + 7) / 8;
+		t.items16 += (t.n[e] + 15) / 16;
+	}
+	t.hlo = hlo;
+	t.nh = nh;
+	t.offh = off;
+	off += nh;
+	t.items += (nh + 7) / 8;
+	t.items16 += (nh + 15) / 16;
+	t.row = off + ((mod - off) % 8 + 8) % 8;
+	return t;
+}
+
+constexpr int kRhoRowMod = 2, kForceRowMod = 4;
+constexpr int kLineForceCells = 64;      // cells per force phase when the whole set's tables do not fit
+
+}  // namespace
+
+LinePlan build_line_plan(const Plan &p)
+{
+	LinePlan L;
+	const int d = p.d, nseg = (int)p.segs.size();
+	if (d < 2 || p.real_segs < 1)
+		return L;
+	// lines: the (sorted) segments of one prefix without a gap of more than 8 last indices
+	std::vector<Line> lines;
+	for (int q = 0; q < nseg; q++) {
+		const Seg &s = p.segs[q];
+		if (s.len == 0)
+			continue;
+		if (std::abs((int64_t)s.start) > (1 << 28))
+			return L;
+		const int last = s.start + s.len - 1;
+		if (!lines.empty() && lines.back().ix.p0 == s.p0 && lines.back().ix.p1 == s.p1 && s.start - lines.back().b <= 8) {
+			lines.back().b = last;
+			lines.back().s1 = q + 1;
+		} else {
+			lines.push_back(Line{LineIdx{s.p0, s.p1, 0, 0}, 0, s.start, last, q, q + 1});
+		}
+	}
+	// centres: all 0 (no centre factor in the kernels) unless centring each line saves more than a seventh of the cells
+	int64_t at0 = 0, centred = 0;
+	for (const Line &l : lines) {
+		at0 += std::max(std::abs(l.a), std::abs(l.b)) / 4 + 1;
+		centred += ((l.b - l.a + 1) / 2) / 4 + 1;
+	}
+	const bool centres = 7 * at0 > 8 * centred + 56;
+	for (Line &l : lines) {
+		l.ix.c = centres ? l.a + (l.b - l.a) / 2 : 0;
+		l.hmax = std::max(std::abs(l.a - l.ix.c), std::abs(l.b - l.ix.c));
+	}
+	std::stable_sort(lines.begin(), lines.end(), [](const Line &x, const Line &y) { return x.hmax / 4 > y.hmax / 4; });
+	// rows and units
+	const int nrow = (int)((lines.size() + kLineRow - 1) / kLineRow);
+	int64_t nunit = 0;
+	for (int r = 0; r < nrow; r++) {
+		const int nj = lines[(size_t)r * kLineRow].hmax / 4 + 1;
+		L.rows.push_back(LineRow{(int)nunit, nj});
+		nunit += nj;
+		if (nunit > (1 << 20))
+			return L;
+	}
+	// A unit costs what 128 slots cost at the matrix unit's rate whether it is full or not; a slot of the segment kernels
+	// costs about 3.5 times as much (12 FP64 operations at 60 % of the pipe against 6 at 90 %).
+	if ((double)nunit * 128.0 > 3.5 * 8.0 * (double)std::max<int64_t>(p.real_segs, kGroupSegs))
+		return L;
+	L.nunit = (int)nunit;
+	L.lines.resize((size_t)nrow * kLineRow);
+	L.cells.assign((size_t)nunit * 64, LineCell{-1, -1, 0, 0});
+	L.cellV.assign((size_t)nunit * 128, 0.0);
+	for (size_t q = 0; q < L.lines.size(); q++) {
+		const Line &l = lines[std::min(q, lines.size() - 1)];
+		L.lines[q] = l.ix;
+		const LineRow &R = L.rows[q / kLineRow];
+		const int i = (int)(q % kLineRow);
+		auto cell = [&](int h) { return ((size_t)(R.ubase + h / 4) * 2 + i / 8) * 32 + 4 * (i % 8) + h % 4; };
+		for (int h = 0; h < 4 * R.nj; h++)
+			L.cells[cell(h)].h = h;
+		if (q >= lines.size())
+			continue;
+		for (int k = l.s0; k < l.s1; k++)
+			for (int m = 0; m < p.segs[k].len; m++) {
+				const int h = p.segs[k].start + m - l.ix.c, slot = m * nseg + k;
+				const size_t c = cell(std::abs(h));
+				(h >= 0 ? L.cells[c].sp : L.cells[c].sm) = slot;
+				L.cellV[2 * c + (h >= 0 ? 0 : 1)] = p.slotV[(size_t)slot];
+			}
+	}
+	// rho tasks: a row's tiles in even shares of up to 4; a few rows at a time, so that a group of consecutive tasks shares
+	// few table entries (16 tasks on 4 rows x 4 shares need 128, on 2 x 8 160)
+	struct T {
+		int r, j0, n;
+	};
+	auto shares = [&](int r) { return (L.rows[r].nj + kLineTiles - 1) / kLineTiles; };
+	int ntotal = 0;
+	for (int r = 0; r < nrow; r++)
+		ntotal += shares(r);
+	// A set of up to 8 tasks runs two blocks to an SM; larger sets in groups of up to 16 tasks, a block to an SM.
+	L.ntask = std::min(kLineMaxTasks, std::max(kLineTasks, (ntotal + 3) / 4 * 4));
+	std::vector<T> tasks;
+	const int rstep = shares(0) >= 4 && nrow > 4 ? 4 : 2;
+	for (int r2 = 0; r2 < nrow; r2 += rstep)
+		for (int i = 0, top = shares(r2); i < top; i++) {
+			const int k = (r2 / rstep) % 2 ? top - 1 - i : i;   // back and forth, so that a group across two bands spans few cells
+			for (int r = r2; r < std::min(nrow, r2 + rstep); r++) {
+				const int nj = L.rows[r].nj, nt = shares(r);
+				if (k < nt)
+					tasks.push_back(T{r, nj * k / nt, nj * (k + 1) / nt - nj * k / nt});
+			}
+		}
+	const size_t ngroup = (tasks.size() + L.ntask - 1) / L.ntask;
+	for (size_t t0 = 0, g = 0; t0 < tasks.size(); g++) {
+		size_t want = (tasks.size() * (g + 1) + ngroup - 1) / ngroup;   // even groups
+		want = std::max(want, t0 + 1);
+		Span a, b, c, h;
+		LineTabs tabs = {};
+		size_t t1 = t0;
+		while (t1 < tasks.size() && t1 < want && t1 - t0 < (size_t)L.ntask) {
+			Span na = a, nb = b, nc = c, nh = h;
+			for (int i = 0; i < kLineRow; i++) {
+				const LineIdx &x = L.lines[(size_t)tasks[t1].r * kLineRow + i];
+				na.add(x.p0);
+				nb.add(x.p1);
+				nc.add(x.c);
+			}
+			nh.add(4 * tasks[t1].j0);
+			nh.add(4 * (tasks[t1].j0 + tasks[t1].n) - 1);
+			if ((int64_t)na.hi - na.lo > kLineMaxRow || (int64_t)nb.hi - nb.lo > kLineMaxRow ||
+			    (int64_t)nc.hi - nc.lo > kLineMaxRow)
+				break;
+			const LineTabs n = line_tabs(d, centres, na, nb, nc, nh.lo, nh.n(), kRhoRowMod);
+			if (n.row > kLineMaxRow)
+				break;
+			a = na, b = nb, c = nc, h = nh;
+			tabs = n;
+			t1++;
+		}
+		if (t1 == t0)
+			return LinePlan();   // one task's tables do not fit
+		tabs.ntask = (int)(t1 - t0);
+		L.group_row = std::max(L.group_row, tabs.row);
+		L.groups.push_back(tabs);
+		// warp w runs on the SM's sub-partition w mod 4, each with its own FP64 unit: the tasks, largest first, go to the
+		// sub-partition with the least work
+		std::vector<T> mine(tasks.begin() + t0, tasks.begin() + t1), at((size_t)L.ntask, T{0, 0, 0});
+		std::stable_sort(mine.begin(), mine.end(), [](const T &x, const T &y) { return x.n > y.n; });
+		int load[4] = {0, 0, 0, 0}, used[4] = {0, 0, 0, 0};
+		for (const T &x : mine) {
+			int s = -1;
+			for (int q = 0; q < 4; q++)
+				if (used[q] < L.ntask / 4 && (s < 0 || load[q] < load[s]))
+					s = q;
+			at[(size_t)(4 * used[s] + s)] = x;
+			used[s]++;
+			load[s] += x.n;
+		}
+		// a unit is 4 DMMAs of 16 cycles per 4 particles; an entry about 21 cycles per 32
+		L.group_cycles += 16.0 * *std::max_element(load, load + 4) + 0.165 * tabs.row;
+		for (const T &x : at) {
+			const LineTask k = x.n ? LineTask{L.rows[x.r].ubase + x.j0, x.n, tabs.offh + 4 * x.j0 - tabs.hlo, x.r}
+			                       : LineTask{0, 0, 0, 0};
+			L.tasks.push_back(k);
+			for (int i = 0; i < kLineRow; i++) {
+				const LineIdx &l = L.lines[(size_t)k.row * kLineRow + i];
+				L.tlines.push_back(k.n ? LineIdx{tabs.off[0] + l.p0 - tabs.lo[0],
+				                                 d == 3 ? tabs.off[1] + l.p1 - tabs.lo[1] : 0,
+				                                 centres ? tabs.off[2] + l.c - tabs.lo[2] : 0, 0}
+				                       : LineIdx{0, 0, 0, 0});
+			}
+		}
+		t0 = t1;
+	}
+	L.group_cycles /= (double)L.groups.size();
+	// force phases: the whole set when its tables fit, else chunks of kLineForceCells cells and of rows
+	const int hall = 4 * (nrow ? L.rows[0].nj : 0);
+	for (int whole = 1; whole >= 0 && L.phases.empty(); whole--) {
+		const int hstep = whole ? hall : kLineForceCells;
+		for (int h0 = 0; h0 < hall; h0 += hstep) {
+			int rmax = 0;   // rows with cells in this chunk (rows are sorted by decreasing extent)
+			while (rmax < nrow && 4 * L.rows[rmax].nj > h0)
+				rmax++;
+			const int nh = std::min(hstep, hall - h0);
+			for (int r0 = 0; r0 < rmax;) {
+				Span a, b, c;
+				LineTabs tabs = {};
+				int r1 = r0;
+				while (r1 < rmax) {
+					Span na = a, nb = b, nc = c;
+					for (int i = 0; i < kLineRow; i++) {
+						const LineIdx &x = L.lines[(size_t)r1 * kLineRow + i];
+						na.add(x.p0);
+						nb.add(x.p1);
+						nc.add(x.c);
+					}
+					if ((int64_t)na.hi - na.lo > kLineMaxRow || (int64_t)nb.hi - nb.lo > kLineMaxRow ||
+					    (int64_t)nc.hi - nc.lo > kLineMaxRow)
+						break;
+					const LineTabs n = line_tabs(d, centres, na, nb, nc, h0, nh, kForceRowMod);
+					if (n.row > kLineMaxRow)
+						break;
+					a = na, b = nb, c = nc;
+					tabs = n;
+					r1++;
+				}
+				if (r1 == r0 || (whole && r1 < rmax)) {
+					if (!whole)
+						return LinePlan();
+					L.phases.clear();
+					h0 = hall;
+					break;
+				}
+				tabs.r0 = r0;
+				tabs.ntask = r1 - r0;
+				L.phase_row = std::max(L.phase_row, tabs.row);
+				L.phases.push_back(tabs);
+				r0 = r1;
+			}
+		}
+	}
+	L.ok = true;
+	return L;
+}
+
 bool cell_geometry(int d, const double *a, double *volume, double *recip)
 {
 	double inv[9] = {0};

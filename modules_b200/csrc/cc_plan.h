@@ -71,6 +71,66 @@ Plan build_plan(int d, int64_t M, const int32_t *modes, const double *V, int L);
 // Cut the plan's segments into at least `want` force splits of similar size whose tables fit kMaxRow entries.
 ForceSplits force_splits(const Plan &p, int want);
 
+// ---------------------------------------------------------------------------------------------------------------
+// line plan: the FP64 contraction of cc_lines.cuh
+// ---------------------------------------------------------------------------------------------------------------
+// The modes of one prefix (p0[, p1]) with last index c - h .. c + h form a LINE of centre c; its CELL h holds the
+// modes c + h and c - h (cell 0 the mode c alone). Lines are sorted by decreasing extent and cut into ROWS of 16; a row
+// has nj column tiles of 4 cells, one row x column tile is a UNIT of 64 cells.
+struct LineRow {
+	int ubase, nj;      // first unit, column tiles
+};
+// Tables a group of units needs per particle: runs exp(2 pi i m s_e), m = lo .. lo + n - 1, for the prefix axes (0, 1),
+// the line centres (2, on the last axis; n = 0 when every centre is 0) and the cells h = hlo .. hlo + nh - 1 (on the last
+// axis), at entry offsets off[] and offh.
+struct alignas(16) LineTabs {
+	int lo[3], n[3], off[3];
+	int hlo, nh, offh;
+	int row;            // entries per particle
+	int items, items16; // table-building work items (8 or 16 consecutive entries of one run) per particle
+	int ntask;          // rho: warps with work. force: rows in the phase
+	int r0;             // force: first row of the phase
+	int pad[3];
+};
+// One warp's part of a rho block group: n column tiles of a row from unit u0 on, whose cells' tables start at hoff.
+struct alignas(16) LineTask {
+	int u0, n, hoff, row;
+};
+// A line's table offsets (within a group's tables) or its indices.
+struct alignas(16) LineIdx {
+	int p0, p1, c, pad;
+};
+// A cell's slots in the k-set's slot order (-1: no such mode) and its h.
+struct alignas(16) LineCell {
+	int sp, sm, h, pad;
+};
+
+constexpr int kLineRow = 16;        // lines per row
+constexpr int kLineTiles = 4;       // column tiles per rho task
+constexpr int kLineTasks = 8;       // rho tasks (warps) per block group of a small set, two blocks to an SM
+constexpr int kLineMaxTasks = 16;   // and of a large one, one block to an SM
+constexpr int kLineMaxRow = 160;    // table entries per particle
+
+struct LinePlan {
+	bool ok = false;                    // false: the k-set stays on the segment kernels
+	int nunit = 0;
+	std::vector<LineRow> rows;
+	std::vector<LineIdx> lines;         // rows x 16: (p0, p1, c)
+	std::vector<LineCell> cells;        // nunit x 64, cell ((u * 2 + half) * 32 + 4 (line & 7) + (h & 3))
+	std::vector<double> cellV;          // two weights per cell (plus, minus; 0 where there is no mode)
+	std::vector<LineTabs> groups;       // rho block groups
+	int ntask = 0;                      // tasks (warps) per group: 8, 12 or 16
+	std::vector<LineTask> tasks;        // groups x ntask (n = 0: none)
+	std::vector<LineIdx> tlines;        // groups x ntask x 16: table offsets of each task's lines
+	std::vector<LineTabs> phases;       // force phases: rows [r0, r0 + ntask) x cells [hlo, hlo + nh)
+	int group_row = 0, phase_row = 0;   // most table entries of a group / phase
+	double group_cycles = 0.0;          // a group's FP64 pipe cycles per particle (its busiest sub-partition), on average
+};
+
+// The line plan of a planned k-set. `ok` is false for d = 1, for sets whose lines fill too little of their units to beat
+// the segment kernels, and for sets whose tables do not fit.
+LinePlan build_line_plan(const Plan &p);
+
 // |det| of the basis (rows a_i) and the reciprocal basis rows b_e with b_e . a_i = 2 pi delta_ei.
 bool cell_geometry(int d, const double *basis, double *volume, double *recip);
 

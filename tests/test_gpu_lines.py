@@ -1,0 +1,87 @@
+"""The line kernels (cc_lines.cuh: FP64 energies and forces as contractions on the FP64 matrix unit) where they can go
+wrong: particle counts around the tiles of 8 to 32 particles and the splits of 8, sets whose lines need centres, sets of one
+row, of several groups and of several force phases, and sets that fall back to the segment kernels, against the plain-C
+oracle.
+
+Tolerance: a phase is at most 11 + 2 products of table entries (each within 2 ulp) away from sincospi, so |d exp| <= 15
+products x 2.2e-16 x sqrt(2) < 5e-15; the oracle forms k.r in Cartesian coordinates, an error of at most |k.r| 2^-53 x d
+(below 2e-13 for the largest |k.r| here, 2 pi 130 x 2). rho is a sum of N phases: 5e-13 N; energies and forces follow with a
+factor 2 and the sums' own rounding: 1e-12 of their scales (E ~ sum|V| N^2 / vol, F ~ 4 sum|V| N kmax / vol)."""
+import numpy as np
+import pytest
+
+import oracle
+
+pytestmark = pytest.mark.gpu
+
+
+def _box(d, m):
+    g = np.stack(np.meshgrid(*[np.arange(-m, m + 1)] * d, indexing="ij"), -1).reshape(-1, d)
+    first = np.array([next((x for x in n if x != 0), 0) for n in g])
+    return g[first > 0]
+
+
+def _set(gpu, d, kind):
+    rng = np.random.default_rng(7)
+    if kind == "stealthy":
+        return gpu.stealthy_kset(d, np.eye(d) * 400 ** (1 / d), 400, 0.45, 3)
+    if kind == "centres":      # lines that follow the prefix and lie off the origin
+        m = _box(d, 5)
+        m[:, -1] += 4 * m[:, 0] + 9
+        return m, rng.uniform(-1, 1, len(m))
+    if kind == "one line row":
+        m = _box(2, 3) if d == 2 else _box(3, 1)
+        return m, rng.uniform(0, 1, len(m))
+    if kind == "phases":       # tables beyond one force phase, several rho groups (2D)
+        m = _box(2, 130)
+        m = m[(m ** 2).sum(1) <= 130 ** 2]
+        return m, rng.uniform(0, 1, len(m))
+    m = np.concatenate([_box(d, 6), _box(d, 3), _box(d, 2)[::-1]])   # repeats, in any order
+    p = rng.permutation(len(m))
+    return m[p], rng.uniform(-1, 1, len(m))
+
+
+@pytest.mark.parametrize("N", [1, 7, 8, 9, 16, 17, 24, 25, 32, 33, 129, 1200, 2500])
+@pytest.mark.parametrize("d,kind", [(2, "stealthy"), (3, "stealthy"), (2, "centres"), (3, "centres"), (2, "one line row"),
+                                    (3, "one line row"), (3, "repeats"), (2, "phases")])
+def test_lines_against_oracle(gpu, d, kind, N):
+    modes, V = _set(gpu, d, kind)
+    if kind == "phases" and N not in (1, 25, 129):
+        pytest.skip("the oracle takes its time on this set")
+    basis = np.eye(d) * 2.0
+    basis[-1, 0] = 0.3          # a skew cell
+    frac = np.random.default_rng(N).random((N, d))
+    frac[0] = 0.0               # the edges of the cell
+    frac[-1] = 1.0 - 2.0 ** -53
+    p = gpu.CCPotential(d, basis, modes, V, 0.25)
+    p.set_path(gpu.PATH_SPLIT)
+    p.set_configuration(frac)
+    E, F = p.energy_and_forces()
+    E0 = p.energy()
+    re, im = p.rho()
+    k = oracle.lattice_k(basis, modes)
+    Eo, Fo, ro, io = oracle.port_eval(d, basis, frac, k, V, 0.25)
+    vol, sumV = abs(np.linalg.det(basis)), np.abs(V).sum()
+    kmax = np.sqrt((np.asarray(k) ** 2).sum(1)).max()
+    assert max(np.abs(re - ro).max(), np.abs(im - io).max()) <= 5e-13 * N
+    assert abs(E - Eo) <= 1e-12 * sumV * N * N / vol
+    assert np.abs(F - Fo).max() <= 1e-12 * 4 * sumV * N * kmax / vol
+    assert E0 == E              # the energy alone, summed in the same order
+    E2, F2 = p.energy_and_forces()
+    assert E2 == E and np.array_equal(F2, F)
+
+
+def test_sets_that_stay_on_the_segment_kernels(gpu):
+    """Isolated modes (no lines to speak of) and 1D sets have no line plan; their results agree with the oracle too."""
+    rng = np.random.default_rng(2)
+    for d in (1, 2, 3):
+        modes = rng.integers(-40, 41, (300, d))
+        V = rng.uniform(0, 1, 300)
+        frac = rng.random((257, d))
+        p = gpu.CCPotential(d, np.eye(d), modes, V)
+        p.set_configuration(frac)
+        E, F = p.energy_and_forces()
+        k = oracle.lattice_k(np.eye(d), modes)
+        Eo, Fo, _, _ = oracle.port_eval(d, np.eye(d), frac, k, V)
+        assert abs(E - Eo) <= 1e-12 * V.sum() * 257 ** 2
+        assert np.abs(F - Fo).max() <= 1e-12 * 4 * V.sum() * 257 * np.sqrt((np.asarray(k) ** 2).sum(1)).max()
