@@ -39,8 +39,17 @@ using cc::kBatchSegsPerSplit;
 
 // an instance's evaluation buffers in the batch arena
 struct BatchBufs {
-	size_t o_part, o_rho, o_u, o_eb, o_tk, o_pg, o_fc;
+	size_t o_part, o_rho, o_u, o_eb, o_tk, o_pg, o_fc, o_w;
 };
+
+// Particles whose tables a line rho block stages at once (two blocks share an SM).
+int batch_line_chunk(const cc::LineGroups &g, int per_split)
+{
+	int c = 8;
+	while (c < per_split && c < 64 && (size_t)2 * c * g.row * sizeof(double2) <= 96 * 1024)
+		c *= 2;
+	return c;
+}
 
 // tile shapes the autotuner times: particles per rho block, segments per force block
 constexpr int kTuneSplits[] = {32, 64, 128, 256, 512, 1024};
@@ -49,13 +58,13 @@ constexpr int kTuneSegs[] = {32, 64, 128, 256, 512, 1024};
 // dynamic shared memory the fused kernel is allowed (its largest table rows in FP64, any dimension)
 size_t mbatch_smem_cap()
 {
-	return std::max(rho_smem<double2>(cc::kMaxRow, kBatchChunk, 8), force_smem<double2>(cc::kMaxRow, 3));
+	return std::max((size_t)100 * 1024, std::max(rho_smem<double2>(cc::kMaxRow, kBatchChunk, 8), force_smem<double2>(cc::kMaxRow, 3)));
 }
 
-template <int MODE> int mbatch_launch_t(const cc::MBatchArgs &a, size_t smem, cudaStream_t st)
+template <auto KERNEL, class ARGS> int mbatch_launch_t(const ARGS &a, const int *totals, size_t smem, cudaStream_t st)
 {
-	static const cudaError_t attr = cudaFuncSetAttribute(
-	    cc::cc_mbatch_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mbatch_smem_cap());
+	static const cudaError_t attr =
+	    cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mbatch_smem_cap());
 	if (attr != cudaSuccess)
 		return fail(CC_ERR_CUDA, std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(attr));
 	// resident blocks per SM for this shared memory size (looked up once per size)
@@ -67,16 +76,15 @@ template <int MODE> int mbatch_launch_t(const cc::MBatchArgs &a, size_t smem, cu
 		auto it = per_sm.find(smem);
 		if (it == per_sm.end()) {
 			int n = 0;
-			CC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, cc::cc_mbatch_kernel<MODE>, cc::kMBatchThreads,
-			                                                      smem));
+			CC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, KERNEL, cc::kMBatchThreads, smem));
 			it = per_sm.emplace(smem, std::max(1, n)).first;
 		}
 		resident = it->second * sm_count();
 	}
-	const int total = a.total[0] + a.total[1] + a.total[2];
+	const int total = totals[0] + totals[1] + totals[2];
 	if (total <= 0)
 		return CC_OK;
-	CC_CUDA(launch_pdl_n(cc::cc_mbatch_kernel<MODE>, dim3(std::min(total, resident)), dim3(cc::kMBatchThreads), smem,
+	CC_CUDA(launch_pdl_n(KERNEL, dim3(std::min(total, resident)), dim3(cc::kMBatchThreads), smem,
 	                     st, a));
 	return CC_OK;
 }
@@ -89,9 +97,9 @@ int cc::launch_mbatch(int mode, const MBatchArgs &a, int rho_row, int force_row,
 		return CC_OK;
 	const size_t smem = std::max(rho_smem<double2>(rho_row, kBatchChunk, 8), force_smem<double2>(force_row, maxd));
 	switch (mode) {
-	case 0: return mbatch_launch_t<0>(a, smem, st);
-	case 1: return mbatch_launch_t<1>(a, smem, st);
-	default: return mbatch_launch_t<2>(a, smem, st);
+	case 0: return mbatch_launch_t<cc::cc_mbatch_kernel<0> >(a, a.total, smem, st);
+	case 1: return mbatch_launch_t<cc::cc_mbatch_kernel<1> >(a, a.total, smem, st);
+	default: return mbatch_launch_t<cc::cc_mbatch_kernel<2> >(a, a.total, smem, st);
 	}
 }
 
@@ -110,11 +118,22 @@ struct cc_batch {
 	cc::ReduceArgs *d_red[2] = {nullptr, nullptr};
 	cc::ForceArgs *d_force[2] = {nullptr, nullptr};
 	int *d_dim = nullptr;                    // B
-	int *d_pre = nullptr;                    // 4 x (B + 1): rho, reduce, force, reduce + force items per instance
+	int *d_pre = nullptr;                    // 3 queues (one per mode) of 4 x (B + 1): rho, reduce, force, reduce +
+	                                         // force items per instance
 	int *d_shape = nullptr;                  // 3 x B
+	// instances with a line plan: their FP64 descriptors (set 0 / 1), and the two item counts of every instance
+	bool any_line = false, all_line = false;
+	cc::LineRhoArgs *d_lrho[2] = {nullptr, nullptr};
+	cc::LineReduceArgs *d_lred[2] = {nullptr, nullptr};
+	cc::LineForceArgs *d_lforce[2] = {nullptr, nullptr};
+	int *d_own = nullptr;                    // 6 x B
+	size_t line_smem = 0;
+	std::vector<cc::LineRhoArgs> lrho;       // host copies of set 0
+	std::vector<cc::LineReduceArgs> lred;
+	std::vector<cc::LineForceArgs> lforce;
 	unsigned *d_queue = nullptr;             // 2 words
 	unsigned *d_count = nullptr;             // 3 x B completion counts + 1 error word
-	int total[3] = {0, 0, 0};
+	int total[3][3] = {};                    // items per mode and phase
 	int rho_row = 1, force_row = 1, maxd = 1;
 	unsigned wait_spins = 0, wait_phantom = 0;   // cc_batch_set_wait_test
 	std::vector<cc::RhoArgs> rho;            // host copies of set 0 (in `order`)
@@ -131,19 +150,19 @@ struct cc_batch {
 
 namespace {
 
-cc::MBatchArgs batch_args(const cc_batch *b, int set, int want_stage)
+cc::MBatchArgs batch_args(const cc_batch *b, int set, int mode)
 {
 	cc::MBatchArgs a;
 	a.rho = b->d_rho[set];
 	a.red = b->d_red[set];
 	a.force = b->d_force[set];
 	a.dim = b->d_dim;
-	a.pre = b->d_pre;
+	a.pre = b->d_pre + (size_t)mode * 4 * (b->order.size() + 1);
 	a.shape = b->d_shape;
 	a.B = (int)b->order.size();
 	for (int k = 0; k < 3; k++)
-		a.total[k] = b->total[k];
-	a.want_stage = want_stage;
+		a.total[k] = b->total[mode][k];
+	a.want_stage = mode == 1 ? 0 : 1;
 	a.queue = b->d_queue;
 	a.count = b->d_count;
 	a.spins = b->wait_spins;
@@ -156,10 +175,14 @@ cc::MBatchArgs batch_args(const cc_batch *b, int set, int want_stage)
 int batch_build(cc_batch *b, int per_split, int segs_per_split)
 {
 	const int B = (int)b->order.size();
-	std::vector<int> pre(4 * (B + 1), 0), shape(3 * B, 0), dim(B, 0);
+	std::vector<int> pre(3 * 4 * (B + 1), 0), shape(3 * B, 0), dim(B, 0), own(6 * B, 0);
 	b->rho.clear();
 	b->red.clear();
 	b->force.clear();
+	b->lrho.clear();
+	b->lred.clear();
+	b->lforce.clear();
+	b->line_smem = 0;
 	b->rho_row = b->force_row = 1;
 	b->maxd = 1;
 	for (int k = 0; k < B; k++) {
@@ -225,25 +248,100 @@ int batch_build(cc_batch *b, int per_split, int segs_per_split)
 		b->red.push_back(rr);
 		b->force.push_back(fa);
 		const int c[3] = {p.nbgroups() * nsplit, nchunks, pgroups * fa.nksplit};
-		const int sh[3] = {p.nbgroups(), nchunks, pgroups};
-		for (int ph = 0; ph < 3; ph++) {
-			pre[ph * (B + 1) + k + 1] = pre[ph * (B + 1) + k] + c[ph];
-			shape[ph * B + k] = sh[ph];
+		cc::LineRhoArgs lr = {};
+		cc::LineReduceArgs ld = {};
+		cc::LineForceArgs lf = {};
+		for (int ph = 0; ph < 3; ph++)
+			own[ph * B + k] = c[ph];
+		if (h->main.lplan.ok) {
+			const cc::LinePlan &L = h->main.lplan;
+			const DevLines &dl = h->main.line;
+			lr.frac = ra.frac;
+			lr.N = ra.N;
+			lr.per_split = per_split;
+			lr.chunk = batch_line_chunk(L.groups8(), per_split);
+			lr.log2chunk = __builtin_ctz((unsigned)lr.chunk);
+			lr.ngroup = L.groups8().count();
+			lr.nunit = L.nunit;
+			lr.ntask = cc::kLineTasks;
+			lr.groups = dl.narrow.groups;
+			lr.tasks = dl.narrow.tasks;
+			lr.tlines = dl.narrow.tlines;
+			lr.partial = ra.partial;
+			ld.partial = lr.partial;
+			ld.nsplit = nsplit;
+			ld.nunit = L.nunit;
+			ld.cells = dl.cells;
+			ld.cellV = dl.cellV;
+			ld.rho_offset = h->rho_offset;
+			ld.weights = b->arena.at<double2>(q.o_w);
+			ld.eblock = rr.eblock;
+			lf.frac = ra.frac;
+			lf.N = ra.N;
+			lf.nphase = (int)L.phases.size();
+			lf.phases = dl.phases;
+			lf.rows = dl.rows;
+			lf.lines = dl.lines;
+			lf.weights = ld.weights;
+			for (int e = 0; e < 9; e++)
+				lf.recip[e] = h->recip[e];
+			lf.fscale = fa.fscale;
+			lf.F_out = fa.F_out;
+			lf.eblock = rr.eblock;
+			lf.neblock = (L.nunit + cc::kLineWideUnits - 1) / cc::kLineWideUnits;
+			lf.inv_vol = fa.inv_vol;
+			lf.shift = fa.shift;
+			lf.E_out = fa.E_out;
+			lf.tiles = 1;   // set below
+			const int lc[3] = {lr.ngroup * nsplit, lf.neblock, (int)((n + 8 * cc::kLineBatchMT - 1) / (8 * cc::kLineBatchMT))};
+			for (int ph = 0; ph < 3; ph++)
+				own[(3 + ph) * B + k] = lc[ph];
+			b->line_smem = std::max(b->line_smem, std::max(cc::line_rho_smem(L.groups8().row, lr.chunk, h->d),
+			                                               cc::line_force_smem(L.phase_row, cc::kLineBatchMT, 8, h->d)));
 		}
+		b->lrho.push_back(lr);
+		b->lred.push_back(ld);
+		b->lforce.push_back(lf);
+		const int sh[3] = {p.nbgroups(), nchunks, pgroups};
+		for (int ph = 0; ph < 3; ph++)
+			shape[ph * B + k] = sh[ph];
 		dim[k] = h->d;
 		b->rho_row = std::max(b->rho_row, p.block_max_row);
 		b->force_row = std::max(b->force_row, f->host.max_row);
 		b->maxd = std::max(b->maxd, h->d);
 	}
-	for (int ph = 0; ph < 3; ph++)
-		b->total[ph] = pre[ph * (B + 1) + B];
-	for (int k = 0; k < B; k++)   // each instance's reduce and force items, consecutive in the queue
-		pre[3 * (B + 1) + k + 1] = pre[3 * (B + 1) + k] + (pre[(B + 1) + k + 1] - pre[(B + 1) + k]) +
-		                           (pre[2 * (B + 1) + k + 1] - pre[2 * (B + 1) + k]);
+	// Line force items: several tiles each where the batch has many (a tile's results do not depend on it), so that an
+	// item's fixed cost (queue, descriptor, completion: 4 us) stays small beside its tiles (10 to 20 us each).
+	int64_t tiles = 0;
+	for (int k = 0; k < B; k++)
+		tiles += own[5 * B + k];
+	const int per_item = (int)std::max<int64_t>(1, std::min<int64_t>(8, tiles / (6 * 2 * sm_count())));
+	for (int k = 0; k < B; k++) {
+		b->lforce[k].tiles = per_item;
+		own[5 * B + k] = (own[5 * B + k] + per_item - 1) / per_item;
+	}
+	// the queue of each mode: 0 line items where there is a line plan, 1 segment items, 2 (an instance's stage decides) the
+	// larger of the two counts
+	for (int mode = 0; mode < 3; mode++) {
+		int *q = pre.data() + (size_t)mode * 4 * (B + 1);
+		for (int k = 0; k < B; k++) {
+			int c[3];
+			for (int ph = 0; ph < 3; ph++) {
+				const int seg = own[ph * B + k], line = own[(3 + ph) * B + k];
+				c[ph] = mode == 1 || line == 0 ? seg : mode == 0 ? line : std::max(seg, line);
+				q[ph * (B + 1) + k + 1] = q[ph * (B + 1) + k] + c[ph];
+			}
+			q[3 * (B + 1) + k + 1] = q[3 * (B + 1) + k] + c[1] + c[2];   // its reduce and force items, consecutive
+		}
+		for (int ph = 0; ph < 3; ph++)
+			b->total[mode][ph] = q[ph * (B + 1) + B];
+	}
 	int rc;
 	if ((rc = upload_into(b->d_rho[0], b->rho)) || (rc = upload_into(b->d_red[0], b->red)) ||
 	    (rc = upload_into(b->d_force[0], b->force)) || (rc = upload_into(b->d_pre, pre)) ||
-	    (rc = upload_into(b->d_shape, shape)) || (rc = upload_into(b->d_dim, dim)))
+	    (rc = upload_into(b->d_shape, shape)) || (rc = upload_into(b->d_dim, dim)) ||
+	    (rc = upload_into(b->d_lrho[0], b->lrho)) || (rc = upload_into(b->d_lred[0], b->lred)) ||
+	    (rc = upload_into(b->d_lforce[0], b->lforce)) || (rc = upload_into(b->d_own, own)))
 		return rc;
 	b->per_split = per_split;
 	b->segs_per_split = segs_per_split;
@@ -256,7 +354,25 @@ int batch_build(cc_batch *b, int per_split, int segs_per_split)
 int batch_eval(cc_batch *b, int set, int precision, cudaStream_t st)
 {
 	const int mode = precision == CC_PREC_SCHEDULE ? 2 : precision == CC_PREC_MIXED ? 1 : 0;
-	return cc::launch_mbatch(mode, batch_args(b, set, mode == 1 ? 0 : 1), b->rho_row, b->force_row, b->maxd, st);
+	if (b->any_line) {
+		cc::LBatchArgs a;
+		a.m = batch_args(b, set, mode);
+		a.lrho = b->d_lrho[set];
+		a.lred = b->d_lred[set];
+		a.lforce = b->d_lforce[set];
+		a.own = b->d_own;
+		// segment items need their own shared memory: mixed ones, and those of instances without a line plan
+		size_t smem = mode == 1 ? 0 : b->line_smem;
+		if (mode != 0 || !b->all_line)
+			smem = std::max(smem, std::max(rho_smem<double2>(b->rho_row, kBatchChunk, 8),
+			                               force_smem<double2>(b->force_row, b->maxd)));
+		switch (mode) {
+		case 0: return mbatch_launch_t<cc::cc_lbatch_kernel<0> >(a, a.m.total, smem, st);
+		case 1: return mbatch_launch_t<cc::cc_lbatch_kernel<1> >(a, a.m.total, smem, st);
+		default: return mbatch_launch_t<cc::cc_lbatch_kernel<2> >(a, a.m.total, smem, st);
+		}
+	}
+	return cc::launch_mbatch(mode, batch_args(b, set, mode), b->rho_row, b->force_row, b->maxd, st);
 }
 
 // A bounded wait of the fused kernel that ran out leaves the error word set: report it (after a synchronisation of
@@ -314,17 +430,24 @@ int cc_batch_create(int count, cc_handle *const *handles, const int64_t *N, cc_b
 		}
 		const int max_nsplit = (int)((n + kTuneSplits[0] - 1) / kTuneSplits[0]);
 		const int nchunks = (p.nslot + 31) / 32, pgroups = (int)((n + 31) / 32);
+		const cc::LinePlan &L = h->main.lplan;
+		const size_t row = std::max((size_t)p.nslot, L.ok ? (size_t)L.nunit * 128 : 0);   // entries of a partial row
+		b->any_line |= L.ok;
 		b->off_frac[i] = b->arena.take(sizeof(double) * n * h->d);
 		b->off_F[i] = b->arena.take(sizeof(double) * n * h->d);
 		b->off_E[i] = b->arena.take(sizeof(double));
-		q.o_part = b->arena.take(sizeof(double2) * (size_t)max_nsplit * p.nslot);
+		q.o_part = b->arena.take(sizeof(double2) * (size_t)max_nsplit * row);
 		q.o_rho = b->arena.take(sizeof(double2) * p.nslot);
 		q.o_u = b->arena.take(sizeof(double2) * p.nslot);
-		q.o_eb = b->arena.take(sizeof(double) * nchunks);
+		q.o_eb = b->arena.take(sizeof(double) * std::max(nchunks, L.nunit));
+		q.o_w = b->arena.take(sizeof(double2) * (size_t)L.nunit * 256);
 		q.o_tk = b->arena.take(sizeof(unsigned));
 		q.o_pg = b->arena.take(sizeof(double) * (size_t)max_nks * n * h->d);
 		q.o_fc = b->arena.take(sizeof(unsigned) * pgroups);
 	}
+	b->all_line = true;
+	for (int i = 0; i < count; i++)
+		b->all_line &= handles[i]->main.lplan.ok;
 	int rc;
 	if ((rc = dev_alloc(&b->arena.base, b->arena.used))) {
 		cc_batch_destroy(b);
@@ -346,7 +469,10 @@ int cc_batch_create(int count, cc_handle *const *handles, const int64_t *N, cc_b
 	const int B = count;
 	if ((rc = dev_alloc(&b->d_rho[0], B)) || (rc = dev_alloc(&b->d_red[0], B)) || (rc = dev_alloc(&b->d_force[0], B)) ||
 	    (rc = dev_alloc(&b->d_rho[1], B)) || (rc = dev_alloc(&b->d_red[1], B)) || (rc = dev_alloc(&b->d_force[1], B)) ||
-	    (rc = dev_alloc(&b->d_pre, 4 * (B + 1))) || (rc = dev_alloc(&b->d_shape, 3 * B)) ||
+	    (rc = dev_alloc(&b->d_pre, 3 * 4 * (B + 1))) || (rc = dev_alloc(&b->d_shape, 3 * B)) ||
+	    (rc = dev_alloc(&b->d_lrho[0], B)) || (rc = dev_alloc(&b->d_lred[0], B)) ||
+	    (rc = dev_alloc(&b->d_lforce[0], B)) || (rc = dev_alloc(&b->d_lrho[1], B)) ||
+	    (rc = dev_alloc(&b->d_lred[1], B)) || (rc = dev_alloc(&b->d_lforce[1], B)) || (rc = dev_alloc(&b->d_own, 6 * B)) ||
 	    (rc = dev_alloc(&b->d_dim, B)) || (rc = dev_alloc(&b->d_queue, 2)) || (rc = dev_alloc(&b->d_count, 3 * B + 1)) ||
 	    (rc = (cudaMemset(b->d_queue, 0, 2 * sizeof(unsigned)) == cudaSuccess &&
 	                   cudaMemset(b->d_count, 0, (3 * B + 1) * sizeof(unsigned)) == cudaSuccess
@@ -421,7 +547,11 @@ int cc_batch_destroy(cc_batch *b)
 		cudaFree(b->d_rho[w]);
 		cudaFree(b->d_red[w]);
 		cudaFree(b->d_force[w]);
+		cudaFree(b->d_lrho[w]);
+		cudaFree(b->d_lred[w]);
+		cudaFree(b->d_lforce[w]);
 	}
+	cudaFree(b->d_own);
 	cudaFree(b->d_dim);
 	cudaFree(b->d_pre);
 	cudaFree(b->d_shape);
@@ -596,6 +726,9 @@ int cc_batch_minimize(cc_batch *b, double *const *frac, const cc_lbfgs_opts *opt
 	std::vector<cc::RhoArgs> ra = b->rho;
 	std::vector<cc::ReduceArgs> rr = b->red;
 	std::vector<cc::ForceArgs> fa = b->force;
+	std::vector<cc::LineRhoArgs> lra = b->lrho;
+	std::vector<cc::LineReduceArgs> lrr = b->lred;
+	std::vector<cc::LineForceArgs> lfa = b->lforce;
 	for (int k = 0; k < count; k++) {
 		const int i = b->order[k];
 		lbo[k] = lbi[i];
@@ -612,9 +745,17 @@ int cc_batch_minimize(cc_batch *b, double *const *frac, const cc_lbfgs_opts *opt
 		fa[k].F_out = nullptr;
 		fa[k].skip = status;
 		fa[k].stage = stage;
+		lra[k].frac = ra[k].frac;
+		lra[k].skip = lrr[k].skip = lfa[k].skip = status;
+		lra[k].stage = lrr[k].stage = lfa[k].stage = stage;
+		lfa[k].frac = fa[k].frac;
+		lfa[k].E_out = fa[k].E_out;
+		lfa[k].gfrac_out = fa[k].gfrac_out;
+		lfa[k].F_out = nullptr;
 	}
 	if ((rc = upload_into(b->d_lb, lbo)) || (rc = upload_into(b->d_rho[1], ra)) || (rc = upload_into(b->d_red[1], rr)) ||
-	    (rc = upload_into(b->d_force[1], fa)))
+	    (rc = upload_into(b->d_force[1], fa)) || (rc = upload_into(b->d_lrho[1], lra)) ||
+	    (rc = upload_into(b->d_lred[1], lrr)) || (rc = upload_into(b->d_lforce[1], lfa)))
 		return rc;
 	cudaStream_t st = b->stream;
 	const bool sched = o.precision == CC_PREC_SCHEDULE;

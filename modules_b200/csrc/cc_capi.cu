@@ -111,9 +111,15 @@ int cci::upload_kset(DevKSet &k, const cc::Plan &plan)
 #define CC_PUT(v) put((v).data(), (v).size() * sizeof((v)[0]))
 	const size_t o_segs = CC_PUT(plan.segs), o_bstart = CC_PUT(plan.bstart), o_bspec = CC_PUT(plan.bspec),
 	             o_slotV = CC_PUT(plan.slotV), o_mode = CC_PUT(plan.mode_slot);
-	const size_t o_rows = CC_PUT(L.rows), o_lines = CC_PUT(L.lines), o_tlines = CC_PUT(L.tlines), o_cells = CC_PUT(L.cells),
-	             o_cellV = CC_PUT(L.cellV), o_groups = CC_PUT(L.groups), o_phases = CC_PUT(L.phases),
-	             o_tasks = CC_PUT(L.tasks);
+	const size_t o_rows = CC_PUT(L.rows), o_lines = CC_PUT(L.lines), o_cells = CC_PUT(L.cells), o_cellV = CC_PUT(L.cellV),
+	             o_phases = CC_PUT(L.phases);
+	const cc::LineGroups *lg[2] = {&L.wide, &L.narrow};
+	size_t o_groups[2], o_tasks[2], o_tlines[2];
+	for (int i = 0; i < 2; i++) {
+		o_groups[i] = CC_PUT(lg[i]->groups);
+		o_tasks[i] = CC_PUT(lg[i]->tasks);
+		o_tlines[i] = CC_PUT(lg[i]->tlines);
+	}
 #undef CC_PUT
 	const size_t nslot = plan.slotV.size(), M = plan.mode_slot.size();
 	const size_t nred = (nslot + 31) / 32, nlred = (size_t)L.nunit * (64 / cc::kLineRedCells);
@@ -144,12 +150,17 @@ int cci::upload_kset(DevKSet &k, const cc::Plan &plan)
 	k.eblock = reinterpret_cast<double *>(b + o_eb);
 	k.line.rows = reinterpret_cast<cc::LineRow *>(b + o_rows);
 	k.line.lines = reinterpret_cast<cc::LineIdx *>(b + o_lines);
-	k.line.tlines = reinterpret_cast<cc::LineIdx *>(b + o_tlines);
 	k.line.cells = reinterpret_cast<cc::LineCell *>(b + o_cells);
 	k.line.cellV = reinterpret_cast<double2 *>(b + o_cellV);
-	k.line.groups = reinterpret_cast<cc::LineTabs *>(b + o_groups);
 	k.line.phases = reinterpret_cast<cc::LineTabs *>(b + o_phases);
-	k.line.tasks = reinterpret_cast<cc::LineTask *>(b + o_tasks);
+	DevLines::Groups *dg[2] = {&k.line.wide, &k.line.narrow};
+	for (int i = 0; i < 2; i++) {
+		dg[i]->groups = reinterpret_cast<cc::LineTabs *>(b + o_groups[i]);
+		dg[i]->tasks = reinterpret_cast<cc::LineTask *>(b + o_tasks[i]);
+		dg[i]->tlines = reinterpret_cast<cc::LineIdx *>(b + o_tlines[i]);
+	}
+	if (L.narrow.ntask == 0)
+		k.line.narrow = k.line.wide;
 	k.line.weights = reinterpret_cast<double2 *>(b + o_w);
 	k.line.eblock = reinterpret_cast<double *>(b + o_leb);
 	return CC_OK;
@@ -200,9 +211,9 @@ Launch choose_line_launch(const cc::LinePlan &p, int d, int64_t N)
 	l.line = true;
 	l.csize = 1;
 	const int sms = sm_count();
-	const int64_t G = std::max<int64_t>(1, (int64_t)p.groups.size());
-	const int per_sm = p.ntask <= cc::kLineTasks ? 2 : 1;
-	const double particle_us = p.group_cycles / (kLinePipe * 1965.0);
+	const int64_t G = std::max<int64_t>(1, (int64_t)p.wide.count());
+	const int per_sm = p.wide.ntask <= cc::kLineTasks ? 2 : 1;
+	const double particle_us = p.wide.cycles / (kLinePipe * 1965.0);
 	double best = 1e300;
 	l.nsplit = 1;
 	l.per_split = 8;
@@ -222,9 +233,9 @@ Launch choose_line_launch(const cc::LinePlan &p, int d, int64_t N)
 			break;
 	}
 	// chunks: a power of two that holds a split, or as many particles as fit (and have a thread per coordinate)
-	const size_t row = (size_t)p.group_row * sizeof(double2);
+	const size_t row = (size_t)p.wide.row * sizeof(double2);
 	const size_t room = (per_sm == 2 ? 100 : 204) * 1024;
-	const int most = std::min(cc::kLineMaxChunk, p.ntask * 32 / d);
+	const int most = std::min(cc::kLineMaxChunk, p.wide.ntask * 32 / d);
 	l.chunk = 8;
 	while (l.chunk < l.per_split && 2 * l.chunk <= most && 2 * l.chunk * row <= room)
 		l.chunk *= 2;
@@ -698,17 +709,17 @@ int run_rho(cc_handle *h, DevKSet &k, int64_t N, const double *d_frac, double *d
 		a.per_split = N > 0 ? l.per_split : 0;
 		a.chunk = l.chunk;
 		a.log2chunk = __builtin_ctz((unsigned)l.chunk);
-		a.ngroup = (int)L.groups.size();
+		a.ngroup = L.wide.count();
 		a.nunit = L.nunit;
-		a.ntask = L.ntask;
-		a.groups = k.line.groups;
-		a.tasks = k.line.tasks;
-		a.tlines = k.line.tlines;
+		a.ntask = L.wide.ntask;
+		a.groups = k.line.wide.groups;
+		a.tasks = k.line.wide.tasks;
+		a.tlines = k.line.wide.tlines;
 		a.partial = k.partial;
 		a.skip = h->d_skip;
 		a.frac_copy = (&k == &h->main) ? h->rho_copy : nullptr;
 		a.early = (h->early_call && &k == &h->main && !a.skip && !a.frac_copy) ? 1 : 0;
-		const size_t smem = cc::line_rho_smem(L.group_row, l.chunk, h->d);
+		const size_t smem = cc::line_rho_smem(L.wide.row, l.chunk, h->d);
 		if (int rc = h->d == 2 ? launch_line_rho_t<2>(a, nsplit, smem, st) : launch_line_rho_t<3>(a, nsplit, smem, st))
 			return rc;
 		if (after_rho)

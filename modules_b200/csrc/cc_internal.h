@@ -50,11 +50,15 @@ struct Launch {
 // A line plan (cc_plan.h) on the device.
 struct DevLines {
 	const cc::LineRow *rows = nullptr;
-	const cc::LineIdx *lines = nullptr, *tlines = nullptr;
+	const cc::LineIdx *lines = nullptr;
 	const cc::LineCell *cells = nullptr;
 	const double2 *cellV = nullptr;
-	const cc::LineTabs *groups = nullptr, *phases = nullptr;
-	const cc::LineTask *tasks = nullptr;
+	const cc::LineTabs *phases = nullptr;
+	struct Groups {
+		const cc::LineTabs *groups = nullptr;
+		const cc::LineTask *tasks = nullptr;
+		const cc::LineIdx *tlines = nullptr;
+	} wide, narrow;                 // narrow: of blocks of 8 warps (the wide ones where these have 8)
 	double2 *weights = nullptr;     // nunit * 256
 	double *eblock = nullptr;       // one per reduce block
 };

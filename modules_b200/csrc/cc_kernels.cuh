@@ -1250,6 +1250,26 @@ __device__ __forceinline__ int4 mbatch_decode(const MBatchArgs &A, int item)
 	return within < nred ? make_int4(item, 1, b, within) : make_int4(item, 2, b, within - nred);
 }
 
+// Count a finished item (queue position, phase, instance, item within the phase).
+__device__ __forceinline__ void mbatch_done(const MBatchArgs &A, const int4 it)
+{
+	// the item's results are visible before its count rises
+	__threadfence();
+	__syncthreads();
+	if (threadIdx.x == 0) {
+		const int phase = it.y, b = it.z;
+		const int *pre = A.pre + phase * (A.B + 1);
+		unsigned *cnt = A.count + phase * A.B + b;
+		const unsigned done = atomicAdd(cnt, 1u) + 1u;
+		if (phase == 2 && done == (unsigned)(__ldg(pre + b + 1) - __ldg(pre + b))) {
+			// the instance's last item: its counts start from zero in the next launch
+			A.count[b] = 0u;
+			A.count[A.B + b] = 0u;
+			*cnt = 0u;
+		}
+	}
+}
+
 template <int MODE>
 __global__ void __launch_bounds__(kMBatchThreads, 3) cc_mbatch_kernel(MBatchArgs A)
 {
@@ -1275,21 +1295,7 @@ __global__ void __launch_bounds__(kMBatchThreads, 3) cc_mbatch_kernel(MBatchArgs
 			mbatch_item<2, MODE>(A, it.y, it.z, it.w);
 		else
 			mbatch_item<1, MODE>(A, it.y, it.z, it.w);
-		// the item's results are visible before its count rises
-		__threadfence();
-		__syncthreads();
-		if (threadIdx.x == 0) {
-			const int phase = it.y, b = it.z;
-			const int *pre = A.pre + phase * (A.B + 1);
-			unsigned *cnt = A.count + phase * A.B + b;
-			const unsigned done = atomicAdd(cnt, 1u) + 1u;
-			if (phase == 2 && done == (unsigned)(__ldg(pre + b + 1) - __ldg(pre + b))) {
-				// the instance's last item: its counts start from zero in the next launch
-				A.count[b] = 0u;
-				A.count[A.B + b] = 0u;
-				*cnt = 0u;
-			}
-		}
+		mbatch_done(A, it);
 	}
 	queue_leave(A.queue);
 }

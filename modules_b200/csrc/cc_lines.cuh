@@ -463,6 +463,84 @@ __device__ __forceinline__ void line_reduce_body(const LineReduceArgs &a, const 
 	}
 }
 
+// Item `item` of the reduction in the batch launch: two units (128 cells, a thread per component), every component summed
+// over the rows in row order. Wide items, as reduce_body_wide: a batch's many small reductions cost few of them.
+constexpr int kLineWideUnits = 2;
+__device__ __forceinline__ void line_reduce_wide_body(const LineReduceArgs &a, const int item, const ItemCtl ctl)
+{
+	double2 *sh = &body_shared().red[0][0];   // 256 entries
+	double *she = body_shared().pos;          // one energy per warp
+	const int unit = item * kLineWideUnits + ((int)threadIdx.x >> 7), part = threadIdx.x & 127;
+	const int half = part >> 6, comp = (part >> 5) & 1, lane = part & 31;
+	const bool on = unit < a.nunit;
+	const int cell = unit * 64 + half * 32 + lane;
+	LineCell cl = {-1, -1, 0, 0};
+	double2 V = make_double2(0.0, 0.0);
+	if (on) {
+		cl = load_rec(a.cells + cell);
+		V = __ldg(a.cellV + cell);
+	}
+	if (ctl.ready)
+		wait_ready(ctl.ready, ctl.ready_need, ctl.err, ctl.ready_spins);
+	if (eval_skipped(a.skip, ctl.stage, ctl.want_stage))
+		return;
+	double2 v = make_double2(0.0, 0.0);
+	if (on) {
+		const double2 *p = a.partial + (size_t)unit * 128 + part;
+		const size_t stride = (size_t)a.nunit * 128;
+		int s = 0;
+		for (; s + 8 <= a.nsplit; s += 8) {
+			double2 x[8];
+#pragma unroll
+			for (int i = 0; i < 8; i++)
+				x[i] = __ldcg(p + (size_t)(s + i) * stride);
+#pragma unroll
+			for (int i = 0; i < 8; i++) {
+				v.x += x[i].x;
+				v.y += x[i].y;
+			}
+		}
+		for (; s < a.nsplit; s++) {
+			const double2 x = __ldcg(p + (size_t)s * stride);
+			v.x += x.x;
+			v.y += x.y;
+		}
+	}
+	sh[threadIdx.x] = v;
+	__syncthreads();
+	const double2 ra = sh[threadIdx.x & ~32], ia = sh[threadIdx.x | 32];   // (Re A, Re B), (Im A, Im B)
+	double e = 0.0;
+	double2 up = make_double2(0.0, 0.0), um = up;
+	if (cl.sp >= 0) {
+		const double2 r = make_double2(ra.x - ia.y + a.rho_offset, ia.x + ra.y);
+		e = V.x * (r.x * r.x + r.y * r.y);
+		up = make_double2(V.x * r.x, -V.x * r.y);
+	}
+	if (cl.sm >= 0) {
+		const double2 r = make_double2(ra.x + ia.y + a.rho_offset, ia.x - ra.y);
+		e += V.y * (r.x * r.x + r.y * r.y);
+		um = make_double2(V.y * r.x, -V.y * r.y);
+	}
+	if (on) {
+		a.weights[line_weight_at(cell, 2 * comp)] = line_weight(2 * comp, cl.h, up, um);
+		a.weights[line_weight_at(cell, 2 * comp + 1)] = line_weight(2 * comp + 1, cl.h, up, um);
+	}
+	e = comp == 0 ? e : 0.0;
+#pragma unroll
+	for (int o = 16; o > 0; o >>= 1)
+		e += __shfl_down_sync(0xffffffffu, e, o);
+	if ((threadIdx.x & 31) == 0)
+		she[threadIdx.x >> 5] = e;
+	__syncthreads();
+	if (threadIdx.x == 0) {
+		double t = 0.0;
+#pragma unroll
+		for (int w = 0; w < 8; w++)
+			t += she[w];
+		a.eblock[item] = t;
+	}
+}
+
 static __global__ void __launch_bounds__(kLineRedThreads) cc_line_reduce_kernel(LineReduceArgs a)
 {
 	line_reduce_body(a, blockIdx.x, gridDim.x, ItemCtl{a.stage, a.want_stage});
@@ -488,6 +566,7 @@ struct LineForceArgs {
 	const double *frac;       // N x D
 	int N;
 	int nphase;
+	int tiles;                // in a batch: tiles per item
 	const LineTabs *phases;
 	const LineRow *rows;
 	const LineIdx *lines;     // rows x 16
@@ -523,24 +602,22 @@ __device__ __forceinline__ void line_energy_body(const LineForceArgs &a, const I
 // MT = 1: 13.7 us per evaluation with four pairs, 15.9 with two; MT = 2 with 16 warps: 13.6 and 13.3).
 __host__ __device__ constexpr int line_nt(int mt) { return mt == 1 ? 4 : 2; }
 
-// Block `tile` = 8 MT particles, W warps. Per phase the particles' tables are built, then the warps take the phase's rows
+// Tiles [tile0, tile1) of 8 MT particles each, W warps. Per tile and phase the particles' tables are built, then the warps take the phase's rows
 // in turn (8 / NT warps a row, NT line pairs each) and contract the row's cells: per 4 cells NT weight fragments of 512 B
 // from L2 (read once per block, in fragment order) against MT table fragments from shared memory, 2 MT NT DMMAs. What is
 // left beside the DMMAs is instructions per step and the product with X per task, so weights with T's and D's factors
 // written out (64 B a cell) beat 32 B ones expanded here (2D N=1e5: 2.05 against 2.17 ms per evaluation; 3D N=20000: 178
 // against 187 us), and a ring of asynchronous copies for the weights gains nothing over loads one step ahead.
 template <int D, int MT, int W>
-__device__ __forceinline__ void line_force_body(const LineForceArgs &a, const int tile, const ItemCtl ctl)
+__device__ __forceinline__ void line_force_body(const LineForceArgs &a, const int tile0, const int tile1, const ItemCtl ctl)
 {
 	constexpr int P = 8 * MT, E = MT <= 2 ? 8 : 16, NT = line_nt(MT), SUB = 8 / NT, LOG2P = MT == 1 ? 3 : MT == 2 ? 4 : 5;
 	extern __shared__ __align__(16) unsigned char smem[];
 	double *pos = reinterpret_cast<double *>(smem);    // P x D
 	double2 *tab = reinterpret_cast<double2 *>(smem + line_pos_bytes(P, D));
-	double *sh_g = reinterpret_cast<double *>(smem);   // after the loops: W warps x P x D
+	double *sh_g = reinterpret_cast<double *>(tab);    // after the loops: W warps x P x D
 	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 	const int t = lane & 3, g = lane >> 2;
-	const int pbase = tile * P;
-	const int nvalid = min(P, a.N - pbase);
 	LineTabs tb = load_rec(a.phases);
 	// (as force_body: a finished instance builds no tables, but waits for its reduce items where there are any)
 	if (eval_skipped(a.skip, ctl.stage, ctl.want_stage)) {
@@ -548,169 +625,187 @@ __device__ __forceinline__ void line_force_body(const LineForceArgs &a, const in
 			wait_ready(ctl.ready, ctl.ready_need, ctl.err, ctl.ready_spins);
 		return;
 	}
-	if ((int)threadIdx.x < nvalid * D)
-		pos[threadIdx.x] = a.frac[(size_t)pbase * D + threadIdx.x];
-	__syncthreads();
-	// The tables need only the positions, which the rho pass of this evaluation has already read: they are built while
-	// the reduce kernel still runs (programmatic dependent launch).
-	build_line_tables<D, E>(tb, pos, LOG2P, P, nvalid, tab);
-	cudaGridDependencySynchronize();
-	if (ctl.ready)
-		wait_ready(ctl.ready, ctl.ready_need, ctl.err, ctl.ready_spins);
-	if (eval_skipped(a.skip, ctl.stage, ctl.want_stage))
-		return;
-	double gs[MT][D];
-#pragma unroll
-	for (int m = 0; m < MT; m++)
-#pragma unroll
-		for (int e = 0; e < D; e++)
-			gs[m][e] = 0.0;
-
-	for (int ph = 0; ph < a.nphase; ph++) {
-		if (ph > 0) {
-			tb = load_rec(a.phases + ph);
-			__syncthreads();
-			build_line_tables<D, E>(tb, pos, LOG2P, P, nvalid, tab);
+	// coordinate threadIdx.x of a tile, loaded a tile ahead
+	auto load = [&](int tile) {
+		return (int)threadIdx.x < min(P, a.N - tile * P) * D ? a.frac[(size_t)tile * P * D + threadIdx.x] : 0.0;
+	};
+	double next = load(tile0);
+	for (int tile = tile0; tile < tile1; tile++) {
+		const int pbase = tile * P;
+		const int nvalid = min(P, a.N - pbase);
+		if (tile > tile0) {
+			tb = load_rec(a.phases);
+			__syncthreads();   // the previous tile's sums are read
 		}
+		if ((int)threadIdx.x < P * D)
+			pos[threadIdx.x] = next;
 		__syncthreads();
-		const bool centres = tb.n[2] > 0;
-		const int jb = tb.hlo >> 2, je = (tb.hlo + tb.nh) >> 2;
-		const double2 *trow = tab + (size_t)g * tb.row;
-		// the weights are read one step ahead, across tasks; a task's row record one task ahead
-		const int ntask = tb.ntask * SUB;
-		int2 ri = make_int2(0, 0), rn = ri;
-		double2 bq[NT];
-		auto row_rec = [&](int q) { return __ldg(reinterpret_cast<const int2 *>(a.rows) + tb.r0 + q / SUB); };
-		auto first_w = [&](int q, int2 x) { return a.weights + ((size_t)(x.x + jb) * 8 + (q % SUB) * NT) * 32 + lane; };
-		if (warp < ntask) {
-			ri = row_rec(warp);
-			const double2 *w = first_w(warp, ri);
-#pragma unroll
-			for (int n = 0; n < NT; n++)
-				bq[n] = __ldcg(w + n * 32);
+		// The tables need only the positions, which the rho pass of this evaluation has already read: they are built while
+		// the reduce kernel still runs (programmatic dependent launch).
+		build_line_tables<D, E>(tb, pos, LOG2P, P, nvalid, tab);
+		if (tile == tile0) {
+			cudaGridDependencySynchronize();
+			if (ctl.ready)
+				wait_ready(ctl.ready, ctl.ready_need, ctl.err, ctl.ready_spins);
+			if (eval_skipped(a.skip, ctl.stage, ctl.want_stage))
+				return;
 		}
-		for (int s = warp; s < ntask; s += W) {
-			const int r = tb.r0 + s / SUB, pair = (s % SUB) * NT;
-			const bool more = s + W < ntask;
-			if (more)
-				rn = row_rec(s + W);
-			const int nj = min(je, ri.y) - jb;   // > 0: the phase's rows all reach its first cells
-			const double2 *w = first_w(s, ri);
-			const double2 *wn = more ? first_w(s + W, rn) : w;
-			ri = rn;
-			double2 acc[MT][NT];
-			LineIdx li[NT];
-#pragma unroll
-			for (int n = 0; n < NT; n++)
-				li[n] = load_rec(a.lines + (size_t)r * kLineRow + (pair + n) * 2 + (t >> 1));
-#pragma unroll
-			for (int m = 0; m < MT; m++)
-#pragma unroll
-				for (int n = 0; n < NT; n++)
-					acc[m][n] = make_double2(0.0, 0.0);
-			const double2 *th = trow + tb.offh + t;
-			for (int j = 0; j < nj; j++, th += 4) {
-				double2 f[NT];
-#pragma unroll
-				for (int n = 0; n < NT; n++)
-					f[n] = bq[n];   // lane (t, g): cell 4 j + t, line g / 4 of the pair, component g % 4
-				w = j + 1 < nj ? w + 8 * 32 : wn;
-#pragma unroll
-				for (int n = 0; n < NT; n++)
-					bq[n] = __ldcg(w + n * 32);
-				// (C_h, S_h) of particle 8 m + g, h = 4 j + t
-				double2 c[MT];
-#pragma unroll
-				for (int m = 0; m < MT; m++)
-					c[m] = th[m * 8 * tb.row];
-#pragma unroll
-				for (int m = 0; m + 1 < MT; m += 2)
-#pragma unroll
-					for (int n = 0; n < NT; n++)
-						dmma16(acc[m][n], acc[m + 1][n], c[m].x, c[m + 1].x, c[m].y, c[m + 1].y, f[n].x, f[n].y);
-				if (MT & 1) {
-#pragma unroll
-					for (int n = 0; n < NT; n++)
-						dmma(acc[MT - 1][n], c[MT - 1].x, f[n].x);
-#pragma unroll
-					for (int n = 0; n < NT; n++)
-						dmma(acc[MT - 1][n], c[MT - 1].y, f[n].y);
-				}
-			}
-			// lane (g, t): particle 8 m + g, line t / 2 of pair n: T for even t, D for odd t. Stage by stage over the MT x NT
-			// tiles: each FP64 operation may wait behind another warp's matrix instructions, so the chains run side by side.
-			double2 x[MT][NT];
-#pragma unroll
-			for (int n = 0; n < NT; n++) {
-				const int o0 = tb.off[0] + li[n].p0 - tb.lo[0], o1 = tb.off[1] + li[n].p1 - tb.lo[1];
-#pragma unroll
-				for (int m = 0; m < MT; m++) {
-					x[m][n] = trow[m * 8 * tb.row + o0];
-					if (D == 3)
-						x[m][n] = cmul(x[m][n], trow[m * 8 * tb.row + o1]);
-				}
-			}
-			if (centres) {
-#pragma unroll
-				for (int n = 0; n < NT; n++)
-#pragma unroll
-					for (int m = 0; m < MT; m++)
-						x[m][n] = cmul(x[m][n], trow[m * 8 * tb.row + tb.off[2] + li[n].c - tb.lo[2]]);
-			}
-			double S[MT][NT];
-#pragma unroll
-			for (int m = 0; m < MT; m++)
-#pragma unroll
-				for (int n = 0; n < NT; n++)
-					S[m][n] = x[m][n].y * acc[m][n].x;
-#pragma unroll
-			for (int m = 0; m < MT; m++)
-#pragma unroll
-				for (int n = 0; n < NT; n++)
-					S[m][n] = fma(x[m][n].x, acc[m][n].y, S[m][n]);
-#pragma unroll
-			for (int n = 0; n < NT; n++) {
-				const double k0 = (t & 1) ? 0.0 : (double)li[n].p0;
-				const double k1 = (t & 1) ? 0.0 : (double)li[n].p1;
-				const double kl = (t & 1) ? 1.0 : (double)li[n].c;
-#pragma unroll
-				for (int m = 0; m < MT; m++) {
-					gs[m][0] = fma(k0, S[m][n], gs[m][0]);
-					if (D == 3)
-						gs[m][1] = fma(k1, S[m][n], gs[m][1]);
-					gs[m][D - 1] = fma(kl, S[m][n], gs[m][D - 1]);
-				}
-			}
-		}
-	}
-	cudaTriggerProgrammaticLaunchCompletion();
-	// the four lanes of a particle, then the warps in order
-#pragma unroll
-	for (int m = 0; m < MT; m++)
-#pragma unroll
-		for (int e = 0; e < D; e++) {
-			gs[m][e] += __shfl_xor_sync(0xffffffffu, gs[m][e], 1);
-			gs[m][e] += __shfl_xor_sync(0xffffffffu, gs[m][e], 2);
-		}
-	__syncthreads();
-	if (t == 0) {
+		if (tile + 1 < tile1)
+			next = load(tile + 1);
+		double gs[MT][D];
 #pragma unroll
 		for (int m = 0; m < MT; m++)
 #pragma unroll
 			for (int e = 0; e < D; e++)
-				sh_g[(warp * P + m * 8 + g) * D + e] = gs[m][e];
-	}
-	__syncthreads();
-	if ((int)threadIdx.x < nvalid) {
-		double v[D];
+				gs[m][e] = 0.0;
+
+		for (int ph = 0; ph < a.nphase; ph++) {
+			if (ph > 0) {
+				tb = load_rec(a.phases + ph);
+				__syncthreads();
+				build_line_tables<D, E>(tb, pos, LOG2P, P, nvalid, tab);
+			}
+			__syncthreads();
+			const bool centres = tb.n[2] > 0;
+			const int jb = tb.hlo >> 2, je = (tb.hlo + tb.nh) >> 2;
+			const double2 *trow = tab + (size_t)g * tb.row;
+			// the weights are read one step ahead, across tasks; a task's row record one task ahead
+			const int ntask = tb.ntask * SUB;
+			int2 ri = make_int2(0, 0), rn = ri;
+			double2 bq[NT];
+			auto row_rec = [&](int q) { return __ldg(reinterpret_cast<const int2 *>(a.rows) + tb.r0 + q / SUB); };
+			auto first_w = [&](int q, int2 x) { return a.weights + ((size_t)(x.x + jb) * 8 + (q % SUB) * NT) * 32 + lane; };
+			if (warp < ntask) {
+				ri = row_rec(warp);
+				const double2 *w = first_w(warp, ri);
 #pragma unroll
-		for (int e = 0; e < D; e++) {
-			v[e] = sh_g[threadIdx.x * D + e];
+				for (int n = 0; n < NT; n++)
+					bq[n] = __ldcg(w + n * 32);
+			}
+			for (int s = warp; s < ntask; s += W) {
+				const int r = tb.r0 + s / SUB, pair = (s % SUB) * NT;
+				const bool more = s + W < ntask;
+				if (more)
+					rn = row_rec(s + W);
+				const int nj = min(je, ri.y) - jb;   // > 0: the phase's rows all reach its first cells
+				const double2 *w = first_w(s, ri);
+				const double2 *wn = more ? first_w(s + W, rn) : w;
+				ri = rn;
+				double2 acc[MT][NT];
+				LineIdx li[NT];
 #pragma unroll
-			for (int w2 = 1; w2 < W; w2++)
-				v[e] += sh_g[(w2 * P + threadIdx.x) * D + e];
+				for (int n = 0; n < NT; n++)
+					li[n] = load_rec(a.lines + (size_t)r * kLineRow + (pair + n) * 2 + (t >> 1));
+#pragma unroll
+				for (int m = 0; m < MT; m++)
+#pragma unroll
+					for (int n = 0; n < NT; n++)
+						acc[m][n] = make_double2(0.0, 0.0);
+				const double2 *th = trow + tb.offh + t;
+				for (int j = 0; j < nj; j++, th += 4) {
+					double2 f[NT];
+#pragma unroll
+					for (int n = 0; n < NT; n++)
+						f[n] = bq[n];   // lane (t, g): cell 4 j + t, line g / 4 of the pair, component g % 4
+					w = j + 1 < nj ? w + 8 * 32 : wn;
+#pragma unroll
+					for (int n = 0; n < NT; n++)
+						bq[n] = __ldcg(w + n * 32);
+					// (C_h, S_h) of particle 8 m + g, h = 4 j + t
+					double2 c[MT];
+#pragma unroll
+					for (int m = 0; m < MT; m++)
+						c[m] = th[m * 8 * tb.row];
+#pragma unroll
+					for (int m = 0; m + 1 < MT; m += 2)
+#pragma unroll
+						for (int n = 0; n < NT; n++)
+							dmma16(acc[m][n], acc[m + 1][n], c[m].x, c[m + 1].x, c[m].y, c[m + 1].y, f[n].x, f[n].y);
+					if (MT & 1) {
+#pragma unroll
+						for (int n = 0; n < NT; n++)
+							dmma(acc[MT - 1][n], c[MT - 1].x, f[n].x);
+#pragma unroll
+						for (int n = 0; n < NT; n++)
+							dmma(acc[MT - 1][n], c[MT - 1].y, f[n].y);
+					}
+				}
+				// lane (g, t): particle 8 m + g, line t / 2 of pair n: T for even t, D for odd t. Stage by stage over the MT x NT
+				// tiles: each FP64 operation may wait behind another warp's matrix instructions, so the chains run side by side.
+				double2 x[MT][NT];
+#pragma unroll
+				for (int n = 0; n < NT; n++) {
+					const int o0 = tb.off[0] + li[n].p0 - tb.lo[0], o1 = tb.off[1] + li[n].p1 - tb.lo[1];
+#pragma unroll
+					for (int m = 0; m < MT; m++) {
+						x[m][n] = trow[m * 8 * tb.row + o0];
+						if (D == 3)
+							x[m][n] = cmul(x[m][n], trow[m * 8 * tb.row + o1]);
+					}
+				}
+				if (centres) {
+#pragma unroll
+					for (int n = 0; n < NT; n++)
+#pragma unroll
+						for (int m = 0; m < MT; m++)
+							x[m][n] = cmul(x[m][n], trow[m * 8 * tb.row + tb.off[2] + li[n].c - tb.lo[2]]);
+				}
+				double S[MT][NT];
+#pragma unroll
+				for (int m = 0; m < MT; m++)
+#pragma unroll
+					for (int n = 0; n < NT; n++)
+						S[m][n] = x[m][n].y * acc[m][n].x;
+#pragma unroll
+				for (int m = 0; m < MT; m++)
+#pragma unroll
+					for (int n = 0; n < NT; n++)
+						S[m][n] = fma(x[m][n].x, acc[m][n].y, S[m][n]);
+#pragma unroll
+				for (int n = 0; n < NT; n++) {
+					const double k0 = (t & 1) ? 0.0 : (double)li[n].p0;
+					const double k1 = (t & 1) ? 0.0 : (double)li[n].p1;
+					const double kl = (t & 1) ? 1.0 : (double)li[n].c;
+#pragma unroll
+					for (int m = 0; m < MT; m++) {
+						gs[m][0] = fma(k0, S[m][n], gs[m][0]);
+						if (D == 3)
+							gs[m][1] = fma(k1, S[m][n], gs[m][1]);
+						gs[m][D - 1] = fma(kl, S[m][n], gs[m][D - 1]);
+					}
+				}
+			}
 		}
-		write_force_out<D>(a.F_out, a.gfrac_out, a.recip, a.fscale, pbase + threadIdx.x, v);
+		if (tile + 1 == tile1)
+			cudaTriggerProgrammaticLaunchCompletion();
+		// the four lanes of a particle, then the warps in order
+#pragma unroll
+		for (int m = 0; m < MT; m++)
+#pragma unroll
+			for (int e = 0; e < D; e++) {
+				gs[m][e] += __shfl_xor_sync(0xffffffffu, gs[m][e], 1);
+				gs[m][e] += __shfl_xor_sync(0xffffffffu, gs[m][e], 2);
+			}
+		__syncthreads();
+		if (t == 0) {
+#pragma unroll
+			for (int m = 0; m < MT; m++)
+#pragma unroll
+				for (int e = 0; e < D; e++)
+					sh_g[(warp * P + m * 8 + g) * D + e] = gs[m][e];
+		}
+		__syncthreads();
+		if ((int)threadIdx.x < nvalid) {
+			double v[D];
+#pragma unroll
+			for (int e = 0; e < D; e++) {
+				v[e] = sh_g[threadIdx.x * D + e];
+#pragma unroll
+				for (int w2 = 1; w2 < W; w2++)
+					v[e] += sh_g[(w2 * P + threadIdx.x) * D + e];
+			}
+			write_force_out<D>(a.F_out, a.gfrac_out, a.recip, a.fscale, pbase + threadIdx.x, v);
+		}
 	}
 }
 
@@ -721,9 +816,8 @@ __host__ __device__ constexpr size_t line_rho_smem(int row, int chunk, int d)
 }
 __host__ __device__ constexpr size_t line_force_smem(int row, int mt, int warps, int d)
 {
-	const size_t tables = line_pos_bytes(8 * mt, d) + (size_t)row * 8 * mt * sizeof(double2);
-	const size_t sums = (size_t)warps * 8 * mt * d * sizeof(double);
-	return tables > sums ? tables : sums;
+	const size_t tables = (size_t)row * 8 * mt * sizeof(double2), sums = (size_t)warps * 8 * mt * d * sizeof(double);
+	return line_pos_bytes(8 * mt, d) + (tables > sums ? tables : sums);
 }
 
 // 8 warps: two blocks to an SM; 16 warps: one, for grids of one wave (8 warps alone on an SM leave its matrix units idle
@@ -736,7 +830,154 @@ __global__ void __launch_bounds__(32 * W, W == 8 ? 2 : 1) cc_line_force_kernel(L
 	if (tile < 0)
 		line_energy_body(a, ItemCtl{a.stage, a.want_stage});
 	else
-		line_force_body<D, MT, W>(a, tile, ItemCtl{a.stage, a.want_stage});
+		line_force_body<D, MT, W>(a, tile, tile + 1, ItemCtl{a.stage, a.want_stage});
+}
+
+// ---------------------------------------------------------------------------------------------------------------
+// fused batch evaluation with line plans
+// ---------------------------------------------------------------------------------------------------------------
+// The launch of cc_mbatch_kernel (one work queue, phases ordered by completion counts) for batches in which some instance
+// has a line plan: such an instance's FP64 items are line items, its mixed items (and every item of the other instances)
+// segment items. An instance's phase holds the larger of its two item counts, so that the queue does not depend on the
+// stages; the surplus items do nothing and are counted.
+struct LBatchArgs {
+	MBatchArgs m;
+	const LineRhoArgs *lrho;
+	const LineReduceArgs *lred;
+	const LineForceArgs *lforce;
+	const int *own;       // 6 x B: segment items of the three phases, line items (0: no line plan)
+};
+
+union LineItemDesc {
+	RhoArgs rho;
+	ReduceArgs red;
+	ForceArgs force;
+	LineRhoArgs lrho;
+	LineReduceArgs lred;
+	LineForceArgs lforce;
+};
+__device__ __forceinline__ LineItemDesc &line_item_desc()
+{
+	__shared__ LineItemDesc s;
+	return s;
+}
+
+// The bodies as calls: inlined together into one kernel they spill (1.4 KB a thread at 128 registers).
+template <int D> __device__ __noinline__ void line_rho_call(const LineRhoArgs &r, int local, const ItemCtl &ctl)
+{
+	line_rho_body<D>(r, local % r.ngroup, local / r.ngroup, ctl);
+}
+constexpr int kLineBatchMT = 3;      // tiles of 8 particles in a batch's force tile
+template <int D> __device__ __noinline__ void line_force_call(const LineForceArgs &f, int local, const ItemCtl &ctl)
+{
+	constexpr int P = 8 * kLineBatchMT;
+	const int ntile = (f.N + P - 1) / P, t0 = local * f.tiles;
+	line_force_body<D, kLineBatchMT, 8>(f, t0, min(ntile, t0 + f.tiles), ctl);
+}
+template <int D, bool MIXED> __device__ __noinline__ void seg_rho_call(const RhoArgs &r, int ng, int local, const ItemCtl &ctl)
+{
+	rho_body<D, 8, MIXED, false>(r, local % ng, local / ng, ctl);
+}
+template <int D, bool MIXED> __device__ __noinline__ void seg_force_call(const ForceArgs &f, int pg, int local, const ItemCtl &ctl)
+{
+	force_body<D, 8, MIXED>(f, local % pg, local / pg, ctl);
+}
+
+// MODE as mbatch_item: 0 FP64, 1 mixed, 2 each instance at the precision of its stage word
+template <int D, int MODE>
+__device__ __forceinline__ void lbatch_item(const LBatchArgs &L, int phase, int b, int local)
+{
+	const MBatchArgs &A = L.m;
+	ItemCtl ctl;
+	ctl.err = A.count + 3 * A.B;
+	ctl.ready_spins = A.spins;
+	ctl.want_stage = A.want_stage;
+	const int *stage = A.rho[b].stage;
+	const bool mixed = MODE == 1 || (MODE == 2 && stage && *(volatile const int *)stage == 0);
+	const int nline = __ldg(L.own + (3 + phase) * A.B + b);
+	const bool line = !mixed && D >= 2 && nline > 0;
+	ctl.stage = MODE == 2 ? nullptr : stage;
+	if (phase > 0) {
+		ctl.ready = A.count + (phase - 1) * A.B + b;
+		ctl.ready_need = (unsigned)(__ldg(A.pre + (phase - 1) * (A.B + 1) + b + 1) - __ldg(A.pre + (phase - 1) * (A.B + 1) + b)) +
+		                 (phase == 1 && b == 0 ? A.phantom : 0u);
+	}
+	if (local >= (line ? nline : __ldg(L.own + phase * A.B + b)))
+		return;
+	if constexpr (MODE != 1 && D >= 2) {
+		if (line) {
+			if (phase == 0) {
+				const LineRhoArgs &r = stage_desc(L.lrho + b, line_item_desc().lrho);
+				line_rho_call<D>(r, local, ctl);
+			} else if (phase == 1) {
+				line_reduce_wide_body(stage_desc(L.lred + b, line_item_desc().lred), local, ctl);
+			} else {
+				const LineForceArgs &f = stage_desc(L.lforce + b, line_item_desc().lforce);
+				line_force_call<D>(f, local, ctl);
+				// the instance's first force item also sums the energy (its reduce items are complete)
+				if (local == 0 && f.E_out && !eval_skipped(f.skip, ctl.stage, ctl.want_stage)) {
+					const double e = line_energy_sum(f.eblock, f.neblock);
+					if (threadIdx.x == 0)
+						*f.E_out = e * f.inv_vol + f.shift;
+				}
+			}
+			return;
+		}
+	}
+	if (phase == 0) {
+		const RhoArgs &r = stage_desc(A.rho + b, line_item_desc().rho);
+		const int ng = __ldg(A.shape + b);
+		if constexpr (MODE != 0) {
+			if (mixed) {
+				seg_rho_call<D, true>(r, ng, local, ctl);
+				return;
+			}
+		}
+		if constexpr (MODE != 1)
+			seg_rho_call<D, false>(r, ng, local, ctl);
+	} else if (phase == 1) {
+		reduce_body_wide(stage_desc(A.red + b, line_item_desc().red), local, ctl);
+	} else {
+		const ForceArgs &f = stage_desc(A.force + b, line_item_desc().force);
+		const int pg = __ldg(A.shape + 2 * A.B + b);
+		if constexpr (MODE != 0) {
+			if (mixed) {
+				seg_force_call<D, true>(f, pg, local, ctl);
+				return;
+			}
+		}
+		if constexpr (MODE != 1)
+			seg_force_call<D, false>(f, pg, local, ctl);
+	}
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(kMBatchThreads, MODE == 1 ? 3 : 2) cc_lbatch_kernel(LBatchArgs L)
+{
+	const MBatchArgs &A = L.m;
+	__shared__ int4 sh_item;
+	const int T = A.total[0] + A.total[1] + A.total[2];
+	cudaGridDependencySynchronize();
+	for (;;) {
+		__syncthreads();
+		if (threadIdx.x == 0) {
+			const int item = (int)atomicAdd(A.queue, 1u);
+			sh_item = item < T ? mbatch_decode(A, item) : make_int4(item, 0, 0, 0);
+		}
+		__syncthreads();
+		const int4 it = sh_item;
+		if (it.x >= T)
+			break;
+		const int d = __ldg(A.dim + it.z);
+		if (d == 3)
+			lbatch_item<3, MODE>(L, it.y, it.z, it.w);
+		else if (d == 2)
+			lbatch_item<2, MODE>(L, it.y, it.z, it.w);
+		else
+			lbatch_item<1, MODE>(L, it.y, it.z, it.w);
+		mbatch_done(A, it);
+	}
+	queue_leave(A.queue);
 }
 
 }  // namespace cc

@@ -289,6 +289,96 @@ LineTabs line_tabs(int d, bool centres, const Span &a, const Span &b, const Span
 constexpr int kRhoRowMod = 2, kForceRowMod = 4;
 constexpr int kLineForceCells = 64;      // cells per force phase when the whole set's tables do not fit
 
+// Block groups of `ntask` tasks; false when a task's tables do not fit.
+bool line_groups(const LinePlan &L, int d, bool centres, int ntask, LineGroups *out)
+{
+	LineGroups &G = *out;
+	G = LineGroups();
+	G.ntask = ntask;
+	const int nrow = (int)L.rows.size();
+	// rho tasks: a row's tiles in even shares of up to 4; a few rows at a time, so that a group of consecutive tasks shares
+	// few table entries (16 tasks on 4 rows x 4 shares need 128, on 2 x 8 160)
+	struct T {
+		int r, j0, n;
+	};
+	auto shares = [&](int r) { return (L.rows[r].nj + kLineTiles - 1) / kLineTiles; };
+	std::vector<T> tasks;
+	const int rstep = ntask > kLineTasks && shares(0) >= 4 && nrow > 4 ? 4 : 2;
+	for (int r2 = 0; r2 < nrow; r2 += rstep)
+		for (int i = 0, top = shares(r2); i < top; i++) {
+			const int k = (r2 / rstep) % 2 ? top - 1 - i : i;   // back and forth, so that a group across two bands spans few cells
+			for (int r = r2; r < std::min(nrow, r2 + rstep); r++) {
+				const int nj = L.rows[r].nj, nt = shares(r);
+				if (k < nt)
+					tasks.push_back(T{r, nj * k / nt, nj * (k + 1) / nt - nj * k / nt});
+			}
+		}
+	const size_t ngroup = (tasks.size() + ntask - 1) / ntask;
+	for (size_t t0 = 0, g = 0; t0 < tasks.size(); g++) {
+		size_t want = (tasks.size() * (g + 1) + ngroup - 1) / ngroup;   // even groups
+		want = std::max(want, t0 + 1);
+		Span a, b, c, h;
+		LineTabs tabs = {};
+		size_t t1 = t0;
+		while (t1 < tasks.size() && t1 < want && t1 - t0 < (size_t)ntask) {
+			Span na = a, nb = b, nc = c, nh = h;
+			for (int i = 0; i < kLineRow; i++) {
+				const LineIdx &x = L.lines[(size_t)tasks[t1].r * kLineRow + i];
+				na.add(x.p0);
+				nb.add(x.p1);
+				nc.add(x.c);
+			}
+			nh.add(4 * tasks[t1].j0);
+			nh.add(4 * (tasks[t1].j0 + tasks[t1].n) - 1);
+			if ((int64_t)na.hi - na.lo > kLineMaxRow || (int64_t)nb.hi - nb.lo > kLineMaxRow ||
+			    (int64_t)nc.hi - nc.lo > kLineMaxRow)
+				break;
+			const LineTabs n = line_tabs(d, centres, na, nb, nc, nh.lo, nh.n(), kRhoRowMod);
+			if (n.row > kLineMaxRow)
+				break;
+			a = na, b = nb, c = nc, h = nh;
+			tabs = n;
+			t1++;
+		}
+		if (t1 == t0)
+			return false;
+		tabs.ntask = (int)(t1 - t0);
+		G.row = std::max(G.row, tabs.row);
+		G.groups.push_back(tabs);
+		// warp w runs on the SM's sub-partition w mod 4, each with its own FP64 unit: the tasks, largest first, go to the
+		// sub-partition with the least work
+		std::vector<T> mine(tasks.begin() + t0, tasks.begin() + t1), at((size_t)ntask, T{0, 0, 0});
+		std::stable_sort(mine.begin(), mine.end(), [](const T &x, const T &y) { return x.n > y.n; });
+		int load[4] = {0, 0, 0, 0}, used[4] = {0, 0, 0, 0};
+		for (const T &x : mine) {
+			int s = -1;
+			for (int q = 0; q < 4; q++)
+				if (used[q] < ntask / 4 && (s < 0 || load[q] < load[s]))
+					s = q;
+			at[(size_t)(4 * used[s] + s)] = x;
+			used[s]++;
+			load[s] += x.n;
+		}
+		// a unit is 4 DMMAs of 16 cycles per 4 particles; an entry about 21 cycles per 32
+		G.cycles += 16.0 * *std::max_element(load, load + 4) + 0.165 * tabs.row;
+		for (const T &x : at) {
+			const LineTask k = x.n ? LineTask{L.rows[x.r].ubase + x.j0, x.n, tabs.offh + 4 * x.j0 - tabs.hlo, x.r}
+			                       : LineTask{0, 0, 0, 0};
+			G.tasks.push_back(k);
+			for (int i = 0; i < kLineRow; i++) {
+				const LineIdx &l = L.lines[(size_t)k.row * kLineRow + i];
+				G.tlines.push_back(k.n ? LineIdx{tabs.off[0] + l.p0 - tabs.lo[0],
+				                                 d == 3 ? tabs.off[1] + l.p1 - tabs.lo[1] : 0,
+				                                 centres ? tabs.off[2] + l.c - tabs.lo[2] : 0, 0}
+				                       : LineIdx{0, 0, 0, 0});
+			}
+		}
+		t0 = t1;
+	}
+	G.cycles /= (double)G.groups.size();
+	return true;
+}
+
 }  // namespace
 
 LinePlan build_line_plan(const Plan &p)
@@ -361,91 +451,13 @@ LinePlan build_line_plan(const Plan &p)
 				L.cellV[2 * c + (h >= 0 ? 0 : 1)] = p.slotV[(size_t)slot];
 			}
 	}
-	// rho tasks: a row's tiles in even shares of up to 4; a few rows at a time, so that a group of consecutive tasks shares
-	// few table entries (16 tasks on 4 rows x 4 shares need 128, on 2 x 8 160)
-	struct T {
-		int r, j0, n;
-	};
-	auto shares = [&](int r) { return (L.rows[r].nj + kLineTiles - 1) / kLineTiles; };
 	int ntotal = 0;
 	for (int r = 0; r < nrow; r++)
-		ntotal += shares(r);
+		ntotal += (L.rows[r].nj + kLineTiles - 1) / kLineTiles;
 	// A set of up to 8 tasks runs two blocks to an SM; larger sets in groups of up to 16 tasks, a block to an SM.
-	L.ntask = std::min(kLineMaxTasks, std::max(kLineTasks, (ntotal + 3) / 4 * 4));
-	std::vector<T> tasks;
-	const int rstep = shares(0) >= 4 && nrow > 4 ? 4 : 2;
-	for (int r2 = 0; r2 < nrow; r2 += rstep)
-		for (int i = 0, top = shares(r2); i < top; i++) {
-			const int k = (r2 / rstep) % 2 ? top - 1 - i : i;   // back and forth, so that a group across two bands spans few cells
-			for (int r = r2; r < std::min(nrow, r2 + rstep); r++) {
-				const int nj = L.rows[r].nj, nt = shares(r);
-				if (k < nt)
-					tasks.push_back(T{r, nj * k / nt, nj * (k + 1) / nt - nj * k / nt});
-			}
-		}
-	const size_t ngroup = (tasks.size() + L.ntask - 1) / L.ntask;
-	for (size_t t0 = 0, g = 0; t0 < tasks.size(); g++) {
-		size_t want = (tasks.size() * (g + 1) + ngroup - 1) / ngroup;   // even groups
-		want = std::max(want, t0 + 1);
-		Span a, b, c, h;
-		LineTabs tabs = {};
-		size_t t1 = t0;
-		while (t1 < tasks.size() && t1 < want && t1 - t0 < (size_t)L.ntask) {
-			Span na = a, nb = b, nc = c, nh = h;
-			for (int i = 0; i < kLineRow; i++) {
-				const LineIdx &x = L.lines[(size_t)tasks[t1].r * kLineRow + i];
-				na.add(x.p0);
-				nb.add(x.p1);
-				nc.add(x.c);
-			}
-			nh.add(4 * tasks[t1].j0);
-			nh.add(4 * (tasks[t1].j0 + tasks[t1].n) - 1);
-			if ((int64_t)na.hi - na.lo > kLineMaxRow || (int64_t)nb.hi - nb.lo > kLineMaxRow ||
-			    (int64_t)nc.hi - nc.lo > kLineMaxRow)
-				break;
-			const LineTabs n = line_tabs(d, centres, na, nb, nc, nh.lo, nh.n(), kRhoRowMod);
-			if (n.row > kLineMaxRow)
-				break;
-			a = na, b = nb, c = nc, h = nh;
-			tabs = n;
-			t1++;
-		}
-		if (t1 == t0)
-			return LinePlan();   // one task's tables do not fit
-		tabs.ntask = (int)(t1 - t0);
-		L.group_row = std::max(L.group_row, tabs.row);
-		L.groups.push_back(tabs);
-		// warp w runs on the SM's sub-partition w mod 4, each with its own FP64 unit: the tasks, largest first, go to the
-		// sub-partition with the least work
-		std::vector<T> mine(tasks.begin() + t0, tasks.begin() + t1), at((size_t)L.ntask, T{0, 0, 0});
-		std::stable_sort(mine.begin(), mine.end(), [](const T &x, const T &y) { return x.n > y.n; });
-		int load[4] = {0, 0, 0, 0}, used[4] = {0, 0, 0, 0};
-		for (const T &x : mine) {
-			int s = -1;
-			for (int q = 0; q < 4; q++)
-				if (used[q] < L.ntask / 4 && (s < 0 || load[q] < load[s]))
-					s = q;
-			at[(size_t)(4 * used[s] + s)] = x;
-			used[s]++;
-			load[s] += x.n;
-		}
-		// a unit is 4 DMMAs of 16 cycles per 4 particles; an entry about 21 cycles per 32
-		L.group_cycles += 16.0 * *std::max_element(load, load + 4) + 0.165 * tabs.row;
-		for (const T &x : at) {
-			const LineTask k = x.n ? LineTask{L.rows[x.r].ubase + x.j0, x.n, tabs.offh + 4 * x.j0 - tabs.hlo, x.r}
-			                       : LineTask{0, 0, 0, 0};
-			L.tasks.push_back(k);
-			for (int i = 0; i < kLineRow; i++) {
-				const LineIdx &l = L.lines[(size_t)k.row * kLineRow + i];
-				L.tlines.push_back(k.n ? LineIdx{tabs.off[0] + l.p0 - tabs.lo[0],
-				                                 d == 3 ? tabs.off[1] + l.p1 - tabs.lo[1] : 0,
-				                                 centres ? tabs.off[2] + l.c - tabs.lo[2] : 0, 0}
-				                       : LineIdx{0, 0, 0, 0});
-			}
-		}
-		t0 = t1;
-	}
-	L.group_cycles /= (double)L.groups.size();
+	const int ntask = std::min(kLineMaxTasks, std::max(kLineTasks, (ntotal + 3) / 4 * 4));
+	if (!line_groups(L, d, centres, ntask, &L.wide) || (ntask > kLineTasks && !line_groups(L, d, centres, kLineTasks, &L.narrow)))
+		return LinePlan();   // one task's tables do not fit
 	// force phases: the whole set when its tables fit, else chunks of kLineForceCells cells and of rows
 	const int hall = 4 * (nrow ? L.rows[0].nj : 0);
 	for (int whole = 1; whole >= 0 && L.phases.empty(); whole--) {

@@ -111,6 +111,17 @@ constexpr int kLineTasks = 8;       // rho tasks (warps) per block group of a sm
 constexpr int kLineMaxTasks = 16;   // and of a large one, one block to an SM
 constexpr int kLineMaxRow = 160;    // table entries per particle
 
+// The rho pass's block groups: `ntask` tasks (warps) each.
+struct LineGroups {
+	int ntask = 0;
+	std::vector<LineTabs> groups;
+	std::vector<LineTask> tasks;        // groups x ntask (n = 0: none)
+	std::vector<LineIdx> tlines;        // groups x ntask x 16: table offsets of each task's lines
+	int row = 0;                        // most table entries of a group
+	double cycles = 0.0;                // a group's FP64 pipe cycles per particle (its busiest sub-partition), on average
+	int count() const { return (int)groups.size(); }
+};
+
 struct LinePlan {
 	bool ok = false;                    // false: the k-set stays on the segment kernels
 	int nunit = 0;
@@ -118,13 +129,11 @@ struct LinePlan {
 	std::vector<LineIdx> lines;         // rows x 16: (p0, p1, c)
 	std::vector<LineCell> cells;        // nunit x 64, cell ((u * 2 + half) * 32 + 4 (line & 7) + (h & 3))
 	std::vector<double> cellV;          // two weights per cell (plus, minus; 0 where there is no mode)
-	std::vector<LineTabs> groups;       // rho block groups
-	int ntask = 0;                      // tasks (warps) per group: 8, 12 or 16
-	std::vector<LineTask> tasks;        // groups x ntask (n = 0: none)
-	std::vector<LineIdx> tlines;        // groups x ntask x 16: table offsets of each task's lines
+	LineGroups wide;                    // for one configuration: 8 tasks per group (a small set), 12 or 16
+	LineGroups narrow;                  // for blocks of 8 warps when wide's are larger (else empty: wide serves)
+	const LineGroups &groups8() const { return wide.ntask == 8 ? wide : narrow; }
 	std::vector<LineTabs> phases;       // force phases: rows [r0, r0 + ntask) x cells [hlo, hlo + nh)
-	int group_row = 0, phase_row = 0;   // most table entries of a group / phase
-	double group_cycles = 0.0;          // a group's FP64 pipe cycles per particle (its busiest sub-partition), on average
+	int phase_row = 0;                  // most table entries of a phase
 };
 
 // The line plan of a planned k-set. `ok` is false for d = 1, for sets whose lines fill too little of their units to beat

@@ -66,7 +66,7 @@ int main()
 		const Plan p = build_plan(d, M, modes.data(), V.data(), 8);
 		const LinePlan L = build_line_plan(p);
 		std::printf("d=%d M=%ld ok=%d rows=%zu units=%d groups=%zu phases=%zu\n", d, M, (int)L.ok, L.rows.size(), L.nunit,
-		            L.groups.size(), L.phases.size());
+		            L.wide.groups.size(), L.phases.size());
 		if (!L.ok)
 			continue;
 		const int N = 11;   // particles, padded to 12 (rho) and 16 (forces) as the kernels pad theirs
@@ -78,20 +78,22 @@ int main()
 			x ^= x << 17;
 			v = (double)(x >> 11) / 9007199254740992.0;
 		}
-		// rho groups
-		CHECK(L.ntask >= 8 && L.ntask <= 16 && L.ntask % 4 == 0);
-		CHECK(L.tasks.size() == L.groups.size() * L.ntask && L.tlines.size() == L.tasks.size() * kLineRow);
-		std::vector<Z> part((size_t)L.nunit * 128);
+		// rho groups, of one configuration and of blocks of 8 warps
+		std::vector<Z> part;
+		for (const LineGroups *G : {&L.groups8(), &L.wide}) {
+		CHECK(G->ntask >= 8 && G->ntask <= 16 && G->ntask % 4 == 0 && L.groups8().ntask == 8);
+		CHECK(G->tasks.size() == G->groups.size() * G->ntask && G->tlines.size() == G->tasks.size() * kLineRow);
+		part.assign((size_t)L.nunit * 128, Z(NAN, NAN));
 		std::vector<int> wrote(part.size(), 0);
-		for (size_t grp = 0; grp < L.groups.size(); grp++) {
-			const LineTabs &tb = L.groups[grp];
+		for (size_t grp = 0; grp < G->groups.size(); grp++) {
+			const LineTabs &tb = G->groups[grp];
 			CHECK(tb.row % 4 == 2);
 			std::vector<std::vector<Z> > tab;
 			for (int j = 0; j < N; j++)
 				tab.push_back(tables(d, tb, &s[(size_t)j * d]));
 			int active = 0;
-			for (int w = 0; w < L.ntask; w++) {
-				const LineTask task = L.tasks[grp * L.ntask + w];
+			for (int w = 0; w < G->ntask; w++) {
+				const LineTask task = G->tasks[grp * G->ntask + w];
 				CHECK(task.n >= 0 && task.n <= kLineTiles);
 				active += task.n > 0;
 				if (!task.n)
@@ -99,7 +101,7 @@ int main()
 				for (int half = 0; half < 2; half++)
 					for (int lane = 0; lane < 32; lane++) {
 						const int g = lane >> 2, t = lane & 3;
-						const LineIdx l = L.tlines[(grp * L.ntask + w) * kLineRow + half * 8 + g];
+						const LineIdx l = G->tlines[(grp * G->ntask + w) * kLineRow + half * 8 + g];
 						for (int j = 0; j < task.n; j++) {
 							Z A = 0, B = 0;
 							for (int i = 0; i < N; i++) {
@@ -132,6 +134,7 @@ int main()
 		}
 		for (int w : wrote)
 			CHECK(w == 1);
+		}
 		// reduction: every slot with a mode once, equal to the direct sum; weights in place
 		std::vector<Z> u((size_t)p.nslot), wts((size_t)L.nunit * 256, Z(NAN, NAN));
 		std::vector<int> slots((size_t)p.nslot, 0), wset(wts.size(), 0);
