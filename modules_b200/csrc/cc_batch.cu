@@ -4,7 +4,7 @@
 // (cc_mbatch_kernel, cc_kernels.cuh) per energy + gradient step, whose work queue holds the rho blocks, split-reduction
 // chunks and force blocks of every instance; per-instance completion counts order the three phases of an instance.
 // Its batched L-BFGS (cc_batch_minimize) keeps every instance's positions, gradient and history on the device and
-// captures blocks of iterations (one fused evaluation and the L-BFGS kernels each) in CUDA graphs. The reference
+// enqueues blocks of iterations (one fused evaluation and the L-BFGS kernels each). The reference
 // evaluates one configuration per Objective call (potential/StructureOptimization.cpp:447-578).
 #include "cc_internal.h"
 #include "cc_multi_launch.h"
@@ -112,6 +112,7 @@ struct cc_batch {
 	std::vector<BatchBufs> bufs;
 	int per_split = 0, segs_per_split = 0;   // the tile shape in use
 	cudaStream_t stream = nullptr;
+	unsigned char *meta = nullptr;           // one allocation for the arrays down to d_count
 	// the fused launch's descriptors in `order`: set 0 evaluates the batch positions into the batch outputs, set 1 a
 	// minimisation's trial points into its L-BFGS buffers
 	cc::RhoArgs *d_rho[2] = {nullptr, nullptr};
@@ -143,9 +144,15 @@ struct cc_batch {
 	// into the CUDA driver once the batch has run one
 	unsigned char *lb_base = nullptr;
 	size_t lb_cap = 0;
-	cc::LbInst *d_lb = nullptr;              // the instances in `order`
+	cc::LbInst *d_lb = nullptr;              // the instances in `order`, their start values and final positions
+	cc::LbStart *d_start = nullptr;
+	double **d_final = nullptr;
 	cc::LbBrief *d_brief = nullptr;
 	int d_lb_cap = 0;
+	// Host transfers go through one pinned buffer and one copy each way: positions, forces and energies of all instances
+	// are contiguous in the arena (a copy per instance costs 8 to 15 us of driver time).
+	size_t pos_bytes = 0, F_off = 0, F_bytes = 0, E_off = 0;
+	unsigned char *h_pin = nullptr;          // positions, or forces + energies + error word, or status + error word
 };
 
 namespace {
@@ -375,17 +382,90 @@ int batch_eval(cc_batch *b, int set, int precision, cudaStream_t st)
 	return cc::launch_mbatch(mode, batch_args(b, set, mode), b->rho_row, b->force_row, b->maxd, st);
 }
 
-// A bounded wait of the fused kernel that ran out leaves the error word set: report it (after a synchronisation of
-// the batch's stream) and clear it.
+// A bounded wait of the fused kernel that ran out leaves the error word set: `err` is its copy (read after a
+// synchronisation of the batch's stream); report and clear it.
+int batch_check_wait(cc_batch *b, unsigned err)
+{
+	if (err) {
+		CC_CUDA(cudaMemset(b->d_count + 3 * b->order.size(), 0, sizeof(unsigned)));
+		return fail(CC_ERR_TIMEOUT, "a bounded wait of the fused batch kernel ran out");
+	}
+	return CC_OK;
+}
+
 int batch_check_wait(cc_batch *b)
 {
 	unsigned err = 0;
-	const unsigned *w = b->d_count + 3 * b->order.size();
-	CC_CUDA(cudaMemcpy(&err, w, sizeof(unsigned), cudaMemcpyDeviceToHost));
-	if (err) {
-		CC_CUDA(cudaMemset(const_cast<unsigned *>(w), 0, sizeof(unsigned)));
-		return fail(CC_ERR_TIMEOUT, "a bounded wait of the fused batch kernel ran out");
+	CC_CUDA(cudaMemcpy(&err, b->d_count + 3 * b->order.size(), sizeof(unsigned), cudaMemcpyDeviceToHost));
+	return batch_check_wait(b, err);
+}
+
+// The pinned buffer, made once with room for every transfer of the batch (pinning 2 MB takes over a millisecond).
+int batch_pin(cc_batch *b)
+{
+	if (b->h_pin)
+		return CC_OK;
+	const size_t count = b->h.size();
+	const size_t bytes = std::max(b->pos_bytes, std::max(b->F_bytes + count * sizeof(double), count * sizeof(cc::LbBrief)) +
+	                                                sizeof(unsigned));
+	const cudaError_t e = cudaHostAlloc(reinterpret_cast<void **>(&b->h_pin), bytes, cudaHostAllocDefault);
+	if (e != cudaSuccess) {
+		cudaGetLastError();
+		b->h_pin = nullptr;
+		return fail(CC_ERR_OOM, std::string("cudaHostAlloc: ") + cudaGetErrorString(e));
 	}
+	return CC_OK;
+}
+
+// Every instance's coordinates, wrapped into [0, 1) (floor twice), into the pinned buffer at its place among the
+// positions. Coordinates already in [0, 1) are checked and copied in one pass.
+int batch_stage(cc_batch *b, const double *const *frac)
+{
+	if (int rc = batch_pin(b))
+		return rc;
+	for (size_t i = 0; i < b->h.size(); i++) {
+		const size_t n = (size_t)b->N[i] * b->h[i]->d;
+		const double *x = frac[i];
+		double *w = reinterpret_cast<double *>(b->h_pin + (b->off_frac[i] - b->off_frac[0]));
+		long bad = 0;
+		for (size_t k = 0; k < n; k++) {
+			const double v = x[k];
+			w[k] = v;
+			bad |= (long)!(v >= 0.0) | (long)!(v < 1.0);
+		}
+		if (!bad)
+			continue;
+		for (size_t k = 0; k < n; k++) {
+			if (!std::isfinite(x[k]))
+				return fail(CC_ERR_ARG, "non-finite fractional coordinate");
+			const double v = x[k] - std::floor(x[k]);
+			w[k] = v - std::floor(v);
+		}
+	}
+	return CC_OK;
+}
+
+// Energies, the error word and, if F is not null, forces of the evaluation just enqueued on the batch's stream.
+int batch_results(cc_batch *b, double *E, double *const *F)
+{
+	const size_t count = b->h.size(), e_bytes = count * sizeof(double), fb = F ? b->F_bytes : 0;
+	if (int rc = batch_pin(b))
+		return rc;
+	cudaStream_t st = b->stream;
+	if (fb)
+		CC_CUDA(cudaMemcpyAsync(b->h_pin, b->arena.base + b->F_off, fb, cudaMemcpyDeviceToHost, st));
+	CC_CUDA(cudaMemcpyAsync(b->h_pin + fb, b->arena.base + b->E_off, e_bytes, cudaMemcpyDeviceToHost, st));
+	CC_CUDA(cudaMemcpyAsync(b->h_pin + fb + e_bytes, b->d_count + 3 * count, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
+	CC_CUDA(cudaStreamSynchronize(st));
+	unsigned err;
+	std::memcpy(&err, b->h_pin + fb + e_bytes, sizeof(err));
+	if (int rc = batch_check_wait(b, err))
+		return rc;
+	std::memcpy(E, b->h_pin + fb, e_bytes);
+	if (F)
+		for (size_t i = 0; i < count; i++)
+			if (F[i])
+				std::memcpy(F[i], b->h_pin + (b->off_F[i] - b->F_off), sizeof(double) * b->N[i] * b->h[i]->d);
 	return CC_OK;
 }
 
@@ -413,6 +493,16 @@ int cc_batch_create(int count, cc_handle *const *handles, const int64_t *N, cc_b
 	b->off_F.resize(count);
 	b->off_E.resize(count);
 	b->bufs.resize(count);
+	for (int i = 0; i < count; i++)
+		b->off_frac[i] = b->arena.take(sizeof(double) * N[i] * handles[i]->d);
+	b->pos_bytes = b->arena.used - b->off_frac[0];
+	for (int i = 0; i < count; i++)
+		b->off_F[i] = b->arena.take(sizeof(double) * N[i] * handles[i]->d);
+	b->F_off = b->off_F[0];
+	b->F_bytes = b->arena.used - b->F_off;
+	b->E_off = b->arena.take(sizeof(double) * count);
+	for (int i = 0; i < count; i++)
+		b->off_E[i] = b->E_off + sizeof(double) * i;
 	for (int i = 0; i < count; i++) {
 		cc_handle *h = handles[i];
 		const cc::Plan &p = h->main.plan;
@@ -433,9 +523,6 @@ int cc_batch_create(int count, cc_handle *const *handles, const int64_t *N, cc_b
 		const cc::LinePlan &L = h->main.lplan;
 		const size_t row = std::max((size_t)p.nslot, L.ok ? (size_t)L.nunit * 128 : 0);   // entries of a partial row
 		b->any_line |= L.ok;
-		b->off_frac[i] = b->arena.take(sizeof(double) * n * h->d);
-		b->off_F[i] = b->arena.take(sizeof(double) * n * h->d);
-		b->off_E[i] = b->arena.take(sizeof(double));
 		q.o_part = b->arena.take(sizeof(double2) * (size_t)max_nsplit * row);
 		q.o_rho = b->arena.take(sizeof(double2) * p.nslot);
 		q.o_u = b->arena.take(sizeof(double2) * p.nslot);
@@ -466,20 +553,37 @@ int cc_batch_create(int count, cc_handle *const *handles, const int64_t *N, cc_b
 	std::stable_sort(b->order.begin(), b->order.end(), [&](int x, int y) {
 		return (double)N[x] * handles[x]->main.plan.real_segs > (double)N[y] * handles[y]->main.plan.real_segs;
 	});
-	const int B = count;
-	if ((rc = dev_alloc(&b->d_rho[0], B)) || (rc = dev_alloc(&b->d_red[0], B)) || (rc = dev_alloc(&b->d_force[0], B)) ||
-	    (rc = dev_alloc(&b->d_rho[1], B)) || (rc = dev_alloc(&b->d_red[1], B)) || (rc = dev_alloc(&b->d_force[1], B)) ||
-	    (rc = dev_alloc(&b->d_pre, 3 * 4 * (B + 1))) || (rc = dev_alloc(&b->d_shape, 3 * B)) ||
-	    (rc = dev_alloc(&b->d_lrho[0], B)) || (rc = dev_alloc(&b->d_lred[0], B)) ||
-	    (rc = dev_alloc(&b->d_lforce[0], B)) || (rc = dev_alloc(&b->d_lrho[1], B)) ||
-	    (rc = dev_alloc(&b->d_lred[1], B)) || (rc = dev_alloc(&b->d_lforce[1], B)) || (rc = dev_alloc(&b->d_own, 6 * B)) ||
-	    (rc = dev_alloc(&b->d_dim, B)) || (rc = dev_alloc(&b->d_queue, 2)) || (rc = dev_alloc(&b->d_count, 3 * B + 1)) ||
-	    (rc = (cudaMemset(b->d_queue, 0, 2 * sizeof(unsigned)) == cudaSuccess &&
-	                   cudaMemset(b->d_count, 0, (3 * B + 1) * sizeof(unsigned)) == cudaSuccess
-	               ? CC_OK
-	               : fail(CC_ERR_CUDA, "batch initialisation failed")))) {
+	// descriptors, queues and counts: pieces of one allocation, zeroed
+	const size_t B = (size_t)count;
+	size_t used = 0;
+	std::vector<std::pair<void **, size_t> > pieces;
+	auto take = [&](auto **p, size_t n) {
+		pieces.push_back(std::make_pair(reinterpret_cast<void **>(p), used));
+		used += (n * sizeof(**p) + 255) / 256 * 256;
+	};
+	for (int w = 0; w < 2; w++) {
+		take(&b->d_rho[w], B);
+		take(&b->d_red[w], B);
+		take(&b->d_force[w], B);
+		take(&b->d_lrho[w], B);
+		take(&b->d_lred[w], B);
+		take(&b->d_lforce[w], B);
+	}
+	take(&b->d_pre, 3 * 4 * (B + 1));
+	take(&b->d_shape, 3 * B);
+	take(&b->d_own, 6 * B);
+	take(&b->d_dim, B);
+	take(&b->d_queue, 2);
+	take(&b->d_count, 3 * B + 1);
+	if ((rc = dev_alloc(&b->meta, used))) {
 		cc_batch_destroy(b);
 		return rc;
+	}
+	for (const auto &p : pieces)
+		*p.first = b->meta + p.second;
+	if (cudaMemset(b->meta, 0, used) != cudaSuccess) {
+		cc_batch_destroy(b);
+		return fail(CC_ERR_CUDA, "batch initialisation failed");
 	}
 	if ((rc = batch_build(b, kBatchPerSplit, kBatchSegsPerSplit))) {
 		cc_batch_destroy(b);
@@ -543,24 +647,14 @@ int cc_batch_destroy(cc_batch *b)
 		return CC_OK;
 	if (b->stream)
 		cudaStreamSynchronize(b->stream);
-	for (int w = 0; w < 2; w++) {
-		cudaFree(b->d_rho[w]);
-		cudaFree(b->d_red[w]);
-		cudaFree(b->d_force[w]);
-		cudaFree(b->d_lrho[w]);
-		cudaFree(b->d_lred[w]);
-		cudaFree(b->d_lforce[w]);
-	}
-	cudaFree(b->d_own);
-	cudaFree(b->d_dim);
-	cudaFree(b->d_pre);
-	cudaFree(b->d_shape);
-	cudaFree(b->d_queue);
-	cudaFree(b->d_count);
+	cudaFree(b->meta);
 	cudaFree(b->arena.base);
 	cudaFree(b->lb_base);
 	cudaFree(b->d_lb);
 	cudaFree(b->d_brief);
+	cudaFree(b->d_start);
+	cudaFree(b->d_final);
+	cudaFreeHost(b->h_pin);
 	if (b->stream)
 		cudaStreamDestroy(b->stream);
 	delete b;
@@ -571,19 +665,10 @@ int cc_batch_set_positions(cc_batch *b, const double *const *frac)
 {
 	if (!b || !frac)
 		return fail(CC_ERR_ARG, "invalid batch arguments");
-	for (size_t i = 0; i < b->h.size(); i++) {
-		const size_t n = (size_t)b->N[i] * b->h[i]->d;
-		std::vector<double> w(n);
-		for (size_t k = 0; k < n; k++) {
-			if (!std::isfinite(frac[i][k]))
-				return fail(CC_ERR_ARG, "non-finite fractional coordinate");
-			double v = frac[i][k] - std::floor(frac[i][k]);
-			w[k] = v - std::floor(v);
-		}
-		CC_CUDA(cudaMemcpyAsync(b->arena.at<double>(b->off_frac[i]), w.data(), sizeof(double) * n,
-		                        cudaMemcpyHostToDevice, b->stream));
-		CC_CUDA(cudaStreamSynchronize(b->stream));
-	}
+	if (int rc = batch_stage(b, frac))
+		return rc;
+	CC_CUDA(cudaMemcpyAsync(b->arena.base + b->off_frac[0], b->h_pin, b->pos_bytes, cudaMemcpyHostToDevice, b->stream));
+	CC_CUDA(cudaStreamSynchronize(b->stream));
 	return CC_OK;
 }
 
@@ -611,16 +696,7 @@ int cc_batch_energy_grad(cc_batch *b, double *E, double *const *F, int precision
 		return fail(CC_ERR_ARG, "invalid batch arguments");
 	if (int rc = cc_batch_eval_device(b, precision, b->stream))
 		return rc;
-	CC_CUDA(cudaStreamSynchronize(b->stream));
-	if (int rc = batch_check_wait(b))
-		return rc;
-	for (size_t i = 0; i < b->h.size(); i++) {
-		CC_CUDA(cudaMemcpy(&E[i], b->arena.at<double>(b->off_E[i]), sizeof(double), cudaMemcpyDeviceToHost));
-		if (F && F[i])
-			CC_CUDA(cudaMemcpy(F[i], b->arena.at<double>(b->off_F[i]), sizeof(double) * b->N[i] * b->h[i]->d,
-			                   cudaMemcpyDeviceToHost));
-	}
-	return CC_OK;
+	return batch_results(b, E, F);
 }
 
 int cc_batch_minimize(cc_batch *b, double *const *frac, const cc_lbfgs_opts *opts, cc_lbfgs_result *results)
@@ -635,12 +711,6 @@ int cc_batch_minimize(cc_batch *b, double *const *frac, const cc_lbfgs_opts *opt
 	    (o.precision != CC_PREC_FP64 && o.precision != CC_PREC_MIXED && o.precision != CC_PREC_SCHEDULE))
 		return fail(CC_ERR_ARG, "invalid minimisation options");
 	const int count = (int)b->h.size(), m = o.history;
-	for (int i = 0; i < count; i++) {
-		const size_t n = (size_t)b->N[i] * b->h[i]->d;
-		for (size_t k = 0; k < n; k++)
-			if (!std::isfinite(frac[i][k]))
-				return fail(CC_ERR_ARG, "non-finite start");
-	}
 	int maxn = 0;
 	for (int i = 0; i < count; i++)
 		maxn = std::max(maxn, (int)(b->N[i] * b->h[i]->d));
@@ -649,9 +719,13 @@ int cc_batch_minimize(cc_batch *b, double *const *frac, const cc_lbfgs_opts *opt
 	Arena ar;
 	std::vector<size_t> ox(count), og(count), od(count), oxt(count), ogt(count), oS(count), oY(count), op(count),
 	    ost(count);
+	for (int i = 0; i < count; i++)   // laid out as the batch's positions: one copy brings every start
+		ox[i] = ar.take(8 * (size_t)b->N[i] * b->h[i]->d);
+	for (int i = 0; i < count; i++)
+		ost[i] = ar.take(sizeof(cc::LbState));
+	const size_t st_bytes = ar.used - ost[0];
 	for (int i = 0; i < count; i++) {
 		const size_t n = (size_t)b->N[i] * b->h[i]->d;
-		ox[i] = ar.take(8 * n);
 		og[i] = ar.take(8 * n);
 		od[i] = ar.take(8 * n);
 		oxt[i] = ar.take(8 * n);
@@ -659,9 +733,10 @@ int cc_batch_minimize(cc_batch *b, double *const *frac, const cc_lbfgs_opts *opt
 		oS[i] = ar.take(8 * n * m);
 		oY[i] = ar.take(8 * n * m);
 		op[i] = ar.take(8 * (size_t)nblk * cc::lb_ndots(m));
-		ost[i] = ar.take(sizeof(cc::LbState));
 	}
 	int rc;
+	if ((rc = batch_stage(b, frac)))   // (a non-finite start changes nothing)
+		return rc;
 	if (b->lb_cap < ar.used) {
 		cudaFree(b->lb_base);
 		b->lb_base = nullptr;
@@ -673,28 +748,23 @@ int cc_batch_minimize(cc_batch *b, double *const *frac, const cc_lbfgs_opts *opt
 	if (b->d_lb_cap < count) {
 		cudaFree(b->d_lb);
 		cudaFree(b->d_brief);
+		cudaFree(b->d_start);
+		cudaFree(b->d_final);
 		b->d_lb = nullptr;
 		b->d_brief = nullptr;
+		b->d_start = nullptr;
+		b->d_final = nullptr;
 		b->d_lb_cap = 0;
-		if ((rc = dev_alloc(&b->d_lb, (size_t)count)) || (rc = dev_alloc(&b->d_brief, count)))
+		if ((rc = dev_alloc(&b->d_lb, (size_t)count)) || (rc = dev_alloc(&b->d_brief, count)) ||
+		    (rc = dev_alloc(&b->d_start, count)) || (rc = dev_alloc(&b->d_final, count)))
 			return rc;
 		b->d_lb_cap = count;
 	}
 	ar.base = b->lb_base;
 	std::vector<cc::LbInst> lbi(count);   // by instance index
-	cc::LbState s0;
-	std::memset(&s0, 0, sizeof(s0));
-	s0.E = INFINITY;
-	s0.gamma = 1.0;
-	s0.gtol = o.gtol;
-	s0.ftol = o.ftol;
-	s0.max_evals = o.max_evals;
-	s0.m = m;
-	s0.newslot = -1;
 	for (int i = 0; i < count; i++) {
-		const size_t n = (size_t)b->N[i] * b->h[i]->d;
 		cc::LbInst &l = lbi[i];
-		l.n = (int)n;
+		l.n = (int)(b->N[i] * b->h[i]->d);
 		l.m = m;
 		l.x = ar.at<double>(ox[i]);
 		l.g = ar.at<double>(og[i]);
@@ -705,24 +775,12 @@ int cc_batch_minimize(cc_batch *b, double *const *frac, const cc_lbfgs_opts *opt
 		l.Y = ar.at<double>(oY[i]);
 		l.part = ar.at<double>(op[i]);
 		l.st = ar.at<cc::LbState>(ost[i]);
-		std::vector<double> x0(n);
-		for (size_t k = 0; k < n; k++) {
-			double v = frac[i][k] - std::floor(frac[i][k]);
-			x0[k] = v - std::floor(v);
-		}
-		CC_CUDA(cudaMemcpy(l.x, x0.data(), 8 * n, cudaMemcpyHostToDevice));
-		CC_CUDA(cudaMemcpy(l.xt, x0.data(), 8 * n, cudaMemcpyHostToDevice));
-		CC_CUDA(cudaMemset(l.g, 0, 8 * n));
-		CC_CUDA(cudaMemset(l.d, 0, 8 * n));
-		s0.stopval = o.stopval == CC_STOPVAL_GROUND_STATE ? 1e-20 * (double)b->N[i] : o.stopval;
-		s0.sched = o.precision == CC_PREC_SCHEDULE;
-		s0.stage = o.precision == CC_PREC_FP64 ? 1 : 0;
-		s0.switch_E = o.switch_energy_per_particle * (double)b->N[i];
-		CC_CUDA(cudaMemcpy(l.st, &s0, sizeof(s0), cudaMemcpyHostToDevice));
 	}
 	// the L-BFGS instances in the launch order, and the minimisation descriptors (set 1): evaluate at x_trial into
 	// the L-BFGS buffers, skip finished instances
 	std::vector<cc::LbInst> lbo(count);
+	std::vector<cc::LbStart> start(count);
+	std::vector<double *> final_pos(count);
 	std::vector<cc::RhoArgs> ra = b->rho;
 	std::vector<cc::ReduceArgs> rr = b->red;
 	std::vector<cc::ForceArgs> fa = b->force;
@@ -732,6 +790,9 @@ int cc_batch_minimize(cc_batch *b, double *const *frac, const cc_lbfgs_opts *opt
 	for (int k = 0; k < count; k++) {
 		const int i = b->order[k];
 		lbo[k] = lbi[i];
+		start[k].stopval = o.stopval == CC_STOPVAL_GROUND_STATE ? 1e-20 * (double)b->N[i] : o.stopval;
+		start[k].switch_E = o.switch_energy_per_particle * (double)b->N[i];
+		final_pos[k] = b->arena.at<double>(b->off_frac[i]);
 		const int *status = &lbi[i].st->status, *stage = &lbi[i].st->stage;
 		ra[k].frac = lbi[i].xt;
 		ra[k].skip = status;
@@ -757,73 +818,60 @@ int cc_batch_minimize(cc_batch *b, double *const *frac, const cc_lbfgs_opts *opt
 	    (rc = upload_into(b->d_force[1], fa)) || (rc = upload_into(b->d_lrho[1], lra)) ||
 	    (rc = upload_into(b->d_lred[1], lrr)) || (rc = upload_into(b->d_lforce[1], lfa)))
 		return rc;
+	if ((rc = upload_into(b->d_start, start)) || (rc = upload_into(b->d_final, final_pos)))
+		return rc;
 	cudaStream_t st = b->stream;
 	const bool sched = o.precision == CC_PREC_SCHEDULE;
-	// schedule: each instance at its stage's precision while some instance is in the mixed stage; then FP64 only
-	auto iterations = [&](int prec) -> int {
-		for (int it = 0; it < o.iters_per_check; it++) {
+	CC_CUDA(cudaMemcpyAsync(b->lb_base + ox[0], b->h_pin, b->pos_bytes, cudaMemcpyHostToDevice, st));
+	CC_CUDA(cudaMemsetAsync(b->lb_base + ost[0], 0, st_bytes, st));
+	const dim3 all((maxn + 255) / 256, count);
+	cc::lb_start_kernel<<<all, 256, 0, st>>>(b->d_lb, b->d_start, o.gtol, o.ftol, o.max_evals,
+	                                         o.precision == CC_PREC_FP64 ? 1 : 0, sched ? 1 : 0);
+	CC_CUDA(cudaGetLastError());
+	// A block of iterations is enqueued kernel by kernel: an iteration keeps the GPU busy for far longer (40 us and more)
+	// than its four launches take, and capturing a graph of them on every call cost 2 ms. Schedule: each instance at its
+	// stage's precision while some instance is in the mixed stage; then FP64 only.
+	auto iterations = [&](int prec, int count_it) -> int {
+		for (int it = 0; it < count_it; it++) {
 			if (int r2 = batch_eval(b, 1, prec, st))
 				return r2;
 			CC_CUDA(cc::lb_step(b->d_lb, count, nblk, maxn, st, count == 1 ? &lbo[0] : nullptr));
-			CC_CUDA(cudaGetLastError());
 		}
 		return CC_OK;
 	};
-	auto make_graph = [&](int prec, cudaGraphExec_t *out) -> int {
-		cudaGraph_t g = nullptr;
-		CC_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-		const int r2 = iterations(prec);
-		cudaError_t e = cudaStreamEndCapture(st, &g);
-		if (r2)
-			return r2;
-		if (e != cudaSuccess)
-			return fail(CC_ERR_CUDA, std::string("cudaStreamEndCapture: ") + cudaGetErrorString(e));
-		e = cudaGraphInstantiate(out, g, 0);
-		cudaGraphDestroy(g);
-		if (e != cudaSuccess)
-			return fail(CC_ERR_CUDA, std::string("cudaGraphInstantiate: ") + cudaGetErrorString(e));
-		return CC_OK;
-	};
-	cudaGraphExec_t gexec[2] = {nullptr, nullptr};
-	auto destroy_graphs = [&]() {
-		for (auto &ge : gexec)
-			if (ge)
-				cudaGraphExecDestroy(ge);
-	};
-	// kernel attributes and occupancy are looked up outside the capture: one eager evaluation of every mode in use
-	if ((rc = batch_eval(b, 0, o.precision, st)) || (sched && (rc = batch_eval(b, 0, CC_PREC_FP64, st))))
-		return rc;
-	CC_CUDA(cudaStreamSynchronize(st));
-	if ((rc = make_graph(o.precision, &gexec[0])) || (sched && (rc = make_graph(CC_PREC_FP64, &gexec[1])))) {
-		destroy_graphs();
-		return rc;
-	}
 	std::vector<cc::LbBrief> hs(count);   // in launch order
+	const size_t hs_bytes = sizeof(cc::LbBrief) * count;
+	CC_CUDA(cudaStreamSynchronize(st));   // the staged starts are out of the pinned buffer
 	int stage = 0;
+	int64_t left = o.max_evals;   // an instance still running has made one evaluation per iteration
 	const int64_t max_rounds = o.max_evals / o.iters_per_check + 2;
 	for (int64_t round = 0; round < max_rounds; round++) {
-		cudaError_t e = cudaGraphLaunch(gexec[stage], st);
-		if (e == cudaSuccess)
-			e = cudaStreamSynchronize(st);
-		if (e != cudaSuccess) {
-			destroy_graphs();
-			return fail(CC_ERR_CUDA, std::string("batch minimisation: ") + cudaGetErrorString(e));
-		}
-		if ((rc = batch_check_wait(b))) {
-			destroy_graphs();
-			return rc;
-		}
+		const int its = (int)std::max<int64_t>(1, std::min<int64_t>(o.iters_per_check, left));
+		left -= its;
+		rc = iterations(stage ? CC_PREC_FP64 : o.precision, its);
 		bool running = false, any_mixed = false;
-		cc::lb_brief_kernel<<<(count + 127) / 128, 128, 0, st>>>(b->d_lb, count, b->d_brief);
-		e = cudaGetLastError();
-		if (e == cudaSuccess)
-			e = cudaMemcpyAsync(hs.data(), b->d_brief, sizeof(cc::LbBrief) * count, cudaMemcpyDeviceToHost, st);
-		if (e == cudaSuccess)
-			e = cudaStreamSynchronize(st);
-		if (e != cudaSuccess) {
-			destroy_graphs();
-			return fail(CC_ERR_CUDA, std::string("batch minimisation status: ") + cudaGetErrorString(e));
+		cudaError_t e = cudaSuccess;
+		if (!rc) {
+			cc::lb_brief_kernel<<<(count + 127) / 128, 128, 0, st>>>(b->d_lb, count, b->d_brief);
+			e = cudaGetLastError();
+			if (e == cudaSuccess)
+				e = cudaMemcpyAsync(b->h_pin, b->d_brief, hs_bytes, cudaMemcpyDeviceToHost, st);
+			if (e == cudaSuccess)
+				e = cudaMemcpyAsync(b->h_pin + hs_bytes, b->d_count + 3 * count, sizeof(unsigned), cudaMemcpyDeviceToHost,
+				                    st);
 		}
+		const cudaError_t es = cudaStreamSynchronize(st);
+		if (rc)
+			return rc;
+		if (e == cudaSuccess)
+			e = es;
+		if (e != cudaSuccess)
+			return fail(CC_ERR_CUDA, std::string("batch minimisation: ") + cudaGetErrorString(e));
+		unsigned err;
+		std::memcpy(&err, b->h_pin + hs_bytes, sizeof(err));
+		if ((rc = batch_check_wait(b, err)))
+			return rc;
+		std::memcpy(hs.data(), b->h_pin, hs_bytes);
 		for (int k = 0; k < count; k++) {
 			running |= hs[k].status == cc::kLbRunning;
 			any_mixed |= hs[k].status == cc::kLbRunning && hs[k].stage == 0;
@@ -833,23 +881,16 @@ int cc_batch_minimize(cc_batch *b, double *const *frac, const cc_lbfgs_opts *opt
 		if (sched && stage == 0 && !any_mixed)
 			stage = 1;
 	}
-	destroy_graphs();
-	// results: positions wrapped into [0,1), FP64 energies of the results (one batched evaluation)
-	std::vector<const double *> fr(count);
-	for (int i = 0; i < count; i++) {
-		const size_t n = (size_t)b->N[i] * b->h[i]->d;
-		CC_CUDA(cudaMemcpy(frac[i], lbi[i].x, 8 * n, cudaMemcpyDeviceToHost));
-		for (size_t k = 0; k < n; k++) {
-			double v = frac[i][k] - std::floor(frac[i][k]);
-			frac[i][k] = v - std::floor(v);
-		}
-		fr[i] = frac[i];
-	}
-	if ((rc = cc_batch_set_positions(b, fr.data())))
-		return rc;
+	// results: positions wrapped into [0,1) become the bound ones, FP64 energies of the results (one batched evaluation)
+	cc::lb_finish_kernel<<<all, 256, 0, st>>>(b->d_lb, b->d_final);
+	CC_CUDA(cudaGetLastError());
 	std::vector<double> E(count);
-	if ((rc = cc_batch_energy_grad(b, E.data(), nullptr, CC_PREC_FP64)))
+	if ((rc = batch_eval(b, 0, CC_PREC_FP64, st)) || (rc = batch_results(b, E.data(), nullptr)))
 		return rc;
+	CC_CUDA(cudaMemcpyAsync(b->h_pin, b->arena.base + b->off_frac[0], b->pos_bytes, cudaMemcpyDeviceToHost, st));
+	CC_CUDA(cudaStreamSynchronize(st));
+	for (int i = 0; i < count; i++)
+		std::memcpy(frac[i], b->h_pin + (b->off_frac[i] - b->off_frac[0]), sizeof(double) * b->N[i] * b->h[i]->d);
 	if (results)
 		for (int k = 0; k < count; k++) {
 			const int i = b->order[k];

@@ -103,9 +103,9 @@ int cci::upload_kset(DevKSet &k, const cc::Plan &plan)
 	auto room = [](size_t bytes) { return (bytes + 255) / 256 * 256; };
 	auto put = [&](const void *p, size_t bytes) {
 		const size_t at = up.size();
-		up.resize(at + room(bytes));
-		if (bytes)
-			std::memcpy(up.data() + at, p, bytes);
+		const unsigned char *s = static_cast<const unsigned char *>(p);
+		up.insert(up.end(), s, s + bytes);
+		up.resize(room(up.size()));
 		return at;
 	};
 #define CC_PUT(v) put((v).data(), (v).size() * sizeof((v)[0]))

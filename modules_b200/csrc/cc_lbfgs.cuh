@@ -692,6 +692,51 @@ static __global__ void lb_brief_kernel(const LbInst *insts, int count, LbBrief *
 	}
 }
 
+// Start of a batched minimisation: instance blockIdx.y begins at x (already in place), with xt = x, zero gradient and
+// direction and, in its (zeroed) state, a virtual previous point of infinite energy, so that the first evaluation is
+// always accepted.
+struct LbStart {
+	double stopval, switch_E;       // per instance
+};
+static __global__ void lb_start_kernel(const LbInst *insts, const LbStart *start, double gtol, double ftol,
+                                       int64_t max_evals, int stage, int sched)
+{
+	const LbInst in = insts[blockIdx.y];
+	const int j = blockIdx.x * blockDim.x + threadIdx.x;
+	if (j < in.n) {
+		in.xt[j] = in.x[j];
+		in.g[j] = 0.0;
+		in.d[j] = 0.0;
+	}
+	if (j == 0) {
+		LbState *s = in.st;
+		const LbStart w = start[blockIdx.y];
+		s->E = INFINITY;
+		s->gamma = 1.0;
+		s->stopval = w.stopval;
+		s->gtol = gtol;
+		s->ftol = ftol;
+		s->max_evals = max_evals;
+		s->m = in.m;
+		s->newslot = -1;
+		s->stage = stage;
+		s->sched = sched;
+		s->switch_E = w.switch_E;
+	}
+}
+
+// End of a batched minimisation: every instance's point, wrapped into [0, 1) as cc_set_positions wraps, to out[blockIdx.y].
+static __global__ void lb_finish_kernel(const LbInst *insts, double *const *out)
+{
+	const LbInst in = insts[blockIdx.y];
+	const int j = blockIdx.x * blockDim.x + threadIdx.x;
+	if (j >= in.n)
+		return;
+	double v = in.x[j] - floor(in.x[j]);
+	v -= floor(v);
+	out[blockIdx.y][j] = v;
+}
+
 // The three kernels of one L-BFGS step on stream st for `count` instances (insts), at most `cap` dot-product blocks
 // per instance and `maxn` variables in the largest one. Each is launched with programmatic stream serialisation:
 // it is scheduled while the previous kernel drains and waits for it (cudaGridDependencySynchronize) before it reads.
