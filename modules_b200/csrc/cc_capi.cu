@@ -15,6 +15,8 @@
 #include "cc_nufft.cuh"
 #include "cc_plan.h"
 
+#include <immintrin.h>
+
 #include <algorithm>
 #include <cmath>
 #include <cstddef>
@@ -1434,6 +1436,20 @@ int launch_eval_graph(cc_handle *h, int64_t N, int precision, int forces, bool *
 	return CC_OK;
 }
 
+// Wait until a kernel has written `number` to mapped host memory: a short look at the word, which the host sees about 4 us
+// before a stream synchronisation returns. False when it does not come soon (a busy GPU, an error): synchronise then.
+bool wait_number(const volatile unsigned long long *word, unsigned long long number)
+{
+	for (int i = 0; i < 20000; i++) {
+		if (*word == number) {
+			std::atomic_thread_fence(std::memory_order_acquire);
+			return true;
+		}
+		_mm_pause();
+	}
+	return false;
+}
+
 template <typename T> __global__ void fma_probe_kernel(T *out, int iters, T a, T b)
 {
 	T x[8];
@@ -2085,6 +2101,7 @@ int cc_mc_try_move(cc_handle *h, const double *s_prev, const double *s_after, do
 		    (rc = dev_alloc(&h->d_rho_trial, M)) || (rc = dev_alloc(&h->d_rho_cur, M)) ||
 		    (rc = dev_alloc(&h->d_mc_part, nb + 1)))
 			return rc;
+		CC_CUDA(cudaMemset(h->d_mc_part, 0, (nb + 1) * sizeof(double)));   // [nb]: the blocks' ticket
 	}
 	if (!h->mc_valid) {
 		// rho of the bound positions in mode order (FP64), as the cached RhoReal / RhoImag of the reference
@@ -2102,12 +2119,17 @@ int cc_mc_try_move(cc_handle *h, const double *s_prev, const double *s_after, do
 		sp[c] = s_prev[c];
 		sa[c] = s_after[c];
 	}
-	cc::cc_mc_kernel<<<nb, cc::kMcThreads, 0, h->stream>>>(h->d_modes, d, h->d_modeV, h->d_rho_cur, M, sp[0], sp[1],
-	                                                        sp[2], sa[0], sa[1], sa[2], h->d_rho_trial, h->d_mc_part);
-	cc::cc_mc_sum_kernel<<<1, 32, 0, h->stream>>>(h->d_mc_part, nb, 1.0 / h->volume, h->d_mc_part + nb);
+	// the kernel writes dE and then the move's number into the mapped result buffer ([0] and [1], which the forces leave free)
+	volatile unsigned long long *done = reinterpret_cast<volatile unsigned long long *>(h->h_pin + 1);
+	const unsigned long long number = ++h->mc_number;
+	*done = 0;
+	cc::cc_mc_kernel<<<nb, cc::kMcThreads, 0, h->stream>>>(
+	    h->d_modes, d, h->d_modeV, h->d_rho_cur, M, sp[0], sp[1], sp[2], sa[0], sa[1], sa[2], h->d_rho_trial,
+	    h->d_mc_part, reinterpret_cast<unsigned *>(h->d_mc_part + nb), 1.0 / h->volume, h->d_pin,
+	    reinterpret_cast<unsigned long long *>(h->d_pin + 1), number);
 	CC_CUDA(cudaGetLastError());
-	CC_CUDA(cudaMemcpyAsync(h->h_pin, h->d_mc_part + nb, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-	CC_CUDA(cudaStreamSynchronize(h->stream));
+	if (!wait_number(done, number))
+		CC_CUDA(cudaStreamSynchronize(h->stream));
 	*dE = h->h_pin[0];
 	h->mc_pending = true;
 	return CC_OK;

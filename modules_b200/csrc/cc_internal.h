@@ -282,6 +282,7 @@ struct cc_handle {
 	double2 *d_rho_trial = nullptr, *d_rho_cur = nullptr;
 	double *d_mc_part = nullptr;
 	bool mc_valid = false, mc_pending = false;
+	unsigned long long mc_number = 0;   // trial moves made
 	const int *d_skip = nullptr;    // evaluations do nothing while *d_skip != 0 (set by cc_minimize)
 	bool timing = false;            // cc_set_timing
 	bool independent = false;       // cc_set_independent_positions

@@ -1305,7 +1305,9 @@ __global__ void __launch_bounds__(kMBatchThreads, 3) cc_mbatch_kernel(MBatchArgs
 // ---------------------------------------------------------------------------------------------------------------
 // rho'(k) = rho(k) - exp(i k.r_prev) + exp(i k.r_after); dE = sum_k V (|rho'|^2 - |rho|^2) / Volume, with the change
 // formed as 2 Re(conj(rho) delta) + |delta|^2 (no cancellation between two whole energies). Block partial sums in a
-// fixed order; cc_mc_sum_kernel adds the blocks in order.
+// fixed order; the last block to finish (a ticket, no wait) adds them in a fixed order and writes dE and then the move's
+// number into mapped host memory. What bounds it is latency: one kernel whose result the host sees as soon as it is
+// written takes 11 us a move at M = 2724, a second kernel for the sum, a copy and a stream synchronisation took 23.
 constexpr int kMcThreads = 256;
 
 static __global__ void __launch_bounds__(kMcThreads) cc_mc_kernel(const int32_t *__restrict__ modes, int D,
@@ -1313,13 +1315,18 @@ static __global__ void __launch_bounds__(kMcThreads) cc_mc_kernel(const int32_t 
                                                                   const double2 *__restrict__ rho, int M, double sp0,
                                                                   double sp1, double sp2, double sa0, double sa1,
                                                                   double sa2, double2 *__restrict__ rho_trial,
-                                                                  double *__restrict__ bpart)
+                                                                  double *bpart, unsigned *ticket, double inv_vol,
+                                                                  volatile double *out, volatile unsigned long long *done,
+                                                                  unsigned long long number)
 {
 	__shared__ double sh[kMcThreads / 32];
+	__shared__ int sh_last;
 	const int m = blockIdx.x * kMcThreads + threadIdx.x;
 	double e = 0.0;
 	if (m < M) {
 		const double sp[3] = {sp0, sp1, sp2}, sa[3] = {sa0, sa1, sa2};
+		const double2 r = rho[m];
+		const double v = V[m];
 		double hp = 0, lp = 0, ha = 0, la = 0;
 		for (int c = 0; c < D; c++) {
 			const int n = modes[(size_t)m * D + c];
@@ -1330,10 +1337,9 @@ static __global__ void __launch_bounds__(kMcThreads) cc_mc_kernel(const int32_t 
 		tp = __dsub_rn(tp, rint(tp));
 		ta = __dsub_rn(ta, rint(ta));
 		const double2 zp = expi2pi(tp), za = expi2pi(ta);
-		const double2 r = rho[m];
 		const double2 dl = make_double2(za.x - zp.x, za.y - zp.y);
 		rho_trial[m] = make_double2(r.x + dl.x, r.y + dl.y);
-		e = V[m] * (2.0 * (r.x * dl.x + r.y * dl.y) + dl.x * dl.x + dl.y * dl.y);
+		e = v * (2.0 * (r.x * dl.x + r.y * dl.y) + dl.x * dl.x + dl.y * dl.y);
 	}
 	for (int o = 16; o > 0; o >>= 1)
 		e += __shfl_down_sync(0xffffffffu, e, o);
@@ -1345,6 +1351,23 @@ static __global__ void __launch_bounds__(kMcThreads) cc_mc_kernel(const int32_t 
 		for (int w = 0; w < kMcThreads / 32; w++)
 			t += sh[w];
 		bpart[blockIdx.x] = t;
+		__threadfence();
+		sh_last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+	}
+	__syncthreads();
+	if (!sh_last || threadIdx.x >= 32)
+		return;
+	__threadfence();
+	double t = 0.0;
+	for (int b = threadIdx.x; b < (int)gridDim.x; b += 32)
+		t += __ldcg(bpart + b);
+	for (int o = 16; o > 0; o >>= 1)
+		t += __shfl_down_sync(0xffffffffu, t, o);
+	if (threadIdx.x == 0) {
+		*ticket = 0u;
+		*out = t * inv_vol;
+		__threadfence_system();
+		*done = number;
 	}
 }
 

@@ -85,3 +85,35 @@ def test_sets_that_stay_on_the_segment_kernels(gpu):
         Eo, Fo, _, _ = oracle.port_eval(d, np.eye(d), frac, k, V)
         assert abs(E - Eo) <= 1e-12 * V.sum() * 257 ** 2
         assert np.abs(F - Fo).max() <= 1e-12 * 4 * V.sum() * 257 * np.sqrt((np.asarray(k) ** 2).sum(1)).max()
+
+
+@pytest.mark.parametrize("d,M", [(1, 1), (2, 255), (2, 256), (3, 257), (3, 8193)])
+def test_mc_moves_against_whole_energies(gpu, d, M):
+    """Trial moves at the edges of the kernel's blocks of 256 modes and beyond 32 blocks: dE is the difference of the whole
+    energies (to their rounding, 1e-12 of the energy scale), accepted moves accumulate, and an evaluation in between (which
+    writes the same result buffer) changes nothing."""
+    rng = np.random.default_rng(M)
+    modes = rng.integers(-9, 10, (M, d))
+    V = rng.uniform(0, 1, M)
+    N = 40
+    frac = rng.random((N, d))
+    p = gpu.CCPotential(d, np.eye(d), modes, V)
+    q = gpu.CCPotential(d, np.eye(d), modes, V)
+    p.set_configuration(frac)
+    q.set_configuration(frac)
+    E = q.energy()
+    cur = frac.copy()
+    for step in range(6):
+        j = int(rng.integers(N))
+        new = rng.random(d)
+        dE = p.try_move(cur[j], new)
+        assert p.try_move(cur[j], new) == dE   # a second trial of the same move repeats bitwise
+        trial = cur.copy()
+        trial[j] = new
+        q.set_configuration(trial)
+        assert abs(dE - (q.energy() - E)) <= 1e-12 * V.sum() * N * N
+        if step % 2 == 0:
+            p.accept_move()
+            cur, E = trial, q.energy()
+        if step == 3:
+            p.energy_and_forces()
