@@ -2013,28 +2013,35 @@ int cc_structure_factor(cc_handle *h, int64_t K, const int32_t *modes, double *S
 			S[q] = std::nan("");
 		return CC_OK;
 	}
-	std::vector<int32_t> key(modes, modes + K * h->d);
-	if (key != h->sk_modes || h->sk.segs == nullptr) {
+	if (h->sk.segs == nullptr || (size_t)(K * h->d) != h->sk_modes.size() ||
+	    std::memcmp(modes, h->sk_modes.data(), sizeof(int32_t) * K * h->d) != 0) {
 		std::vector<double> ones((size_t)K, 1.0);
 		cc::Plan plan = cc::build_plan(h->d, K, modes, ones.data(), 8);
 		if (int rc = upload_kset(h->sk, plan))
 			return rc;
-		h->sk_modes = key;
+		h->sk_modes.assign(modes, modes + K * h->d);
 	}
 	if (int rc = flush_upload(h))
 		return rc;
 	const Launch l = choose_launch(h->sk, N, precision == CC_PREC_MIXED);
 	const double save_off = h->rho_offset;
 	h->rho_offset = 0.0;   // S(k) of the particles themselves (StructureFactor has no fixed-particle offset)
-	int rc = run_rho(h, h->sk, N, h->d_frac, h->d_E + 1, true, precision == CC_PREC_MIXED, l, h->stream);
+	int rc = run_rho(h, h->sk, N, h->d_frac, h->d_E + 1, false, precision == CC_PREC_MIXED, l, h->stream);
 	h->rho_offset = save_off;
 	if (rc)
 		return rc;
-	std::vector<double2> tmp((size_t)K);
-	CC_CUDA(cudaMemcpyAsync(tmp.data(), h->sk.rho_mode, sizeof(double2) * K, cudaMemcpyDeviceToHost, h->stream));
+	// S(k) leaves the GPU through the pinned result buffer where it fits and holds no forces, else through the k-set's own
+	// buffer and a pageable copy
+	const bool pinned = !h->lastF_valid && (size_t)K + 2 <= h->pin_cap;
+	double *out = pinned ? h->d_pin + 2 : reinterpret_cast<double *>(h->sk.rho_mode);
+	cc::cc_gather_sk_kernel<<<(unsigned)((K + 255) / 256), 256, 0, h->stream>>>(h->sk.rho_slot, h->sk.mode_slot, (int)K,
+	                                                                        (double)N, out);
+	CC_CUDA(cudaGetLastError());
+	if (!pinned)
+		CC_CUDA(cudaMemcpyAsync(S, out, sizeof(double) * K, cudaMemcpyDeviceToHost, h->stream));
 	CC_CUDA(cudaStreamSynchronize(h->stream));
-	for (int64_t q = 0; q < K; q++)
-		S[q] = (tmp[q].x * tmp[q].x + tmp[q].y * tmp[q].y) / (double)N;
+	if (pinned)
+		std::memcpy(S, h->h_pin + 2, sizeof(double) * K);
 	return CC_OK;
 }
 

@@ -797,6 +797,17 @@ static __global__ void cc_gather_rho_kernel(const double2 *__restrict__ rho_slot
 		rho_mode[m] = rho_slot[mode_slot[m]];
 }
 
+// S = |rho|^2 / n in input-mode order, straight to its destination (device or mapped host memory)
+static __global__ void cc_gather_sk_kernel(const double2 *__restrict__ rho_slot, const int *__restrict__ mode_slot, int M,
+                                           double n, double *__restrict__ S)
+{
+	const int m = blockIdx.x * blockDim.x + threadIdx.x;
+	if (m < M) {
+		const double2 r = rho_slot[mode_slot[m]];
+		S[m] = (r.x * r.x + r.y * r.y) / n;
+	}
+}
+
 // E = shift when there is no constraint
 static __global__ void cc_set_scalar_kernel(double *p, double v) { *p = v; }
 
