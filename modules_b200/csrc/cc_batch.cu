@@ -266,14 +266,14 @@ int batch_build(cc_batch *b, int per_split, int segs_per_split)
 			lr.frac = ra.frac;
 			lr.N = ra.N;
 			lr.per_split = per_split;
-			lr.chunk = batch_line_chunk(L.groups8(), per_split);
+			lr.chunk = batch_line_chunk(L.groupings[0], per_split);
 			lr.log2chunk = __builtin_ctz((unsigned)lr.chunk);
-			lr.ngroup = L.groups8().count();
+			lr.ngroup = L.groupings[0].count();
 			lr.nunit = L.nunit;
 			lr.ntask = cc::kLineTasks;
-			lr.groups = dl.narrow.groups;
-			lr.tasks = dl.narrow.tasks;
-			lr.tlines = dl.narrow.tlines;
+			lr.groups = dl.groups[0].groups;
+			lr.tasks = dl.groups[0].tasks;
+			lr.tlines = dl.groups[0].tlines;
 			lr.partial = ra.partial;
 			ld.partial = lr.partial;
 			ld.nsplit = nsplit;
@@ -303,7 +303,7 @@ int batch_build(cc_batch *b, int per_split, int segs_per_split)
 			const int lc[3] = {lr.ngroup * nsplit, lf.neblock, (int)((n + 8 * cc::kLineBatchMT - 1) / (8 * cc::kLineBatchMT))};
 			for (int ph = 0; ph < 3; ph++)
 				own[(3 + ph) * B + k] = lc[ph];
-			b->line_smem = std::max(b->line_smem, std::max(cc::line_rho_smem(L.groups8().row, lr.chunk, h->d),
+			b->line_smem = std::max(b->line_smem, std::max(cc::line_rho_smem(L.groupings[0].row, lr.chunk, h->d),
 			                                               cc::line_force_smem(L.phase_row, cc::kLineBatchMT, 8, h->d)));
 		}
 		b->lrho.push_back(lr);

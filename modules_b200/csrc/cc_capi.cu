@@ -115,12 +115,13 @@ int cci::upload_kset(DevKSet &k, const cc::Plan &plan)
 	             o_slotV = CC_PUT(plan.slotV), o_mode = CC_PUT(plan.mode_slot);
 	const size_t o_rows = CC_PUT(L.rows), o_lines = CC_PUT(L.lines), o_cells = CC_PUT(L.cells), o_cellV = CC_PUT(L.cellV),
 	             o_phases = CC_PUT(L.phases);
-	const cc::LineGroups *lg[2] = {&L.wide, &L.narrow};
-	size_t o_groups[2], o_tasks[2], o_tlines[2];
-	for (int i = 0; i < 2; i++) {
-		o_groups[i] = CC_PUT(lg[i]->groups);
-		o_tasks[i] = CC_PUT(lg[i]->tasks);
-		o_tlines[i] = CC_PUT(lg[i]->tlines);
+	struct Offsets {
+		size_t groups, tasks, tlines;
+	};
+	std::vector<Offsets> og;
+	for (const cc::LineGroups &g : L.groupings) {
+		const size_t a = CC_PUT(g.groups), b = CC_PUT(g.tasks), c = CC_PUT(g.tlines);
+		og.push_back({a, b, c});
 	}
 #undef CC_PUT
 	const size_t nslot = plan.slotV.size(), M = plan.mode_slot.size();
@@ -155,14 +156,9 @@ int cci::upload_kset(DevKSet &k, const cc::Plan &plan)
 	k.line.cells = reinterpret_cast<cc::LineCell *>(b + o_cells);
 	k.line.cellV = reinterpret_cast<double2 *>(b + o_cellV);
 	k.line.phases = reinterpret_cast<cc::LineTabs *>(b + o_phases);
-	DevLines::Groups *dg[2] = {&k.line.wide, &k.line.narrow};
-	for (int i = 0; i < 2; i++) {
-		dg[i]->groups = reinterpret_cast<cc::LineTabs *>(b + o_groups[i]);
-		dg[i]->tasks = reinterpret_cast<cc::LineTask *>(b + o_tasks[i]);
-		dg[i]->tlines = reinterpret_cast<cc::LineIdx *>(b + o_tlines[i]);
-	}
-	if (L.narrow.ntask == 0)
-		k.line.narrow = k.line.wide;
+	for (const Offsets &o : og)
+		k.line.groups.push_back({reinterpret_cast<cc::LineTabs *>(b + o.groups), reinterpret_cast<cc::LineTask *>(b + o.tasks),
+		                         reinterpret_cast<cc::LineIdx *>(b + o.tlines)});
 	k.line.weights = reinterpret_cast<double2 *>(b + o_w);
 	k.line.eblock = reinterpret_cast<double *>(b + o_leb);
 	return CC_OK;
@@ -198,55 +194,64 @@ double grid_cost(int64_t blocks, int wave, double pairs, double fixed_pairs)
 	return (double)waves * (1.0 + pairs / (double)blocks / fixed_pairs);
 }
 
-// The line kernels' grids (B200, CUDA graphs of evaluations, sweeps over 2D and 3D sets of N = 300 to 100000).
-// rho: particle splits (multiples of 8 particles) with the least estimated time: whole waves of blocks, a block's fixed cost
-// (loads, the tables' latency) and its matrix work at 70 % of the pipe, plus the partial rows, which cross L2 twice: 3D
-// N=2000 chi=0.45 takes 6.9 us with 84 splits of 24 particles, 7.9 with 125 of 16 and 8.0 with 42 of 48; 2D N=7001
-// chi=0.37 13.8 with 146 of 48 (one wave), 17.7 with 219 of 32.
+// The line kernels' grids.
+// rho: the grouping and the particle splits (multiples of 8 particles) with the least estimated time: whole waves of blocks,
+// each with a fixed cost and its FP64 cycles at a rate, plus a cost per partial row (the reduction). The constants are a fit
+// to 490 timings of evaluations on B200 (2D and 3D, N = 300 to 100000, every grouping, 8 to 1024 particles per split);
+// what it picks is within 8 % of the best of them, mostly the best. Two blocks of 8 warps share an SM at 1846 cycles per us
+// (of 1965), one alone reaches 1124, a block of 12 or 16 warps 1726: 3D N=2000 chi=0.45 takes 13.3 us with 3 groups of 4
+// tasks and 24 particles a split, 13.7 with 2 of 8, 14.0 with one of 12; 2D N=1e5 1.95 ms with groups of 8, 2.03 of 16; 2D
+// N=7001 26.7 with one wave of wide blocks, 28.4 with groups of 8.
 // force: tiles of 8 particles per block and warps per block, by whole waves of what one wave measured (3D, 67 units: 9.4,
 // 15.2, 20.6 and 28.7 us for 1 to 4 tiles with 8 warps, two blocks to an SM; 9.0, 11.8 and 16.8 for 2 to 4 tiles with 16).
-constexpr double kLineFixedUs = 1.5, kLinePipe = 0.7, kLineL2BytesPerUs = 3e6;
+constexpr double kLineFixedUs = 1.5, kLineRowUs = 0.012;
 
 Launch choose_line_launch(const cc::LinePlan &p, int d, int64_t N)
 {
 	Launch l = {};
 	l.line = true;
 	l.csize = 1;
-	const int sms = sm_count();
-	const int64_t G = std::max<int64_t>(1, (int64_t)p.wide.count());
-	const int per_sm = p.wide.ntask <= cc::kLineTasks ? 2 : 1;
-	const double particle_us = p.wide.cycles / (kLinePipe * 1965.0);
-	double best = 1e300;
 	l.nsplit = 1;
 	l.per_split = 8;
-	const int64_t maxns = std::max<int64_t>(1, std::min<int64_t>((N + 7) / 8, 4096));
-	for (int64_t ns = 1; ns <= maxns; ns++) {
-		const int64_t per = std::max<int64_t>(8, ((N + ns - 1) / ns + 7) / 8 * 8), real = std::max<int64_t>(1, (N + per - 1) / per);
-		const int64_t wave = (int64_t)per_sm * sms, full = G * real / wave, rest = G * real - full * wave;
-		const double us = (double)per * particle_us, last = rest == 0 ? 0.0 : rest <= sms ? us : per_sm * us;
-		const double c = (double)(full + (rest > 0)) * kLineFixedUs + (double)full * per_sm * us + last +
-		                 (double)real * (double)p.nunit * 4096.0 / kLineL2BytesPerUs;
-		if (c < best) {
-			best = c;
-			l.nsplit = (int)real;
-			l.per_split = (int)per;
+	const int sms = sm_count();
+	double best = 1e300;
+	for (size_t gi = 0; gi < p.groupings.size(); gi++) {
+		const cc::LineGroups &g = p.groupings[gi];
+		const int64_t G = std::max<int64_t>(1, (int64_t)g.count());
+		const bool two = g.ntask <= cc::kLineTasks;
+		const int64_t wave = (two ? 2 : 1) * (int64_t)sms, maxns = std::max<int64_t>(1, std::min<int64_t>((N + 7) / 8, 4096));
+		for (int64_t ns = 1; ns <= maxns; ns++) {
+			const int64_t per = std::max<int64_t>(8, ((N + ns - 1) / ns + 7) / 8 * 8),
+			              real = std::max<int64_t>(1, (N + per - 1) / per);
+			const int64_t full = G * real / wave, rest = G * real - full * wave;
+			const double cyc = (double)per * g.cycles;
+			const double full_us = two ? 0.55 + 2.0 * cyc / 1846.0 : 0.28 + cyc / 1726.0;
+			const double last_us = rest == 0 ? 0.0 : two && rest <= sms ? 0.72 + cyc / 1124.0 : full_us;
+			const double c = (double)full * full_us + last_us + (double)real * kLineRowUs;
+			if (c < best) {
+				best = c;
+				l.grouping = (int)gi;
+				l.nsplit = (int)real;
+				l.per_split = (int)per;
+			}
+			if (G * real > 8LL * sms)
+				break;
 		}
-		if (G * real > 8LL * sms)
-			break;
 	}
 	// chunks: a power of two that holds a split, or as many particles as fit (and have a thread per coordinate)
-	const size_t row = (size_t)p.wide.row * sizeof(double2);
-	const size_t room = (per_sm == 2 ? 100 : 204) * 1024;
-	const int most = std::min(cc::kLineMaxChunk, p.wide.ntask * 32 / d);
+	const cc::LineGroups &g = p.groupings[l.grouping];
+	const size_t row = (size_t)g.row * sizeof(double2);
+	const size_t room = (g.ntask <= cc::kLineTasks ? 100 : 204) * 1024;
+	const int most = std::min(cc::kLineMaxChunk, g.ntask * 32 / d);
 	l.chunk = 8;
 	while (l.chunk < l.per_split && 2 * l.chunk <= most && 2 * l.chunk * row <= room)
 		l.chunk *= 2;
 	// force
+	best = 1e300;
 	static const struct {
 		int mt, warps;
 		double unit_us;   // per unit and wave
 	} opt[] = {{1, 8, 0.117}, {2, 8, 0.205}, {3, 8, 0.285}, {4, 8, 0.406}, {2, 16, 0.112}, {3, 16, 0.154}, {4, 16, 0.228}};
-	best = 1e300;
 	l.mt = 1;
 	l.fwarps = 8;
 	for (const auto &o : opt) {
@@ -711,17 +716,19 @@ int run_rho(cc_handle *h, DevKSet &k, int64_t N, const double *d_frac, double *d
 		a.per_split = N > 0 ? l.per_split : 0;
 		a.chunk = l.chunk;
 		a.log2chunk = __builtin_ctz((unsigned)l.chunk);
-		a.ngroup = L.wide.count();
+		const cc::LineGroups &g = L.groupings[l.grouping];
+		const DevLines::Groups &dg = k.line.groups[l.grouping];
+		a.ngroup = g.count();
 		a.nunit = L.nunit;
-		a.ntask = L.wide.ntask;
-		a.groups = k.line.wide.groups;
-		a.tasks = k.line.wide.tasks;
-		a.tlines = k.line.wide.tlines;
+		a.ntask = g.ntask;
+		a.groups = dg.groups;
+		a.tasks = dg.tasks;
+		a.tlines = dg.tlines;
 		a.partial = k.partial;
 		a.skip = h->d_skip;
 		a.frac_copy = (&k == &h->main) ? h->rho_copy : nullptr;
 		a.early = (h->early_call && &k == &h->main && !a.skip && !a.frac_copy) ? 1 : 0;
-		const size_t smem = cc::line_rho_smem(L.wide.row, l.chunk, h->d);
+		const size_t smem = cc::line_rho_smem(g.row, l.chunk, h->d);
 		if (int rc = h->d == 2 ? launch_line_rho_t<2>(a, nsplit, smem, st) : launch_line_rho_t<3>(a, nsplit, smem, st))
 			return rc;
 		if (after_rho)

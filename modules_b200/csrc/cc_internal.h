@@ -44,6 +44,7 @@ struct Launch {
 	int nsplit, per_split, csize, chunk;   // rho: particle splits (a multiple of the cluster size)
 	int want_force;                       // force: requested number of segment splits
 	bool line;                            // FP64 on the line kernels (cc_lines.cuh): nsplit, per_split, chunk as above
+	int grouping;                         // line rho: the plan's grouping
 	int mt, fwarps;                       // line force: tiles of 8 particles per block, warps per block
 };
 
@@ -58,7 +59,8 @@ struct DevLines {
 		const cc::LineTabs *groups = nullptr;
 		const cc::LineTask *tasks = nullptr;
 		const cc::LineIdx *tlines = nullptr;
-	} wide, narrow;                 // narrow: of blocks of 8 warps (the wide ones where these have 8)
+	};
+	std::vector<Groups> groups;     // per grouping of the plan
 	double2 *weights = nullptr;     // nunit * 256
 	double *eblock = nullptr;       // one per reduce block
 };

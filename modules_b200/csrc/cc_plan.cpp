@@ -289,8 +289,8 @@ LineTabs line_tabs(int d, bool centres, const Span &a, const Span &b, const Span
 constexpr int kRhoRowMod = 2, kForceRowMod = 4;
 constexpr int kLineForceCells = 64;      // cells per force phase when the whole set's tables do not fit
 
-// Block groups of `ntask` tasks; false when a task's tables do not fit.
-bool line_groups(const LinePlan &L, int d, bool centres, int ntask, LineGroups *out)
+// Groups of up to `most` tasks for blocks of `ntask` warps; false when a task's tables do not fit.
+bool line_groups(const LinePlan &L, int d, bool centres, int ntask, int most, LineGroups *out)
 {
 	LineGroups &G = *out;
 	G = LineGroups();
@@ -313,14 +313,14 @@ bool line_groups(const LinePlan &L, int d, bool centres, int ntask, LineGroups *
 					tasks.push_back(T{r, nj * k / nt, nj * (k + 1) / nt - nj * k / nt});
 			}
 		}
-	const size_t ngroup = (tasks.size() + ntask - 1) / ntask;
+	const size_t ngroup = (tasks.size() + most - 1) / most;
 	for (size_t t0 = 0, g = 0; t0 < tasks.size(); g++) {
 		size_t want = (tasks.size() * (g + 1) + ngroup - 1) / ngroup;   // even groups
 		want = std::max(want, t0 + 1);
 		Span a, b, c, h;
 		LineTabs tabs = {};
 		size_t t1 = t0;
-		while (t1 < tasks.size() && t1 < want && t1 - t0 < (size_t)ntask) {
+		while (t1 < tasks.size() && t1 < want && t1 - t0 < (size_t)most) {
 			Span na = a, nb = b, nc = c, nh = h;
 			for (int i = 0; i < kLineRow; i++) {
 				const LineIdx &x = L.lines[(size_t)tasks[t1].r * kLineRow + i];
@@ -454,10 +454,19 @@ LinePlan build_line_plan(const Plan &p)
 	int ntotal = 0;
 	for (int r = 0; r < nrow; r++)
 		ntotal += (L.rows[r].nj + kLineTiles - 1) / kLineTiles;
-	// A set of up to 8 tasks runs two blocks to an SM; larger sets in groups of up to 16 tasks, a block to an SM.
-	const int ntask = std::min(kLineMaxTasks, std::max(kLineTasks, (ntotal + 3) / 4 * 4));
-	if (!line_groups(L, d, centres, ntask, &L.wide) || (ntask > kLineTasks && !line_groups(L, d, centres, kLineTasks, &L.narrow)))
-		return LinePlan();   // one task's tables do not fit
+	struct {
+		int warps, tasks;
+	} want[3] = {{kLineTasks, kLineTasks}, {0, 0}, {0, 0}};
+	if (ntotal > kLineTasks / 2 && ntotal <= 4 * kLineMaxTasks)
+		want[1] = {kLineTasks, kLineTasks / 2};
+	if (ntotal > kLineTasks)
+		want[2].warps = want[2].tasks = std::min(kLineMaxTasks, (ntotal + 3) / 4 * 4);
+	for (const auto &w : want)
+		if (w.warps) {
+			L.groupings.emplace_back();
+			if (!line_groups(L, d, centres, w.warps, w.tasks, &L.groupings.back()))
+				return LinePlan();   // one task's tables do not fit
+		}
 	// force phases: the whole set when its tables fit, else chunks of kLineForceCells cells and of rows
 	const int hall = 4 * (nrow ? L.rows[0].nj : 0);
 	for (int whole = 1; whole >= 0 && L.phases.empty(); whole--) {

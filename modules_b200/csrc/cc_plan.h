@@ -107,11 +107,11 @@ struct alignas(16) LineCell {
 
 constexpr int kLineRow = 16;        // lines per row
 constexpr int kLineTiles = 4;       // column tiles per rho task
-constexpr int kLineTasks = 8;       // rho tasks (warps) per block group of a small set, two blocks to an SM
-constexpr int kLineMaxTasks = 16;   // and of a large one, one block to an SM
+constexpr int kLineTasks = 8;       // warps per rho block, two blocks to an SM
+constexpr int kLineMaxTasks = 16;   // or up to 16, one block to an SM
 constexpr int kLineMaxRow = 160;    // table entries per particle
 
-// The rho pass's block groups: `ntask` tasks (warps) each.
+// The rho pass's block groups: blocks of `ntask` warps, each with a task or none.
 struct LineGroups {
 	int ntask = 0;
 	std::vector<LineTabs> groups;
@@ -129,9 +129,9 @@ struct LinePlan {
 	std::vector<LineIdx> lines;         // rows x 16: (p0, p1, c)
 	std::vector<LineCell> cells;        // nunit x 64, cell ((u * 2 + half) * 32 + 4 (line & 7) + (h & 3))
 	std::vector<double> cellV;          // two weights per cell (plus, minus; 0 where there is no mode)
-	LineGroups wide;                    // for one configuration: 8 tasks per group (a small set), 12 or 16
-	LineGroups narrow;                  // for blocks of 8 warps when wide's are larger (else empty: wide serves)
-	const LineGroups &groups8() const { return wide.ntask == 8 ? wide : narrow; }
+	// Groupings of the tasks, the launch's choice: groups of up to 8 tasks in blocks of 8 warps (always), of up to 4 in
+	// blocks of 8 warps (a set of a few groups then has blocks for more SMs), of up to 12 or 16 in blocks as wide.
+	std::vector<LineGroups> groupings;
 	std::vector<LineTabs> phases;       // force phases: rows [r0, r0 + ntask) x cells [hlo, hlo + nh)
 	int phase_row = 0;                  // most table entries of a phase
 };

@@ -66,7 +66,7 @@ int main()
 		const Plan p = build_plan(d, M, modes.data(), V.data(), 8);
 		const LinePlan L = build_line_plan(p);
 		std::printf("d=%d M=%ld ok=%d rows=%zu units=%d groups=%zu phases=%zu\n", d, M, (int)L.ok, L.rows.size(), L.nunit,
-		            L.wide.groups.size(), L.phases.size());
+		            L.ok ? L.groupings[0].groups.size() : 0, L.phases.size());
 		if (!L.ok)
 			continue;
 		const int N = 11;   // particles, padded to 12 (rho) and 16 (forces) as the kernels pad theirs
@@ -78,10 +78,11 @@ int main()
 			x ^= x << 17;
 			v = (double)(x >> 11) / 9007199254740992.0;
 		}
-		// rho groups, of one configuration and of blocks of 8 warps
+		// rho groups, in every grouping
 		std::vector<Z> part;
-		for (const LineGroups *G : {&L.groups8(), &L.wide}) {
-		CHECK(G->ntask >= 8 && G->ntask <= 16 && G->ntask % 4 == 0 && L.groups8().ntask == 8);
+		for (const LineGroups &gr : L.groupings) {
+			const LineGroups *G = &gr;
+		CHECK(G->ntask >= 8 && G->ntask <= 16 && G->ntask % 4 == 0 && L.groupings[0].ntask == 8);
 		CHECK(G->tasks.size() == G->groups.size() * G->ntask && G->tlines.size() == G->tasks.size() * kLineRow);
 		part.assign((size_t)L.nunit * 128, Z(NAN, NAN));
 		std::vector<int> wrote(part.size(), 0);
