@@ -142,6 +142,18 @@ int upload_kset(DevKSet &k, const cc::Plan &plan);
 // The device splits of the force pass into about `want` segment ranges (uploaded on first use, kept by the k-set).
 int get_splits(DevKSet &k, int want, const DevSplits **out);
 
+// What the line kernels of one evaluation write, for evaluations of one handle that run at the same time: a lane of
+// cc_energy_grad_many (lane 0 uses the k-set's own buffers).
+struct LineLane {
+	unsigned char *blob = nullptr;
+	size_t cap = 0;
+	double2 *partial = nullptr, *rho_slot = nullptr, *weights = nullptr;
+	double *eblock = nullptr;
+	unsigned *ticket = nullptr;
+	cudaStream_t stream = nullptr;
+	cudaEvent_t ev = nullptr;
+};
+
 // Device state of cc_minimize (L-BFGS of one configuration), kept by the handle between calls (grow-only).
 struct LbBuffers {
 	double *x = nullptr, *g = nullptr, *d = nullptr, *xt = nullptr, *gt = nullptr, *S = nullptr, *Y = nullptr;
@@ -294,6 +306,8 @@ struct cc_handle {
 	size_t many_cap = 0, many_ecap = 0; // doubles of d_many_in / d_many_F and of d_many_E
 	cudaStream_t copy_stream = nullptr;
 	std::vector<cudaEvent_t> many_ev;   // two per chunk: positions in, results done
+	std::vector<cci::LineLane> lanes;   // its lanes beyond the handle's own buffers and stream
+	const cci::LineLane *lane = nullptr;   // the lane of the evaluation being enqueued (null: the handle's own)
 	bool early_call = false;        // set for the duration of a cc_energy_grad_device call when independent
 	// cc_minimize's state, kept between calls so that a minimisation makes no allocation call into the CUDA driver
 	// once the handle has run one of its size: FP64 / mixed buffers (capacities n variables, m pairs, nblk dot
