@@ -1051,15 +1051,19 @@ int nufft_setup(cc_handle *h)
 	double *d_uV = nullptr;
 	unsigned long long *gi = nullptr;
 	double *gr = nullptr, *epart = nullptr, *gim = nullptr;
-	double2 *spec = nullptr, *coef = nullptr, *rho_u = nullptr, *u_u = nullptr;
+	double2 *spec = nullptr, *coef = nullptr, *rho_u = nullptr;
+	int2 *map = nullptr;
+	unsigned *ticket = nullptr;
+
 	const int64_t nspec = ngrid / a.nf[d - 1] * (a.nf[d - 1] / 2 + 1);
-	const int nblk = std::max(1, (U + 255) / 256);
+	const int nblk = (int)std::max<int64_t>(1, (nspec + 255) / 256);
 	int rc;
 	if ((rc = nu_alloc(h, &d_um, (size_t)std::max(U, 1) * d)) || (rc = nu_alloc(h, &d_uV, (size_t)std::max(U, 1))) ||
 	    (rc = nu_alloc(h, &gi, (size_t)ngrid)) || (rc = nu_alloc(h, &gr, (size_t)ngrid)) ||
 	    (rc = nu_alloc(h, &spec, (size_t)nspec)) || (rc = nu_alloc(h, &coef, (size_t)nspec * d)) ||
 	    (rc = nu_alloc(h, &gim, (size_t)ngrid * d)) ||
-	    (rc = nu_alloc(h, &rho_u, (size_t)std::max(U, 1))) || (rc = nu_alloc(h, &u_u, (size_t)std::max(U, 1))) ||
+	    (rc = nu_alloc(h, &rho_u, (size_t)std::max(U, 1))) ||
+	    (rc = nu_alloc(h, &map, (size_t)nspec)) || (rc = nu_alloc(h, &ticket, 1)) ||
 	    (rc = nu_alloc(h, &epart, (size_t)nblk)) || (rc = nu_alloc(h, &h->d_nu_mode_u, mode_u.size())))
 		return rc;
 	if (U > 0) {
@@ -1067,6 +1071,9 @@ int nufft_setup(cc_handle *h)
 		CC_CUDA(cudaMemcpy(d_uV, uV.data(), uV.size() * sizeof(double), cudaMemcpyHostToDevice));
 	}
 	CC_CUDA(cudaMemcpy(h->d_nu_mode_u, mode_u.data(), mode_u.size() * sizeof(int), cudaMemcpyHostToDevice));
+	CC_CUDA(cudaMemset(map, 0xff, sizeof(int2) * (size_t)nspec));
+	CC_CUDA(cudaMemset(ticket, 0, sizeof(unsigned)));
+	CC_CUDA(cudaMemset(gi, 0, sizeof(unsigned long long) * (size_t)ngrid));
 	a.U = U;
 	a.umodes = d_um;
 	a.uV = d_uV;
@@ -1076,8 +1083,20 @@ int nufft_setup(cc_handle *h)
 	a.coef = coef;
 	a.gim = gim;
 	a.rho_u = rho_u;
-	a.u_u = u_u;
 	a.epart = epart;
+	a.map = map;
+	a.ticket = ticket;
+	if (U > 0) {
+		const unsigned nb = (unsigned)((U + 255) / 256);
+		if (d == 1)
+			cc::nufft_map_kernel<1><<<nb, 256>>>(a, map);
+		else if (d == 2)
+			cc::nufft_map_kernel<2><<<nb, 256>>>(a, map);
+		else
+			cc::nufft_map_kernel<3><<<nb, 256>>>(a, map);
+		CC_CUDA(cudaGetLastError());
+	}
+	CC_CUDA(cudaStreamSynchronize(nullptr));   // the handle's stream does not wait for the legacy one
 	int dims[3] = {a.nf[0], a.nf[1], a.nf[2]};
 	if (cufftPlanMany(&h->nu_p1, d, dims, nullptr, 1, 0, nullptr, 1, 0, CUFFT_D2Z, 1) != CUFFT_SUCCESS)
 		return fail(CC_ERR_CUDA, "cufftPlanMany (D2Z) failed");
@@ -1100,7 +1119,6 @@ int run_nufft_t(cc_handle *h, int64_t N, const double *d_frac, double *d_E, doub
 	cc::NufftDev a = h->nu;
 	a.skip = h->d_skip;
 	const int64_t ngrid = h->nu_ngrid;
-	CC_CUDA(cudaMemsetAsync(a.gi, 0, sizeof(unsigned long long) * ngrid, st));
 	if (N > 0) {
 		cc::nufft_spread_kernel<D><<<(unsigned)((N + cc::kNufftPerBlock - 1) / cc::kNufftPerBlock), cc::kNufftThreads,
 		                             0, st>>>(a, d_frac, (int)N);
@@ -1112,20 +1130,17 @@ int run_nufft_t(cc_handle *h, int64_t N, const double *d_frac, double *d_E, doub
 	    cufftExecD2Z(h->nu_p1, a.gr, reinterpret_cast<cufftDoubleComplex *>(const_cast<double2 *>(a.spec))) !=
 	        CUFFT_SUCCESS)
 		return fail(CC_ERR_CUDA, "cufftExecD2Z failed");
-	cc::nufft_rho_kernel<D><<<h->nu_rho_blocks, 256, 0, st>>>(a, h->rho_offset);
-	CC_CUDA(cudaGetLastError());
-	cc::nufft_energy_kernel<<<1, 32, 0, st>>>(a, h->nu_rho_blocks, 1.0 / h->volume, h->shift, d_E);
+	const bool forces = (d_F || d_gfrac) && N > 0;
+	cc::nufft_spectrum_kernel<D><<<h->nu_rho_blocks, 256, 0, st>>>(a, h->nu_nspec, h->rho_offset, forces ? 1 : 0,
+	                                                              1.0 / h->volume, h->shift, d_E);
 	CC_CUDA(cudaGetLastError());
 	const int M = (int)h->V.size();
 	if (want_rho_mode && M > 0) {
 		cc::nufft_gather_rho_kernel<<<(M + 255) / 256, 256, 0, st>>>(a.rho_u, h->d_nu_mode_u, M, h->main.rho_mode);
 		CC_CUDA(cudaGetLastError());
 	}
-	if (!(d_F || d_gfrac) || N == 0)
+	if (!forces)
 		return CC_OK;
-	CC_CUDA(cudaMemsetAsync(a.coef, 0, sizeof(double2) * h->nu_nspec * D, st));
-	cc::nufft_coef_kernel<D><<<h->nu_rho_blocks, 256, 0, st>>>(a, h->nu_nspec);
-	CC_CUDA(cudaGetLastError());
 	// complex-to-real (the input spectra are overwritten; they are rebuilt every evaluation)
 	if (cufftSetStream(h->nu_p2, st) != CUFFT_SUCCESS ||
 	    cufftExecZ2D(h->nu_p2, reinterpret_cast<cufftDoubleComplex *>(a.coef), a.gim) != CUFFT_SUCCESS)

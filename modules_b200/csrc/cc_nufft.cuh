@@ -39,13 +39,15 @@ struct NufftDev {
 	int U;                    // unique modes
 	const int32_t *umodes;    // U x D
 	const double *uV;         // U summed weights
-	unsigned long long *gi;   // spread grid (fixed point), nf0 * nf1 * nf2
+	const int2 *map;          // per half-spectrum entry m: the unique modes n = m and n = -m, or -1
+	unsigned long long *gi;   // spread grid (fixed point), nf0 * nf1 * nf2; zero between evaluations
 	double *gr;               // the same as doubles
 	const double2 *spec;      // D2Z output: nf0 x nf1 x (nf2/2 + 1) along the last used axis
 	double2 *coef;            // D type-2 half spectra H (Z2D input), the D2Z layout each
 	double *gim;              // D type-2 real grids G (Z2D output), nf0 * nf1 * nf2 each
-	double2 *rho_u, *u_u;     // per unique mode
-	double *epart;            // per block of the rho kernel
+	double2 *rho_u;           // per unique mode
+	double *epart;            // per block of the spectrum kernel
+	unsigned *ticket;         // 1, zero between launches
 	const int *skip;
 };
 
@@ -53,16 +55,6 @@ __device__ __forceinline__ double es_kernel(double t, double beta)
 {
 	const double z = 1.0 - (2.0 * t / kNufftW) * (2.0 * t / kNufftW);
 	return z > 0.0 ? exp(beta * (sqrt(z) - 1.0)) : 0.0;
-}
-
-// kernel weights of one axis for a particle at fine-grid coordinate x: points g0 .. g0 + W - 1
-__device__ __forceinline__ int es_weights(double x, double beta, double *k)
-{
-	const int g0 = (int)ceil(x - 0.5 * kNufftW);
-#pragma unroll
-	for (int t = 0; t < kNufftW; t++)
-		k[t] = es_kernel((double)(g0 + t) - x, beta);
-	return g0;
 }
 
 __device__ __forceinline__ int wrap_index(int g, int n)
@@ -138,54 +130,125 @@ template <int D> __global__ void __launch_bounds__(kNufftThreads) nufft_spread_k
 	}
 }
 
+// (leaves the fixed-point grid zero for the next evaluation)
 static __global__ void nufft_fix_to_double_kernel(NufftDev a, int64_t n)
 {
 	const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
 	if (a.skip && *a.skip)
 		return;
-	if (i < n)
+	if (i < n) {
 		a.gr[i] = (double)a.gi[i] * (1.0 / kNufftFix);
+		a.gi[i] = 0ull;
+	}
 }
 
 __device__ __forceinline__ double phihat_of(const NufftDev &a, int e, int n) { return a.phihat[e][n + a.K[e]]; }
 
-// rho at the unique modes (F_+(n) = conj(F_-(n)) from the D2Z half spectrum, deconvolved), u = V conj(rho), and
-// the energy terms summed per block in mode order.
-template <int D> __global__ void __launch_bounds__(256) nufft_rho_kernel(NufftDev a, double rho_offset)
+// The half-spectrum entry of mode n's grid frequency; false when it lies in the omitted half.
+template <int D> __device__ __forceinline__ bool nufft_entry(const NufftDev &a, const int *n, int sign, size_t *idx)
+{
+	constexpr int L = D - 1;
+	const int half = a.nf[L] / 2 + 1;
+	size_t i = 0;
+	bool in = true;
+#pragma unroll
+	for (int c = 0; c < D; c++) {
+		const int m = wrap_index(sign * n[c], a.nf[c]);
+		if (c == L)
+			in = m < half;
+		i = i * (c == L ? half : a.nf[c]) + m;
+	}
+	*idx = i;
+	return in;
+}
+
+// The entries' modes (set-up; the map was filled with -1).
+template <int D> __global__ void nufft_map_kernel(NufftDev a, int2 *map)
+{
+	const int u = blockIdx.x * blockDim.x + threadIdx.x;
+	if (u >= a.U)
+		return;
+	int n[3] = {0, 0, 0};
+#pragma unroll
+	for (int c = 0; c < D; c++)
+		n[c] = a.umodes[(size_t)u * D + c];
+	size_t i;
+	if (nufft_entry<D>(a, n, 1, &i))
+		map[i].x = u;
+	if (nufft_entry<D>(a, n, -1, &i))
+		map[i].y = u;
+}
+
+// One thread per half-spectrum entry m of the D2Z transform F_-, for the modes n = m (rho = conj(F_-(m)) / phihat) and
+// n = -m (rho = F_-(m) / phihat): rho, u = V conj(rho), the energy terms, and with `forces` the entry of each axis' type-2
+// spectrum H[m] = (A[m] + conj(A[-m])) / 2, A = -i u n_e / phihat (0 where there is no mode). Everything that one entry
+// needs comes from one entry, so rho, the coefficients, their zeroing and the energy are one kernel without atomics. The
+// energy terms are summed per block, the blocks in a fixed order by the last one to finish (a ticket, no wait).
+template <int D>
+__global__ void __launch_bounds__(256) nufft_spectrum_kernel(NufftDev a, int64_t nspec, double rho_offset, int forces,
+                                                             double inv_vol, double shift, double *E_out)
 {
 	__shared__ double sh[8];
-	const int u = blockIdx.x * 256 + threadIdx.x;
+	__shared__ int sh_last;
 	if (a.skip && *a.skip)
 		return;
+	constexpr int L = D - 1;
+	const int half = a.nf[L] / 2 + 1;
+	const int64_t idx = (int64_t)blockIdx.x * 256 + threadIdx.x;
 	double e = 0.0;
-	if (u < a.U) {
-		int n[3] = {0, 0, 0};
-		double ph = 1.0;
+	if (idx < nspec) {
+		const int2 mode = __ldg(a.map + idx);
+		double2 H[D];
 #pragma unroll
-		for (int c = 0; c < D; c++) {
-			n[c] = a.umodes[(size_t)u * D + c];
-			ph *= phihat_of(a, c, n[c]);
+		for (int c = 0; c < D; c++)
+			H[c] = make_double2(0.0, 0.0);
+		if (mode.x >= 0 || mode.y >= 0) {
+			const double2 F = a.spec[idx];
+			int n[D];
+			int64_t q = idx;
+			double ph = 1.0;
+#pragma unroll
+			for (int c = D - 1; c >= 0; c--) {
+				const int ext = c == L ? half : a.nf[c];
+				const int m = (int)(q % ext);
+				q /= ext;
+				n[c] = c != L && m > a.nf[c] / 2 ? m - a.nf[c] : m;
+				ph *= phihat_of(a, c, n[c]);
+			}
+			if (mode.x >= 0) {
+				const double2 rho = make_double2(F.x / ph + rho_offset, -F.y / ph);
+				const double v = __ldg(a.uV + mode.x);
+				a.rho_u[mode.x] = rho;
+				e = v * (rho.x * rho.x + rho.y * rho.y);
+				const double ux = v * rho.x, uy = -v * rho.y;
+#pragma unroll
+				for (int c = 0; c < D; c++) {
+					const double s = (double)n[c] / ph;
+					H[c].x += 0.5 * (uy * s);
+					H[c].y -= 0.5 * (ux * s);
+				}
+			}
+			if (mode.y >= 0) {
+				const double2 rho = make_double2(F.x / ph + rho_offset, F.y / ph);
+				const double v = __ldg(a.uV + mode.y);
+				if (n[L] > 0) {   // (with n[L] = 0 the mode -m has an entry of its own)
+					a.rho_u[mode.y] = rho;
+					e += v * (rho.x * rho.x + rho.y * rho.y);
+				}
+				const double ux = v * rho.x, uy = -v * rho.y;
+#pragma unroll
+				for (int c = 0; c < D; c++) {
+					const double s = (double)-n[c] / ph;
+					H[c].x += 0.5 * (uy * s);
+					H[c].y += 0.5 * (ux * s);
+				}
+			}
 		}
-		// F_-(m) with m = n, or conj(F_-(-n)) when n's last index lies in the omitted half
-		const int L = D - 1, half = a.nf[L] / 2 + 1;
-		int m[3];
-		bool flip = wrap_index(n[L], a.nf[L]) >= half;
+		if (forces) {
 #pragma unroll
-		for (int c = 0; c < D; c++)
-			m[c] = wrap_index(flip ? -n[c] : n[c], a.nf[c]);
-		size_t idx = 0;
-#pragma unroll
-		for (int c = 0; c < D; c++)
-			idx = idx * (c == L ? half : a.nf[c]) + m[c];
-		double2 F = a.spec[idx];
-		if (flip)
-			F.y = -F.y;   // F_-(n) = conj(F_-(-n)) for a real grid
-		double2 rho = make_double2(F.x / ph, -F.y / ph);   // rho = F_+(n) / phihat = conj(F_-(n)) / phihat
-		rho.x += rho_offset;
-		a.rho_u[u] = rho;
-		const double v = a.uV[u];
-		a.u_u[u] = make_double2(v * rho.x, -v * rho.y);
-		e = v * (rho.x * rho.x + rho.y * rho.y);
+			for (int c = 0; c < D; c++)
+				a.coef[(size_t)c * nspec + idx] = H[c];
+		}
 	}
 #pragma unroll
 	for (int o = 16; o > 0; o >>= 1)
@@ -198,21 +261,29 @@ template <int D> __global__ void __launch_bounds__(256) nufft_rho_kernel(NufftDe
 		for (int w = 0; w < 8; w++)
 			t += sh[w];
 		a.epart[blockIdx.x] = t;
+		__threadfence();
+		sh_last = atomicAdd(a.ticket, 1u) == gridDim.x - 1;
 	}
-}
-
-static __global__ void nufft_energy_kernel(NufftDev a, int nblocks, double inv_vol, double shift, double *E_out)
-{
-	if (a.skip && *a.skip)
+	__syncthreads();
+	if (!sh_last)
 		return;
-	double e = 0.0;
-	for (int b = threadIdx.x; b < nblocks; b += 32)
-		e += a.epart[b];
+	__threadfence();
+	double t = 0.0;
+	for (int b = threadIdx.x; b < (int)gridDim.x; b += 256)
+		t += __ldcg(a.epart + b);
 #pragma unroll
 	for (int o = 16; o > 0; o >>= 1)
-		e += __shfl_down_sync(0xffffffffu, e, o);
-	if (threadIdx.x == 0)
-		*E_out = e * inv_vol + shift;
+		t += __shfl_down_sync(0xffffffffu, t, o);
+	if ((threadIdx.x & 31) == 0)
+		sh[threadIdx.x >> 5] = t;
+	__syncthreads();
+	if (threadIdx.x == 0) {
+		t = 0.0;
+		for (int w = 0; w < 8; w++)
+			t += sh[w];
+		*E_out = t * inv_vol + shift;
+		*a.ticket = 0u;
+	}
 }
 
 // rho in input-mode order from the unique modes
@@ -221,52 +292,6 @@ static __global__ void nufft_gather_rho_kernel(const double2 *rho_u, const int *
 	const int m = blockIdx.x * blockDim.x + threadIdx.x;
 	if (m < M)
 		rho_mode[m] = rho_u[mode_u[m]];
-}
-
-// type-2 coefficients: with C_e[n] = u_n n_e / phihat(n) and A = -i C_e, the half spectrum of each axis' Hermitian
-// H[m] = (A[m] + conj(A[-m])) / 2 (the spectra were zeroed). Mode n adds A/2 at +n and conj(A)/2 at -n where these lie
-// in the stored half (last index 0 .. nf/2). An entry m receives at most two terms (from the modes m and -m, the
-// modes being unique), and a sum of two terms onto zero does not depend on their order: the result repeats bitwise.
-template <int D> __global__ void __launch_bounds__(256) nufft_coef_kernel(NufftDev a, int64_t nspec)
-{
-	const int u = blockIdx.x * 256 + threadIdx.x;
-	if (a.skip && *a.skip)
-		return;
-	if (u >= a.U)
-		return;
-	constexpr int L = D - 1;
-	const int half = a.nf[L] / 2 + 1;
-	int n[3] = {0, 0, 0};
-	double ph = 1.0;
-	size_t ip = 0, im = 0;
-	bool hp = true, hm = true;
-#pragma unroll
-	for (int c = 0; c < D; c++) {
-		n[c] = a.umodes[(size_t)u * D + c];
-		ph *= phihat_of(a, c, n[c]);
-		const int mp = wrap_index(n[c], a.nf[c]), mm = wrap_index(-n[c], a.nf[c]);
-		if (c == L) {
-			hp = mp < half;
-			hm = mm < half;
-		}
-		ip = ip * (c == L ? half : a.nf[c]) + mp;
-		im = im * (c == L ? half : a.nf[c]) + mm;
-	}
-	const double2 uu = a.u_u[u];
-#pragma unroll
-	for (int c = 0; c < D; c++) {
-		const double s = (double)n[c] / ph;
-		const double cx = uu.x * s, cy = uu.y * s;   // C = cx + i cy, A = cy - i cx
-		double2 *H = a.coef + (size_t)c * nspec;
-		if (hp) {
-			atomicAdd(&H[ip].x, 0.5 * cy);
-			atomicAdd(&H[ip].y, -0.5 * cx);
-		}
-		if (hm) {
-			atomicAdd(&H[im].x, 0.5 * cy);
-			atomicAdd(&H[im].y, 0.5 * cx);
-		}
-	}
 }
 
 struct NufftOut {
