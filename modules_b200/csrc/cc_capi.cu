@@ -93,8 +93,7 @@ int cci::get_splits(DevKSet &k, int want, const DevSplits **out)
 }
 
 
-// The plan's arrays (and the line plan's) go up in one copy into one allocation, followed by what the kernels write,
-// zeroed: slots without a mode are read (with weight 0) but never written on the line path, and the ticket starts at 0.
+// The plan's arrays (and the line plan's) go up in one copy into one allocation; what the kernels write starts at zero: slots without a mode are read (with weight 0) but never written on the line path, and the ticket starts at 0.
 int cci::upload_kset(DevKSet &k, const cc::Plan &plan)
 {
 	k.release();
@@ -132,14 +131,19 @@ int cci::upload_kset(DevKSet &k, const cc::Plan &plan)
 		end += room(std::max<size_t>(bytes, 1));
 		return at;
 	};
-	const size_t o_ticket = take(sizeof(unsigned)), o_rho = take(nslot * sizeof(double2)),
-	             o_u = take(nslot * sizeof(double2)), o_rhom = take(M * sizeof(double2)), o_eb = take(nred * sizeof(double)),
-	             o_w = take((size_t)L.nunit * 8 * 32 * sizeof(double2)), o_leb = take(nlred * sizeof(double));
+	const size_t o_ticket = take(sizeof(unsigned)), o_eb = take(nred * sizeof(double)), o_leb = take(nlred * sizeof(double));
+	// (the larger arrays apart: allocations below 2 MB come out of the driver's blocks, larger ones take a millisecond)
 	if (int rc = dev_alloc(&k.blob, end))
 		return rc;
+	if (int rc = dev_alloc(&k.rho_slot, 2 * nslot))
+		return rc;
+	if (int rc = dev_alloc(&k.rho_mode, M))
+		return rc;
+	k.u_slot = k.rho_slot + nslot;
 	if (!up.empty())
 		CC_CUDA(cudaMemcpy(k.blob, up.data(), up.size(), cudaMemcpyHostToDevice));
 	CC_CUDA(cudaMemset(k.blob + up.size(), 0, end - up.size()));
+	CC_CUDA(cudaMemset(k.rho_slot, 0, 2 * nslot * sizeof(double2)));
 	unsigned char *b = k.blob;
 	k.segs = reinterpret_cast<cc::Seg *>(b + o_segs);
 	k.bstart = reinterpret_cast<int *>(b + o_bstart);
@@ -147,9 +151,6 @@ int cci::upload_kset(DevKSet &k, const cc::Plan &plan)
 	k.slotV = reinterpret_cast<double *>(b + o_slotV);
 	k.mode_slot = reinterpret_cast<int *>(b + o_mode);
 	k.ticket = reinterpret_cast<unsigned *>(b + o_ticket);
-	k.rho_slot = reinterpret_cast<double2 *>(b + o_rho);
-	k.u_slot = reinterpret_cast<double2 *>(b + o_u);
-	k.rho_mode = reinterpret_cast<double2 *>(b + o_rhom);
 	k.eblock = reinterpret_cast<double *>(b + o_eb);
 	k.line.rows = reinterpret_cast<cc::LineRow *>(b + o_rows);
 	k.line.lines = reinterpret_cast<cc::LineIdx *>(b + o_lines);
@@ -159,7 +160,6 @@ int cci::upload_kset(DevKSet &k, const cc::Plan &plan)
 	for (const Offsets &o : og)
 		k.line.groups.push_back({reinterpret_cast<cc::LineTabs *>(b + o.groups), reinterpret_cast<cc::LineTask *>(b + o.tasks),
 		                         reinterpret_cast<cc::LineIdx *>(b + o.tlines)});
-	k.line.weights = reinterpret_cast<double2 *>(b + o_w);
 	k.line.eblock = reinterpret_cast<double *>(b + o_leb);
 	return CC_OK;
 }
@@ -709,9 +709,13 @@ int run_rho(cc_handle *h, DevKSet &k, int64_t N, const double *d_frac, double *d
 		const int nsplit = N > 0 ? l.nsplit : 1;
 		const cc::LinePlan &L = k.lplan;
 		const LineLane *lane = &k == &h->main ? h->lane : nullptr;
-		if (!lane)
+		if (!lane) {
 			if (int rc = ensure_partial(k, (size_t)nsplit * L.nunit * 128))
 				return rc;
+			if (!k.line.weights)
+				if (int rc = dev_alloc(&k.line.weights, (size_t)L.nunit * 256))
+					return rc;
+		}
 		cc::LineRhoArgs a = {};
 		a.frac = d_frac;
 		a.N = (int)N;
@@ -1240,13 +1244,18 @@ cudaEvent_t next_event(cc_handle *h)
 	return h->ev[h->ev_used++];
 }
 
-// CC_PATH_AUTO: the NUFFT path when its estimated time, with a 20 % margin, is below the direct path's. Direct:
-// N x slots at 700 G pairs/s; NUFFT: 3.9e-12 s per particle and kernel point (spread + interpolation, W^d points),
-// 7.2e-12 s per fine-grid point and transform, 80 us of launches and transforms at small sizes. Fitted to B200
-// timings of single evaluations (L2 flushed, FP64 energy + forces): 2D N=1e5 M=40002 0.165 ms NUFFT against 5.1 ms
-// direct; 2D N=2e4 M=8002 0.083 against 0.26; 3D N=2e4 M=12055 0.31 against 0.44; 3D N=1e5 M=60020 1.21 against
-// 9.3; 3D N=2000 M=2724 0.13 against 0.034.
-bool nufft_preferred(cc_handle *h, int64_t N)
+// CC_PATH_AUTO: the NUFFT path when its estimated time, with a 20 % margin, is below the direct path's on the segment kernels
+// (direct N x slots at 700 G pairs/s, NUFFT 3.9e-12 s per particle and kernel point (spread + interpolation, W^d points),
+// 7.2e-12 s per fine-grid point and transform and 80 us) and, in FP64 on the line kernels, also below the direct path's there.
+// The second condition only takes calls off the NUFFT path: its forces are within 7e-13 of 64-bit sums, the line kernels' within
+// 1e-14 (relative, worst component), so no set goes to it for the few tens of microseconds that it would save between the two.
+// 0.8: calls one after another (not in one graph) overlap on the NUFFT path's streams, 3D N=30000 chi=0.3 347 us against 452.
+// Its estimates are fits to evaluations in CUDA graphs on B200 (27 sets, 2D and 3D, N = 3000 to 100000, chi = 0.05 to 0.49; the
+// direct one within 13 %, mostly 5 %): direct 8.8 us + 59 ps per particle and unit + 39 ps per particle and row of lines in 3D +
+// 0.28 ns per particle; NUFFT 24 us + 0.62 ns per particle + 40 ps per grid point in 2D, 70 us + 9.3 ns + 90 ps in 3D. Measured,
+// direct against NUFFT: 2D N=20000 chi=0.05 42.6 / 39.2 us, chi=0.2 102.9 / 40.2; 3D N=20000 chi=0.49 363 / 348, N=30000 chi=0.2
+// 378 / 384, chi=0.45 698 / 422, N=60000 chi=0.05 379 / 650, N=100000 chi=0.05 963 / 1022.
+bool nufft_preferred(cc_handle *h, int64_t N, bool mixed)
 {
 	if (h->main.plan.nslot == 0 || N < 1024 || h->d_slotS0)
 		return false;
@@ -1269,7 +1278,13 @@ bool nufft_preferred(cc_handle *h, int64_t N)
 		return false;
 	const double direct = (double)N * (double)h->main.plan.real_segs * h->main.plan.L / 7e11;
 	const double nufft = 3.9e-12 * (double)N * w + 7.2e-12 * grid * (1 + d) + 8e-5;
-	return 1.2 * nufft < direct;
+	const cc::LinePlan &L = h->main.lplan;
+	if (1.2 * nufft >= direct || mixed || !L.ok)
+		return 1.2 * nufft < direct;
+	const double n = (double)N;
+	const double direct_us = 8.8 + 59e-6 * n * L.nunit + (d == 3 ? 39e-6 * n * (double)L.rows.size() : 0.0) + 2.8e-4 * n;
+	const double nufft_us = d == 2 ? 24.0 + 6.2e-4 * n + 4e-5 * grid : 70.0 + 9.3e-3 * n + 9e-5 * grid;
+	return 0.8 * nufft_us < direct_us;
 }
 
 // ShiftedCCPotential_S2_MultiConfig (potential/CollectiveCoordinatePotential.h:1756-1870): particles
@@ -1355,7 +1370,7 @@ int eval_device(cc_handle *h, int64_t N, const double *d_frac, double *d_E, doub
 			return fail(CC_ERR_CUDA, "cudaEventCreate failed");
 		CC_CUDA(record_timing(e0, st));
 	}
-	if ((h->use_nufft || (h->auto_path && nufft_preferred(h, N))) && h->main.plan.nslot > 0) {
+	if ((h->use_nufft || (h->auto_path && nufft_preferred(h, N, mixed))) && h->main.plan.nslot > 0) {
 		// non-uniform FFT path (FP64 whatever the precision): reported as the force interval
 		if (e1)
 			CC_CUDA(record_timing(e1, st));
@@ -1417,7 +1432,7 @@ int launch_eval_graph(cc_handle *h, int64_t N, int precision, int forces, bool *
 	// Positions from the mapped staging buffer: on the three-kernel path the rho kernel reads them there and stores
 	// them into d_frac for the force kernel; on the NUFFT path a kernel copies them first. Either way the first
 	// kernel of the evaluation reads host memory, and no copy node sits in front of the programmatic dependent launches.
-	const bool nufft = h->use_nufft || (h->auto_path && nufft_preferred(h, N));
+	const bool nufft = h->use_nufft || (h->auto_path && nufft_preferred(h, N, precision == CC_PREC_MIXED));
 	cudaError_t ce = cudaSuccess;
 	int rc;
 	if (nufft) {
@@ -1913,7 +1928,7 @@ static int many_lanes(cc_handle *h, int64_t N, int precision, int *count)
 	*count = 1;
 	DevKSet &k = h->main;
 	if (precision != CC_PREC_FP64 || N == 0 || h->nsub > 1 || h->timing || !k.lplan.ok || k.plan.nslot == 0 || h->use_nufft ||
-	    (h->auto_path && nufft_preferred(h, N)))
+	    (h->auto_path && nufft_preferred(h, N, precision == CC_PREC_MIXED)))
 		return CC_OK;
 	const Launch l = choose_launch(k, N, false);
 	const cc::LinePlan &L = k.lplan;
@@ -2055,7 +2070,7 @@ int cc_rho(cc_handle *h, double *re, double *im, int precision)
 		return rc;
 	const int64_t N = h->N;
 	const size_t M = h->V.size();
-	if ((h->use_nufft || (h->auto_path && nufft_preferred(h, N))) && h->main.plan.nslot > 0) {
+	if ((h->use_nufft || (h->auto_path && nufft_preferred(h, N, precision == CC_PREC_MIXED))) && h->main.plan.nslot > 0) {
 		if (int rc = run_nufft(h, N, h->d_frac, h->d_E, nullptr, nullptr, true, h->stream))
 			return rc;
 	} else {
@@ -2345,7 +2360,7 @@ int cc_eval_path(cc_handle *h, int64_t N, int precision, int *path)
 		return rc;
 	if (!path || N < 0)
 		return fail(CC_ERR_ARG, "invalid cc_eval_path arguments");
-	if (h->nsub <= 1 && (h->use_nufft || (h->auto_path && nufft_preferred(h, N))) && h->main.plan.nslot > 0)
+	if (h->nsub <= 1 && (h->use_nufft || (h->auto_path && nufft_preferred(h, N, precision == CC_PREC_MIXED))) && h->main.plan.nslot > 0)
 		*path = CC_PATH_NUFFT;
 	else
 		*path = CC_PATH_SPLIT;

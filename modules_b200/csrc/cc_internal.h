@@ -69,7 +69,7 @@ struct DevKSet {
 	cc::Plan plan;
 	cc::LinePlan lplan;
 	DevLines line;
-	unsigned char *blob = nullptr;  // one allocation for the arrays below (and the line plan's) but `partial`
+	unsigned char *blob = nullptr;  // one allocation for the plan's arrays and the line plan's
 	cc::Seg *segs = nullptr;
 	int *bstart = nullptr;
 	cc::TabSpec *bspec = nullptr;
@@ -93,6 +93,9 @@ struct DevKSet {
 	void release()
 	{
 		cudaFree(blob);
+		cudaFree(rho_slot);   // (and u_slot)
+		cudaFree(rho_mode);
+		cudaFree(line.weights);
 		cudaFree(partial);
 		for (DevSplits &f : splits) {
 			cudaFree(f.kstart);

@@ -278,7 +278,7 @@ struct LineReduceArgs {
 	const double2 *cellS0;    // S2 targets, or null
 	double npart;
 	double rho_offset;
-	double2 *rho_slot, *u_slot;   // rho and u = V conj(rho) (S2: V dS conj(rho)) per slot; u_slot may be null
+	double2 *rho_slot;            // rho per slot
 	double2 *weights;         // force weights in fragment order (may be null)
 	double *eblock;           // [blocks]
 	unsigned *ticket;
@@ -412,11 +412,8 @@ __device__ __forceinline__ void line_reduce_body(const LineReduceArgs &a, const 
 				e = w * r2;
 			}
 			up = make_double2(w * r.x, -w * r.y);
-			if (q == 0) {
+			if (q == 0)
 				a.rho_slot[cl.sp] = r;
-				if (a.u_slot)
-					a.u_slot[cl.sp] = up;
-			}
 		}
 		if (cl.sm >= 0) {
 			const double2 r = make_double2(ar + bi + a.rho_offset, ai - br);
@@ -430,11 +427,8 @@ __device__ __forceinline__ void line_reduce_body(const LineReduceArgs &a, const 
 				e += w * r2;
 			}
 			um = make_double2(w * r.x, -w * r.y);
-			if (q == 0) {
+			if (q == 0)
 				a.rho_slot[cl.sm] = r;
-				if (a.u_slot)
-					a.u_slot[cl.sm] = um;
-			}
 		}
 		if (a.weights)
 			a.weights[line_weight_at(cell0 + ci, q)] = line_weight(q, cl.h, up, um);

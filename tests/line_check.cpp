@@ -80,61 +80,60 @@ int main()
 		}
 		// rho groups, in every grouping
 		std::vector<Z> part;
-		for (const LineGroups &gr : L.groupings) {
-			const LineGroups *G = &gr;
-		CHECK(G->ntask >= 8 && G->ntask <= 16 && G->ntask % 4 == 0 && L.groupings[0].ntask == 8);
-		CHECK(G->tasks.size() == G->groups.size() * G->ntask && G->tlines.size() == G->tasks.size() * kLineRow);
-		part.assign((size_t)L.nunit * 128, Z(NAN, NAN));
-		std::vector<int> wrote(part.size(), 0);
-		for (size_t grp = 0; grp < G->groups.size(); grp++) {
-			const LineTabs &tb = G->groups[grp];
-			CHECK(tb.row % 4 == 2);
-			std::vector<std::vector<Z> > tab;
-			for (int j = 0; j < N; j++)
-				tab.push_back(tables(d, tb, &s[(size_t)j * d]));
-			int active = 0;
-			for (int w = 0; w < G->ntask; w++) {
-				const LineTask task = G->tasks[grp * G->ntask + w];
-				CHECK(task.n >= 0 && task.n <= kLineTiles);
-				active += task.n > 0;
-				if (!task.n)
-					continue;
-				for (int half = 0; half < 2; half++)
-					for (int lane = 0; lane < 32; lane++) {
-						const int g = lane >> 2, t = lane & 3;
-						const LineIdx l = G->tlines[(grp * G->ntask + w) * kLineRow + half * 8 + g];
-						for (int j = 0; j < task.n; j++) {
-							Z A = 0, B = 0;
-							for (int i = 0; i < N; i++) {
-								const std::vector<Z> &row = tab[i];
-								CHECK(l.p0 >= 0 && l.p0 < tb.row);
-								Z X = row[l.p0];
-								if (d == 3) {
-									CHECK(l.p1 >= 0 && l.p1 < tb.row);
-									X *= row[l.p1];
+		for (const LineGroups &G : L.groupings) {
+			CHECK(G.ntask >= 8 && G.ntask <= 16 && G.ntask % 4 == 0 && L.groupings[0].ntask == 8);
+			CHECK(G.tasks.size() == G.groups.size() * G.ntask && G.tlines.size() == G.tasks.size() * kLineRow);
+			part.assign((size_t)L.nunit * 128, Z(NAN, NAN));
+			std::vector<int> wrote(part.size(), 0);
+			for (size_t grp = 0; grp < G.groups.size(); grp++) {
+				const LineTabs &tb = G.groups[grp];
+				CHECK(tb.row % 4 == 2);
+				std::vector<std::vector<Z> > tab;
+				for (int j = 0; j < N; j++)
+					tab.push_back(tables(d, tb, &s[(size_t)j * d]));
+				int active = 0;
+				for (int w = 0; w < G.ntask; w++) {
+					const LineTask task = G.tasks[grp * G.ntask + w];
+					CHECK(task.n >= 0 && task.n <= kLineTiles);
+					active += task.n > 0;
+					if (!task.n)
+						continue;
+					for (int half = 0; half < 2; half++)
+						for (int lane = 0; lane < 32; lane++) {
+							const int g = lane >> 2, t = lane & 3;
+							const LineIdx l = G.tlines[(grp * G.ntask + w) * kLineRow + half * 8 + g];
+							for (int j = 0; j < task.n; j++) {
+								Z A = 0, B = 0;
+								for (int i = 0; i < N; i++) {
+									const std::vector<Z> &row = tab[i];
+									CHECK(l.p0 >= 0 && l.p0 < tb.row);
+									Z X = row[l.p0];
+									if (d == 3) {
+										CHECK(l.p1 >= 0 && l.p1 < tb.row);
+										X *= row[l.p1];
+									}
+									if (tb.n[2] > 0) {
+										CHECK(l.c >= 0 && l.c < tb.row);
+										X *= row[l.c];
+									}
+									const int c = task.hoff + 4 * j + t;   // columns 2t, 2t + 1 of tile j
+									CHECK(2 * task.hoff + 8 * j + 7 < 2 * tb.row && c >= tb.offh && c < tb.offh + tb.nh);
+									A += X * row[c].real();
+									B += X * row[c].imag();
 								}
-								if (tb.n[2] > 0) {
-									CHECK(l.c >= 0 && l.c < tb.row);
-									X *= row[l.c];
-								}
-								const int c = task.hoff + 4 * j + t;   // columns 2t, 2t + 1 of tile j
-								CHECK(2 * task.hoff + 8 * j + 7 < 2 * tb.row && c >= tb.offh && c < tb.offh + tb.nh);
-								A += X * row[c].real();
-								B += X * row[c].imag();
+								const size_t o = (size_t)task.u0 * 128 + j * 128 + half * 64 + lane;
+								CHECK(o + 32 < part.size());
+								part[o] = Z(A.real(), B.real());
+								part[o + 32] = Z(A.imag(), B.imag());
+								wrote[o]++;
+								wrote[o + 32]++;
 							}
-							const size_t o = (size_t)task.u0 * 128 + j * 128 + half * 64 + lane;
-							CHECK(o + 32 < part.size());
-							part[o] = Z(A.real(), B.real());
-							part[o + 32] = Z(A.imag(), B.imag());
-							wrote[o]++;
-							wrote[o + 32]++;
 						}
-					}
+				}
+				CHECK(active == tb.ntask);
 			}
-			CHECK(active == tb.ntask);
-		}
-		for (int w : wrote)
-			CHECK(w == 1);
+			for (int w : wrote)
+				CHECK(w == 1);
 		}
 		// reduction: every slot with a mode once, equal to the direct sum; weights in place
 		std::vector<Z> u((size_t)p.nslot), wts((size_t)L.nunit * 256, Z(NAN, NAN));

@@ -117,3 +117,21 @@ def test_mc_moves_against_whole_energies(gpu, d, M):
             cur, E = trial, q.energy()
         if step == 3:
             p.energy_and_forces()
+
+
+@pytest.mark.parametrize("d,N,chi", [(2, 12000, 0.20), (2, 100000, 0.20), (3, 30000, 0.05), (3, 60000, 0.05), (3, 30000, 0.45)])
+def test_auto_path(gpu, d, N, chi):
+    """AUTO: FP64 takes the NUFFT path only where mixed precision's rule (the segment kernels') does, and not where the
+    line kernels are faster; either way its results are those of the path that it names, bit by bit."""
+    basis = np.eye(d) * N ** (1 / d)
+    modes, V = gpu.stealthy_kset(d, basis, N, chi)
+    p = gpu.CCPotential(d, basis, modes, V)
+    p.set_configuration(np.random.default_rng(N).random((N, d)))
+    fp64, mixed = p.eval_path(N), p.eval_path(N, gpu.PREC_MIXED)
+    assert fp64 == mixed or (fp64, mixed) == ("split", "nufft")
+    expect = {(2, 12000): "split", (2, 100000): "nufft", (3, 30000): {0.05: "split", 0.45: "nufft"}.get(chi), (3, 60000): "split"}
+    assert fp64 == expect[d, N]
+    E, F = p.energy_and_forces()
+    p.set_path(gpu.PATH_NUFFT if fp64 == "nufft" else gpu.PATH_SPLIT)
+    E1, F1 = p.energy_and_forces()
+    assert E == E1 and np.array_equal(F, F1)
