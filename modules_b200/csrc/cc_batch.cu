@@ -55,10 +55,12 @@ int batch_line_chunk(const cc::LineGroups &g, int per_split)
 constexpr int kTuneSplits[] = {32, 64, 128, 256, 512, 1024};
 constexpr int kTuneSegs[] = {32, 64, 128, 256, 512, 1024};
 
+constexpr size_t kBatchLineSmem = 104 * 1024;   // line items: two blocks to an SM
+
 // dynamic shared memory the fused kernel is allowed (its largest table rows in FP64, any dimension)
 size_t mbatch_smem_cap()
 {
-	return std::max((size_t)100 * 1024, std::max(rho_smem<double2>(cc::kMaxRow, kBatchChunk, 8), force_smem<double2>(cc::kMaxRow, 3)));
+	return std::max(kBatchLineSmem, std::max(rho_smem<double2>(cc::kMaxRow, kBatchChunk, 8), force_smem<double2>(cc::kMaxRow, 3)));
 }
 
 template <auto KERNEL, class ARGS> int mbatch_launch_t(const ARGS &a, const int *totals, size_t smem, cudaStream_t st)
@@ -265,10 +267,15 @@ int batch_build(cc_batch *b, int per_split, int segs_per_split)
 			const DevLines &dl = h->main.line;
 			lr.frac = ra.frac;
 			lr.N = ra.N;
-			lr.per_split = per_split;
-			lr.chunk = batch_line_chunk(L.groupings[0], per_split);
-			lr.log2chunk = __builtin_ctz((unsigned)lr.chunk);
+			// Twice the particles per rho item from 20 items of the instance on: an item's fixed cost (queue, descriptor, table
+			// latencies, partial rows: about 4 us) stays small beside its 4 to 8 us of matrix work. 512 uneven instances
+			// 1.98 -> 1.82 ms, 60 of the benchmark's kind 214 -> 198 us, 128 x 3D N=2000 0.85 -> 0.79 ms. A rule on the instance
+			// alone: its results do not depend on the rest of the batch.
 			lr.ngroup = L.groupings[0].count();
+			lr.per_split = (long)n * lr.ngroup >= 20L * per_split ? 2 * per_split : per_split;
+			const int lsplit = (int)((n + lr.per_split - 1) / lr.per_split);
+			lr.chunk = batch_line_chunk(L.groupings[0], lr.per_split);
+			lr.log2chunk = __builtin_ctz((unsigned)lr.chunk);
 			lr.nunit = L.nunit;
 			lr.ntask = cc::kLineTasks;
 			lr.groups = dl.groups[0].groups;
@@ -276,7 +283,7 @@ int batch_build(cc_batch *b, int per_split, int segs_per_split)
 			lr.tlines = dl.groups[0].tlines;
 			lr.partial = ra.partial;
 			ld.partial = lr.partial;
-			ld.nsplit = nsplit;
+			ld.nsplit = lsplit;
 			ld.nunit = L.nunit;
 			ld.cells = dl.cells;
 			ld.cellV = dl.cellV;
@@ -299,8 +306,8 @@ int batch_build(cc_batch *b, int per_split, int segs_per_split)
 			lf.inv_vol = fa.inv_vol;
 			lf.shift = fa.shift;
 			lf.E_out = fa.E_out;
-			lf.tiles = 1;   // set below
-			const int lc[3] = {lr.ngroup * nsplit, lf.neblock, (int)((n + 8 * cc::kLineBatchMT - 1) / (8 * cc::kLineBatchMT))};
+			lf.tiles = lf.teams = 1;   // set below
+			const int lc[3] = {lr.ngroup * lsplit, lf.neblock, (int)((n + 8 * cc::kLineBatchMT - 1) / (8 * cc::kLineBatchMT))};
 			for (int ph = 0; ph < 3; ph++)
 				own[(3 + ph) * B + k] = lc[ph];
 			b->line_smem = std::max(b->line_smem, std::max(cc::line_rho_smem(L.groupings[0].row, lr.chunk, h->d),
@@ -317,12 +324,31 @@ int batch_build(cc_batch *b, int per_split, int segs_per_split)
 		b->force_row = std::max(b->force_row, f->host.max_row);
 		b->maxd = std::max(b->maxd, h->d);
 	}
-	// Line force items: several tiles each where the batch has many (a tile's results do not depend on it), so that an
-	// item's fixed cost (queue, descriptor, completion: 4 us) stays small beside its tiles (10 to 20 us each).
+	// Line force items. From 1.5 tiles of 24 particles per resident block on, a block's warps work as two teams on 48 particles
+	// (line_force_body: the results are the same) where their tables leave two blocks to an SM: the fixed cost of a tile (table
+	// and reduction latencies: 4 us) is paid half as often, 48 uneven instances 181 -> 151 us, 512 2.11 -> 1.96 ms; with fewer
+	// tiles the longer ones cost more (12 instances 25 against 28 us). Then several tiles per item where the batch has many, so
+	// that an item's fixed cost (queue, descriptor, completion) stays small: two from 4.6 per block on (833 tiles, 2.8 a block:
+	// 250 us with one, 289 with two; 1478, 5.0 a block: 151 and 145).
 	int64_t tiles = 0;
 	for (int k = 0; k < B; k++)
 		tiles += own[5 * B + k];
-	const int per_item = (int)std::max<int64_t>(1, std::min<int64_t>(8, tiles / (6 * 2 * sm_count())));
+	const bool teams = 2 * tiles >= 3 * 2 * sm_count();
+	tiles = 0;
+	for (int k = 0; k < B; k++) {
+		const cc_handle *h = b->h[b->order[k]];
+		const cc::LinePlan &L = h->main.lplan;
+		if (!L.ok)
+			continue;
+		const size_t two = cc::line_force_smem(L.phase_row, cc::kLineBatchMT, 8, h->d, 2);
+		if (teams && L.phases.size() == 1 && two <= kBatchLineSmem) {
+			b->lforce[k].teams = 2;
+			own[5 * B + k] = (own[5 * B + k] + 1) / 2;
+			b->line_smem = std::max(b->line_smem, two);
+		}
+		tiles += own[5 * B + k];
+	}
+	const int per_item = (int)std::max<int64_t>(1, std::min<int64_t>(8, tiles * 10 / (46 * sm_count())));
 	for (int k = 0; k < B; k++) {
 		b->lforce[k].tiles = per_item;
 		own[5 * B + k] = (own[5 * B + k] + per_item - 1) / per_item;

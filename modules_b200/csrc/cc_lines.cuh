@@ -560,7 +560,7 @@ struct LineForceArgs {
 	const double *frac;       // N x D
 	int N;
 	int nphase;
-	int tiles;                // in a batch: tiles per item
+	int tiles, teams;         // in a batch: tiles per item, teams of a block's warps (8 MT particles each)
 	const LineTabs *phases;
 	const LineRow *rows;
 	const LineIdx *lines;     // rows x 16
@@ -596,23 +596,30 @@ __device__ __forceinline__ void line_energy_body(const LineForceArgs &a, const I
 // MT = 1: 13.7 us per evaluation with four pairs, 15.9 with two; MT = 2 with 16 warps: 13.6 and 13.3).
 __host__ __device__ constexpr int line_nt(int mt) { return mt == 1 ? 4 : 2; }
 
-// Tiles [tile0, tile1) of 8 MT particles each, W warps. Per tile and phase the particles' tables are built, then the warps take the phase's rows
-// in turn (8 / NT warps a row, NT line pairs each) and contract the row's cells: per 4 cells NT weight fragments of 512 B
+// Tiles [tile0, tile1), W warps. Per tile (8 MT particles) and phase the particles' tables are built, then the warps take the
+// phase's rows in turn (8 / NT warps a row, NT line pairs each) and contract the row's cells: per 4 cells NT weight fragments of 512 B
 // from L2 (read once per block, in fragment order) against MT table fragments from shared memory, 2 MT NT DMMAs. What is
 // left beside the DMMAs is instructions per step and the product with X per task, so weights with T's and D's factors
 // written out (64 B a cell) beat 32 B ones expanded here (2D N=1e5: 2.05 against 2.17 ms per evaluation; 3D N=20000: 178
 // against 187 us), and a ring of asynchronous copies for the weights gains nothing over loads one step ahead.
+// With two teams (one phase only) a tile is 16 MT particles and each half of the warps contracts half of them with every row:
+// more work between barriers, and rows of few tasks no longer leave warps idle. A warp of a team stands for the two warps of a
+// block of one team one after the other, so that the sums are the same in every bit.
 template <int D, int MT, int W>
-__device__ __forceinline__ void line_force_body(const LineForceArgs &a, const int tile0, const int tile1, const ItemCtl ctl)
+__device__ __forceinline__ void line_force_body(const LineForceArgs &a, const int tile0, const int tile1, const ItemCtl ctl,
+                                                const int teams = 1)
 {
-	constexpr int P = 8 * MT, E = MT <= 2 ? 8 : 16, NT = line_nt(MT), SUB = 8 / NT, LOG2P = MT == 1 ? 3 : MT == 2 ? 4 : 5;
+	constexpr int E = MT <= 2 ? 8 : 16, NT = line_nt(MT), SUB = 8 / NT;
+	const int P = 8 * MT * teams, LOG2P = (MT == 1 ? 3 : MT == 2 ? 4 : 5) + teams - 1, WT = W / teams;
 	extern __shared__ __align__(16) unsigned char smem[];
 	double *pos = reinterpret_cast<double *>(smem);    // P x D
 	double2 *tab = reinterpret_cast<double2 *>(smem + line_pos_bytes(P, D));
-	double *sh_g = reinterpret_cast<double *>(tab);    // after the loops: W warps x P x D
-	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-	const int t = lane & 3, g = lane >> 2;
 	LineTabs tb = load_rec(a.phases);
+	// the sums of W warps x P x D: of one team over the tables, after the loops; else behind them
+	double *sh_g = reinterpret_cast<double *>(teams == 1 ? tab : tab + (size_t)P * tb.row);
+	const int lane = threadIdx.x & 31, team = teams == 1 ? 0 : (int)(threadIdx.x >> 5) / WT;
+	const int warp = (int)(threadIdx.x >> 5) - team * WT;
+	const int t = lane & 3, g = lane >> 2, g0 = team * 8 * MT + g;   // the lane's first particle of the tile
 	// (as force_body: a finished instance builds no tables, but waits for its reduce items where there are any)
 	if (eval_skipped(a.skip, ctl.stage, ctl.want_stage)) {
 		if (ctl.ready)
@@ -647,11 +654,34 @@ __device__ __forceinline__ void line_force_body(const LineForceArgs &a, const in
 		if (tile + 1 < tile1)
 			next = load(tile + 1);
 		double gs[MT][D];
+		auto clear_sums = [&] {
 #pragma unroll
-		for (int m = 0; m < MT; m++)
+			for (int m = 0; m < MT; m++)
 #pragma unroll
-			for (int e = 0; e < D; e++)
-				gs[m][e] = 0.0;
+				for (int e = 0; e < D; e++)
+					gs[m][e] = 0.0;
+		};
+		// the four lanes of a particle; then the sums of "warp" w of W
+		auto add_lanes = [&] {
+#pragma unroll
+			for (int m = 0; m < MT; m++)
+#pragma unroll
+				for (int e = 0; e < D; e++) {
+					gs[m][e] += __shfl_xor_sync(0xffffffffu, gs[m][e], 1);
+					gs[m][e] += __shfl_xor_sync(0xffffffffu, gs[m][e], 2);
+				}
+		};
+		auto store_sums = [&](int w) {
+			if (t == 0) {
+#pragma unroll
+				for (int m = 0; m < MT; m++)
+#pragma unroll
+					for (int e = 0; e < D; e++)
+						sh_g[(w * P + g0 + m * 8) * D + e] = gs[m][e];
+			}
+		};
+		clear_sums();
+		int wsum = warp;   // the warp of a team of one whose tasks this warp is at
 
 		for (int ph = 0; ph < a.nphase; ph++) {
 			if (ph > 0) {
@@ -662,7 +692,7 @@ __device__ __forceinline__ void line_force_body(const LineForceArgs &a, const in
 			__syncthreads();
 			const bool centres = tb.n[2] > 0;
 			const int jb = tb.hlo >> 2, je = (tb.hlo + tb.nh) >> 2;
-			const double2 *trow = tab + (size_t)g * tb.row;
+			const double2 *trow = tab + (size_t)g0 * tb.row;
 			// the weights are read one step ahead, across tasks; a task's row record one task ahead
 			const int ntask = tb.ntask * SUB;
 			int2 ri = make_int2(0, 0), rn = ri;
@@ -676,14 +706,18 @@ __device__ __forceinline__ void line_force_body(const LineForceArgs &a, const in
 				for (int n = 0; n < NT; n++)
 					bq[n] = __ldcg(w + n * 32);
 			}
-			for (int s = warp; s < ntask; s += W) {
+			for (int s = warp, sn; s < ntask; s = sn) {
 				const int r = tb.r0 + s / SUB, pair = (s % SUB) * NT;
-				const bool more = s + W < ntask;
+				sn = s + W;
+				const bool last = sn >= ntask;   // of the tasks of warp wsum
+				if (teams > 1 && last && wsum + WT < W)
+					sn = wsum + WT;
+				const bool more = sn < ntask;
 				if (more)
-					rn = row_rec(s + W);
+					rn = row_rec(sn);
 				const int nj = min(je, ri.y) - jb;   // > 0: the phase's rows all reach its first cells
 				const double2 *w = first_w(s, ri);
-				const double2 *wn = more ? first_w(s + W, rn) : w;
+				const double2 *wn = more ? first_w(sn, rn) : w;
 				ri = rn;
 				double2 acc[MT][NT];
 				LineIdx li[NT];
@@ -768,27 +802,26 @@ __device__ __forceinline__ void line_force_body(const LineForceArgs &a, const in
 						gs[m][D - 1] = fma(kl, S[m][n], gs[m][D - 1]);
 					}
 				}
+				if (teams > 1 && last && more) {
+					add_lanes();
+					store_sums(wsum);
+					clear_sums();
+					wsum += WT;
+				}
 			}
 		}
 		if (tile + 1 == tile1)
 			cudaTriggerProgrammaticLaunchCompletion();
-		// the four lanes of a particle, then the warps in order
-#pragma unroll
-		for (int m = 0; m < MT; m++)
-#pragma unroll
-			for (int e = 0; e < D; e++) {
-				gs[m][e] += __shfl_xor_sync(0xffffffffu, gs[m][e], 1);
-				gs[m][e] += __shfl_xor_sync(0xffffffffu, gs[m][e], 2);
-			}
-		__syncthreads();
-		if (t == 0) {
-#pragma unroll
-			for (int m = 0; m < MT; m++)
-#pragma unroll
-				for (int e = 0; e < D; e++)
-					sh_g[(warp * P + m * 8 + g) * D + e] = gs[m][e];
+		add_lanes();
+		if (teams == 1)
+			__syncthreads();   // the tables are read
+		store_sums(wsum);
+		if (teams > 1 && wsum + WT < W) {   // no tasks of that warp
+			clear_sums();
+			store_sums(wsum + WT);
 		}
 		__syncthreads();
+		// the warps in order
 		if ((int)threadIdx.x < nvalid) {
 			double v[D];
 #pragma unroll
@@ -808,10 +841,11 @@ __host__ __device__ constexpr size_t line_rho_smem(int row, int chunk, int d)
 {
 	return line_pos_bytes(chunk, d) + (size_t)row * chunk * sizeof(double2);
 }
-__host__ __device__ constexpr size_t line_force_smem(int row, int mt, int warps, int d)
+__host__ __device__ constexpr size_t line_force_smem(int row, int mt, int warps, int d, int teams = 1)
 {
-	const size_t tables = (size_t)row * 8 * mt * sizeof(double2), sums = (size_t)warps * 8 * mt * d * sizeof(double);
-	return line_pos_bytes(8 * mt, d) + (tables > sums ? tables : sums);
+	const size_t tables = (size_t)row * 8 * mt * teams * sizeof(double2);
+	const size_t sums = (size_t)warps * 8 * mt * teams * d * sizeof(double);
+	return line_pos_bytes(8 * mt * teams, d) + (teams > 1 ? tables + sums : tables > sums ? tables : sums);
 }
 
 // 8 warps: two blocks to an SM; 16 warps: one, for grids of one wave (8 warps alone on an SM leave its matrix units idle
@@ -864,9 +898,9 @@ template <int D> __device__ __noinline__ void line_rho_call(const LineRhoArgs &r
 constexpr int kLineBatchMT = 3;      // tiles of 8 particles in a batch's force tile
 template <int D> __device__ __noinline__ void line_force_call(const LineForceArgs &f, int local, const ItemCtl &ctl)
 {
-	constexpr int P = 8 * kLineBatchMT;
+	const int P = 8 * kLineBatchMT * f.teams;
 	const int ntile = (f.N + P - 1) / P, t0 = local * f.tiles;
-	line_force_body<D, kLineBatchMT, 8>(f, t0, min(ntile, t0 + f.tiles), ctl);
+	line_force_body<D, kLineBatchMT, 8>(f, t0, min(ntile, t0 + f.tiles), ctl, f.teams);
 }
 template <int D, bool MIXED> __device__ __noinline__ void seg_rho_call(const RhoArgs &r, int ng, int local, const ItemCtl &ctl)
 {
@@ -945,6 +979,19 @@ __device__ __forceinline__ void lbatch_item(const LBatchArgs &L, int phase, int 
 	}
 }
 
+// Queue position -> (phase, instance, item within the phase), phase by phase: by the time an instance's force items come up,
+// its reduce items are long done. (Its force items straight behind its reduce items, as cc_mbatch_kernel has them, waited 5
+// us for them in every block, instance after instance: 48 uneven instances 210 us, with this order 177.)
+__device__ __forceinline__ int4 lbatch_decode(const MBatchArgs &A, int item)
+{
+	int phase = 0, at = item;
+	while (phase < 2 && at >= A.total[phase])
+		at -= A.total[phase++];
+	const int *pre = A.pre + phase * (A.B + 1);
+	const int b = find_instance(pre, A.B, at);
+	return make_int4(item, phase, b, at - __ldg(pre + b));
+}
+
 template <int MODE>
 __global__ void __launch_bounds__(kMBatchThreads, MODE == 1 ? 3 : 2) cc_lbatch_kernel(LBatchArgs L)
 {
@@ -955,8 +1002,8 @@ __global__ void __launch_bounds__(kMBatchThreads, MODE == 1 ? 3 : 2) cc_lbatch_k
 	for (;;) {
 		__syncthreads();
 		if (threadIdx.x == 0) {
-			const int item = (int)atomicAdd(A.queue, 1u);
-			sh_item = item < T ? mbatch_decode(A, item) : make_int4(item, 0, 0, 0);
+			const int item = (int)atomicAdd(A.queue, 1u);   // (taken early, before the last item's end, the tail grows: 187 -> 204 us)
+			sh_item = item < T ? lbatch_decode(A, item) : make_int4(item, 0, 0, 0);
 		}
 		__syncthreads();
 		const int4 it = sh_item;

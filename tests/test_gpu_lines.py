@@ -135,3 +135,35 @@ def test_auto_path(gpu, d, N, chi):
     p.set_path(gpu.PATH_NUFFT if fp64 == "nufft" else gpu.PATH_SPLIT)
     E1, F1 = p.energy_and_forces()
     assert E == E1 and np.array_equal(F, F1)
+
+
+def test_batch_tiles_teams(gpu):
+    """A batch with many force tiles (two teams of warps per tile of 48 particles, several tiles per item, twice the
+    particles per rho item): bitwise what each instance gives in a batch of one, and the single evaluation to 1e-12 of
+    the scales. Particle counts around the tiles of 24 and 48 and the rho items of 64 and 128; the last set's tables
+    are too long for teams."""
+    shapes = [(d, N, 0.4) for d in (2, 3) for N in (23, 24, 25, 47, 48, 49, 97, 433, 640, 641, 1279, 1280, 1281)]
+    shapes += [(2, 20001, 0.02), (3, 15000, 0.02), (2, 6000, 0.9)]
+    assert sum((N + 23) // 24 for _, N, _ in shapes) >= 1.5 * 296
+    rng = np.random.default_rng(3)
+    pots, fracs = [], []
+    for d, N, chi in shapes:
+        basis = np.eye(d) * N ** (1 / d)
+        modes, V = gpu.stealthy_kset(d, basis, N, chi, 3)
+        pots.append(gpu.CCPotential(d, basis, modes, V))
+        fracs.append(rng.random((N, d)))
+    b = gpu.CCBatch(pots, [N for _, N, _ in shapes])
+    b.set_positions(fracs)
+    E, F = b.energy_and_forces()
+    for k, (d, N, _) in enumerate(shapes):
+        one = gpu.CCBatch([pots[k]], [N])
+        one.set_positions([fracs[k]])
+        e1, f1 = one.energy_and_forces()
+        assert e1[0] == E[k] and np.array_equal(f1[0], F[k]), (d, N)
+        pots[k].set_path(gpu.PATH_SPLIT)
+        pots[k].set_configuration(fracs[k])
+        e, f = pots[k].energy_and_forces()
+        modes, V = gpu.stealthy_kset(d, np.eye(d) * N ** (1 / d), N, shapes[k][2], 3)
+        kmax = 2 * np.pi * np.sqrt((np.asarray(modes, float) ** 2).sum(1)).max() / N ** (1 / d)
+        assert abs(E[k] - e) <= 1e-12 * V.sum() * N
+        assert np.abs(F[k] - f).max() <= 1e-12 * 4 * V.sum() * kmax
