@@ -93,8 +93,14 @@ constexpr int kLbMaxBlocks = 64;   // cap of the batched minimisation and the se
 // w + 16, ... over the chunk (every lane up to 8 variables, loads issued together), so the pairs' loads run in
 // parallel across warps instead of one pair after another. Sums have a fixed order (lanes by a fixed tree, chunks in
 // order, warps in order for the non-pair products), so a run repeats bitwise.
-constexpr int kLbDotsThreads = 2 * kLbThreads;   // a chunk of kLbThreads variables; twice as many warps over the pairs
-static __global__ void __launch_bounds__(kLbDotsThreads) lb_dots_kernel(const LbInst *insts, int cap, LbInst one)
+// PAIRS history pairs per warp and step, their loads in flight together. A single instance's few blocks are bound by latency:
+// 16 warps, two pairs (128 registers). The multi-instance launches have hundreds of blocks, most of them past the end of
+// smaller instances; 8 warps of one pair in 80 registers run three of them to an SM instead of one: 48 uneven instances 25 to
+// 40 us per step -> 11 to 19. A pair's sums do not depend on either, and warps past the chunk's 256 variables add zeros
+// to the other products, so an instance's results are the same in both.
+template <int THREADS, int PAIRS>
+static __global__ void __launch_bounds__(THREADS, PAIRS == 1 ? 3 : 1)
+    lb_dots_kernel(const LbInst *insts, int cap, LbInst one)
 {
 	cudaGridDependencySynchronize();   // launched early (programmatic dependent launch): the evaluation is complete
 	const LbInst in = insts ? insts[blockIdx.y] : one;
@@ -102,7 +108,7 @@ static __global__ void __launch_bounds__(kLbDotsThreads) lb_dots_kernel(const Lb
 	const int nblk = lb_blocks(in.n, cap);
 	if ((int)blockIdx.x >= nblk)
 		return;
-	constexpr int kWarps = kLbDotsThreads / 32;
+	constexpr int kWarps = THREADS / 32;
 	const int m = in.m, nd = lb_ndots(m);
 	const int per = (in.n + nblk - 1) / nblk;
 	const int j0 = blockIdx.x * per, j1 = min(in.n, j0 + per);
@@ -124,7 +130,7 @@ static __global__ void __launch_bounds__(kLbDotsThreads) lb_dots_kernel(const Lb
 	if (status != kLbRunning)
 		return;
 	double a[6] = {0, 0, 0, 0, 0, 0};
-	for (int k = threadIdx.x; k < 5 * count; k += kLbDotsThreads)
+	for (int k = threadIdx.x; k < 5 * count; k += THREADS)
 		pr[k] = 0.0;
 	for (int c0 = j0; c0 < j1; c0 += kLbThreads) {
 		const int cn = min(kLbThreads, j1 - c0);
@@ -150,51 +156,47 @@ static __global__ void __launch_bounds__(kLbDotsThreads) lb_dots_kernel(const Lb
 			ssn[threadIdx.x] = sj;
 		}
 		__syncthreads();
-		// two history pairs per step (i and i + kWarps): both pairs' loads are in flight together
-		for (int i = warp; i < count; i += 2 * kWarps) {
-			const int i2 = i + kWarps;
-			const bool two = i2 < count;
-			const double *s = in.S + (size_t)i * in.n + c0, *y = in.Y + (size_t)i * in.n + c0;
-			const double *s2 = in.S + (size_t)(two ? i2 : i) * in.n + c0, *y2 = in.Y + (size_t)(two ? i2 : i) * in.n + c0;
-			double si[kLbThreads / 32], yi[kLbThreads / 32], si2[kLbThreads / 32], yi2[kLbThreads / 32];
+		for (int i = warp; i < count; i += PAIRS * kWarps) {
+			double si[PAIRS][kLbThreads / 32], yi[PAIRS][kLbThreads / 32];
 #pragma unroll
-			for (int e = 0; e < kLbThreads / 32; e++) {
-				const int k = lane + 32 * e;
-				si[e] = k < cn ? s[k] : 0.0;
-				yi[e] = k < cn ? y[k] : 0.0;
-				si2[e] = k < cn && two ? s2[k] : 0.0;
-				yi2[e] = k < cn && two ? y2[k] : 0.0;
+			for (int p = 0; p < PAIRS; p++) {
+				const int ip = i + p * kWarps;
+				const bool on = ip < count;
+				const double *s = in.S + (size_t)(on ? ip : i) * in.n + c0, *y = in.Y + (size_t)(on ? ip : i) * in.n + c0;
+#pragma unroll
+				for (int e = 0; e < kLbThreads / 32; e++) {
+					const int k = lane + 32 * e;
+					si[p][e] = k < cn && on ? s[k] : 0.0;
+					yi[p][e] = k < cn && on ? y[k] : 0.0;
+				}
 			}
-			double b[5] = {0, 0, 0, 0, 0}, b2[5] = {0, 0, 0, 0, 0};
+			double b[PAIRS][5] = {};
 #pragma unroll
 			for (int e = 0; e < kLbThreads / 32; e++) {
 				const int k = lane + 32 * e;
 				if (k < cn) {
-					b[0] += si[e] * sgt[k];
-					b[1] += yi[e] * sgt[k];
-					b[2] += si[e] * syn[k];
-					b[3] += yi[e] * syn[k];
-					b[4] += yi[e] * ssn[k];
-					b2[0] += si2[e] * sgt[k];
-					b2[1] += yi2[e] * sgt[k];
-					b2[2] += si2[e] * syn[k];
-					b2[3] += yi2[e] * syn[k];
-					b2[4] += yi2[e] * ssn[k];
+					const double gt = sgt[k], yn = syn[k], sn = ssn[k];
+#pragma unroll
+					for (int p = 0; p < PAIRS; p++) {
+						b[p][0] += si[p][e] * gt;
+						b[p][1] += yi[p][e] * gt;
+						b[p][2] += si[p][e] * yn;
+						b[p][3] += yi[p][e] * yn;
+						b[p][4] += yi[p][e] * sn;
+					}
 				}
 			}
 #pragma unroll
-			for (int k = 0; k < 5; k++)
-				for (int o = 16; o > 0; o >>= 1) {
-					b[k] += __shfl_down_sync(0xffffffffu, b[k], o);
-					b2[k] += __shfl_down_sync(0xffffffffu, b2[k], o);
-				}
-			if (lane == 0) {
+			for (int p = 0; p < PAIRS; p++)
+#pragma unroll
 				for (int k = 0; k < 5; k++)
-					pr[5 * i + k] += b[k];
-				if (two)
-					for (int k = 0; k < 5; k++)
-						pr[5 * i2 + k] += b2[k];
-			}
+					for (int o = 16; o > 0; o >>= 1)
+						b[p][k] += __shfl_down_sync(0xffffffffu, b[p][k], o);
+			if (lane == 0)
+				for (int p = 0; p < PAIRS; p++)
+					if (i + p * kWarps < count)
+						for (int k = 0; k < 5; k++)
+							pr[5 * (i + p * kWarps) + k] += b[p][k];
 		}
 	}
 #pragma unroll
@@ -208,7 +210,7 @@ static __global__ void __launch_bounds__(kLbDotsThreads) lb_dots_kernel(const Lb
 			red[warp][k] = a[k];
 	__syncthreads();
 	double *out = in.part + (size_t)blockIdx.x * nd;
-	for (int k = threadIdx.x; k < nd; k += kLbDotsThreads) {
+	for (int k = threadIdx.x; k < nd; k += THREADS) {
 		if (k < 5 * m) {
 			out[k] = k / 5 < count ? pr[k] : 0.0;
 			continue;
@@ -760,8 +762,9 @@ static inline cudaError_t lb_step(const LbInst *insts, int count, int cap, int m
 	cfg.attrs = attr;
 	cfg.numAttrs = 1;
 	cfg.gridDim = dim3(cap, count);
-	cfg.blockDim = dim3(kLbDotsThreads);
-	cudaError_t e = cudaLaunchKernelEx(&cfg, lb_dots_kernel, insts, cap, o);
+	cfg.blockDim = dim3(count == 1 ? 2 * kLbThreads : kLbThreads);
+	cudaError_t e = count == 1 ? cudaLaunchKernelEx(&cfg, lb_dots_kernel<2 * kLbThreads, 2>, insts, cap, o)
+	                           : cudaLaunchKernelEx(&cfg, lb_dots_kernel<kLbThreads, 1>, insts, cap, o);
 	if (e != cudaSuccess)
 		return e;
 	cfg.gridDim = dim3(count);
