@@ -1261,24 +1261,28 @@ __device__ __forceinline__ int4 mbatch_decode(const MBatchArgs &A, int item)
 	return within < nred ? make_int4(item, 1, b, within) : make_int4(item, 2, b, within - nred);
 }
 
-// Count a finished item (queue position, phase, instance, item within the phase).
+// Count a finished item (queue position, phase, instance, item within the phase): one thread, once the block's results are
+// visible.
+__device__ __forceinline__ void mbatch_count(const MBatchArgs &A, const int4 it)
+{
+	const int phase = it.y, b = it.z;
+	const int *pre = A.pre + phase * (A.B + 1);
+	unsigned *cnt = A.count + phase * A.B + b;
+	const unsigned done = atomicAdd(cnt, 1u) + 1u;
+	if (phase == 2 && done == (unsigned)(__ldg(pre + b + 1) - __ldg(pre + b))) {
+		// the instance's last item: its counts start from zero in the next launch
+		A.count[b] = 0u;
+		A.count[A.B + b] = 0u;
+		*cnt = 0u;
+	}
+}
 __device__ __forceinline__ void mbatch_done(const MBatchArgs &A, const int4 it)
 {
 	// the item's results are visible before its count rises
 	__threadfence();
 	__syncthreads();
-	if (threadIdx.x == 0) {
-		const int phase = it.y, b = it.z;
-		const int *pre = A.pre + phase * (A.B + 1);
-		unsigned *cnt = A.count + phase * A.B + b;
-		const unsigned done = atomicAdd(cnt, 1u) + 1u;
-		if (phase == 2 && done == (unsigned)(__ldg(pre + b + 1) - __ldg(pre + b))) {
-			// the instance's last item: its counts start from zero in the next launch
-			A.count[b] = 0u;
-			A.count[A.B + b] = 0u;
-			*cnt = 0u;
-		}
-	}
+	if (threadIdx.x == 0)
+		mbatch_count(A, it);
 }
 
 template <int MODE>

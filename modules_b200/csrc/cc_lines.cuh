@@ -20,6 +20,7 @@
 // index and within the columns is free as long as both factors agree on it; the layouts below are chosen so that a lane
 // holds all of a cell (rho) and so that the weights of the forces are read in fragment order.
 #pragma once
+#include <type_traits>
 #include "cc_kernels.cuh"
 
 namespace cc {
@@ -884,11 +885,16 @@ union LineItemDesc {
 	LineReduceArgs lred;
 	LineForceArgs lforce;
 };
-__device__ __forceinline__ LineItemDesc &line_item_desc()
-{
-	__shared__ LineItemDesc s;
-	return s;
-}
+// An item taken from the queue: its place there (it.x), phase, instance and item within the phase, and everything uniform that
+// its body starts from.
+struct LineItem {
+	int4 it;
+	int dim, count;          // items that do work; those beyond them are empty
+	int line, mixed, shape;  // line items; the segment items' precision and groups
+	unsigned need;           // the count its phase waits for
+	const int *stage;
+	LineItemDesc desc;
+};
 
 // The bodies as calls: inlined together into one kernel they spill (1.4 KB a thread at 128 registers).
 template <int D> __device__ __noinline__ void line_rho_call(const LineRhoArgs &r, int local, const ItemCtl &ctl)
@@ -913,34 +919,28 @@ template <int D, bool MIXED> __device__ __noinline__ void seg_force_call(const F
 
 // MODE as mbatch_item: 0 FP64, 1 mixed, 2 each instance at the precision of its stage word
 template <int D, int MODE>
-__device__ __forceinline__ void lbatch_item(const LBatchArgs &L, int phase, int b, int local)
+__device__ __forceinline__ void lbatch_item(const MBatchArgs &A, const LineItem &s)
 {
-	const MBatchArgs &A = L.m;
+	const int phase = s.it.y, b = s.it.z, local = s.it.w;
 	ItemCtl ctl;
 	ctl.err = A.count + 3 * A.B;
 	ctl.ready_spins = A.spins;
 	ctl.want_stage = A.want_stage;
-	const int *stage = A.rho[b].stage;
-	const bool mixed = MODE == 1 || (MODE == 2 && stage && *(volatile const int *)stage == 0);
-	const int nline = __ldg(L.own + (3 + phase) * A.B + b);
-	const bool line = !mixed && D >= 2 && nline > 0;
-	ctl.stage = MODE == 2 ? nullptr : stage;
+	ctl.stage = MODE == 2 ? nullptr : s.stage;
 	if (phase > 0) {
 		ctl.ready = A.count + (phase - 1) * A.B + b;
-		ctl.ready_need = (unsigned)(__ldg(A.pre + (phase - 1) * (A.B + 1) + b + 1) - __ldg(A.pre + (phase - 1) * (A.B + 1) + b)) +
-		                 (phase == 1 && b == 0 ? A.phantom : 0u);
+		ctl.ready_need = s.need;
 	}
-	if (local >= (line ? nline : __ldg(L.own + phase * A.B + b)))
+	if (local >= s.count)
 		return;
 	if constexpr (MODE != 1 && D >= 2) {
-		if (line) {
+		if (s.line) {
 			if (phase == 0) {
-				const LineRhoArgs &r = stage_desc(L.lrho + b, line_item_desc().lrho);
-				line_rho_call<D>(r, local, ctl);
+				line_rho_call<D>(s.desc.lrho, local, ctl);
 			} else if (phase == 1) {
-				line_reduce_wide_body(stage_desc(L.lred + b, line_item_desc().lred), local, ctl);
+				line_reduce_wide_body(s.desc.lred, local, ctl);
 			} else {
-				const LineForceArgs &f = stage_desc(L.lforce + b, line_item_desc().lforce);
+				const LineForceArgs &f = s.desc.lforce;
 				line_force_call<D>(f, local, ctl);
 				// the instance's first force item also sums the energy (its reduce items are complete)
 				if (local == 0 && f.E_out && !eval_skipped(f.skip, ctl.stage, ctl.want_stage)) {
@@ -953,29 +953,25 @@ __device__ __forceinline__ void lbatch_item(const LBatchArgs &L, int phase, int 
 		}
 	}
 	if (phase == 0) {
-		const RhoArgs &r = stage_desc(A.rho + b, line_item_desc().rho);
-		const int ng = __ldg(A.shape + b);
 		if constexpr (MODE != 0) {
-			if (mixed) {
-				seg_rho_call<D, true>(r, ng, local, ctl);
+			if (s.mixed) {
+				seg_rho_call<D, true>(s.desc.rho, s.shape, local, ctl);
 				return;
 			}
 		}
 		if constexpr (MODE != 1)
-			seg_rho_call<D, false>(r, ng, local, ctl);
+			seg_rho_call<D, false>(s.desc.rho, s.shape, local, ctl);
 	} else if (phase == 1) {
-		reduce_body_wide(stage_desc(A.red + b, line_item_desc().red), local, ctl);
+		reduce_body_wide(s.desc.red, local, ctl);
 	} else {
-		const ForceArgs &f = stage_desc(A.force + b, line_item_desc().force);
-		const int pg = __ldg(A.shape + 2 * A.B + b);
 		if constexpr (MODE != 0) {
-			if (mixed) {
-				seg_force_call<D, true>(f, pg, local, ctl);
+			if (s.mixed) {
+				seg_force_call<D, true>(s.desc.force, s.shape, local, ctl);
 				return;
 			}
 		}
 		if constexpr (MODE != 1)
-			seg_force_call<D, false>(f, pg, local, ctl);
+			seg_force_call<D, false>(s.desc.force, s.shape, local, ctl);
 	}
 }
 
@@ -992,31 +988,100 @@ __device__ __forceinline__ int4 lbatch_decode(const MBatchArgs &A, int item)
 	return make_int4(item, phase, b, at - __ldg(pre + b));
 }
 
+// The record of queue position `item` (lane 0's), by one warp.
+template <int MODE> __device__ __forceinline__ void lbatch_fetch(const LBatchArgs &L, int item, LineItem &s)
+{
+	const MBatchArgs &A = L.m;
+	const int lane = threadIdx.x & 31;
+	item = __shfl_sync(0xffffffffu, item, 0);
+	if (item >= A.total[0] + A.total[1] + A.total[2]) {
+		if (lane == 0)
+			s.it = make_int4(item, 0, 0, 0);
+		return;
+	}
+	const int4 it = lbatch_decode(A, item);
+	const int phase = it.y, b = it.z;
+	const int *stage = A.rho[b].stage;
+	const int dim = __ldg(A.dim + b), nseg = __ldg(L.own + phase * A.B + b), nline = __ldg(L.own + (3 + phase) * A.B + b);
+	const bool mixed = MODE == 1 || (MODE == 2 && stage && *(volatile const int *)stage == 0);
+	const bool line = !mixed && dim >= 2 && nline > 0;
+	auto copy = [&](const auto *src, auto &dst) {
+		using T = std::remove_reference_t<decltype(dst)>;
+		static_assert(sizeof(T) % 8 == 0 && alignof(T) >= 8, "descriptors are copied as 8-byte words");
+		const unsigned long long *from = reinterpret_cast<const unsigned long long *>(src);
+		unsigned long long *to = reinterpret_cast<unsigned long long *>(&dst);
+#pragma unroll
+		for (int w = 0; w < (int)(sizeof(T) / 8); w += 32)
+			if (w + lane < (int)(sizeof(T) / 8))
+				to[w + lane] = __ldg(from + w + lane);
+	};
+	if (phase == 0) {
+		if (line)
+			copy(L.lrho + b, s.desc.lrho);
+		else
+			copy(A.rho + b, s.desc.rho);
+	} else if (phase == 1) {
+		if (line)
+			copy(L.lred + b, s.desc.lred);
+		else
+			copy(A.red + b, s.desc.red);
+	} else {
+		if (line)
+			copy(L.lforce + b, s.desc.lforce);
+		else
+			copy(A.force + b, s.desc.force);
+	}
+	if (lane == 0) {
+		s.it = it;
+		s.dim = dim;
+		s.count = line ? nline : nseg;
+		s.line = line;
+		s.mixed = mixed;
+		s.shape = __ldg(A.shape + phase * A.B + b);
+		const int *pre = A.pre + (phase - 1) * (A.B + 1) + b;
+		s.need = phase == 0 ? 0u : (unsigned)(__ldg(pre + 1) - __ldg(pre)) + (phase == 1 && b == 0 ? A.phantom : 0u);
+		s.stage = stage;
+	}
+}
+
+// Between an item and the next one, warp 1 takes the next (position, record and descriptor: three dependent round trips) while
+// warp 0 counts the one that ended: 3 us between items before, when one thread did both in turn and the block then fetched
+// the descriptor. The count does not wait for the fetch (warp 1 only arrives at the barrier before it), and the position is not
+// taken earlier: taken at the start of an item, it kept items that others waited for behind long ones (60 instances 187 -> 204
+// us).
 template <int MODE>
 __global__ void __launch_bounds__(kMBatchThreads, MODE == 1 ? 3 : 2) cc_lbatch_kernel(LBatchArgs L)
 {
 	const MBatchArgs &A = L.m;
-	__shared__ int4 sh_item;
+	__shared__ LineItem items[2];
 	const int T = A.total[0] + A.total[1] + A.total[2];
+	const bool fetches = (threadIdx.x >> 5) == 1;
 	cudaGridDependencySynchronize();
-	for (;;) {
-		__syncthreads();
-		if (threadIdx.x == 0) {
-			const int item = (int)atomicAdd(A.queue, 1u);   // (taken early, before the last item's end, the tail grows: 187 -> 204 us)
-			sh_item = item < T ? lbatch_decode(A, item) : make_int4(item, 0, 0, 0);
+	auto take = [&] { return threadIdx.x == 32 ? (int)atomicAdd(A.queue, 1u) : 0; };
+	if (fetches)
+		lbatch_fetch<MODE>(L, take(), items[0]);
+	__syncthreads();
+	for (int at = 0;; at ^= 1) {
+		const LineItem &s = items[at];
+		if (s.it.x >= T)
+			break;
+		if (s.dim == 3)
+			lbatch_item<3, MODE>(A, s);
+		else if (s.dim == 2)
+			lbatch_item<2, MODE>(A, s);
+		else
+			lbatch_item<1, MODE>(A, s);
+		const int next = take();
+		__threadfence();   // the item's results are visible before its count rises
+		if (fetches) {
+			asm volatile("barrier.cta.arrive 1, %0;" ::"n"(kMBatchThreads) : "memory");
+			lbatch_fetch<MODE>(L, next, items[at ^ 1]);
+		} else {
+			asm volatile("barrier.cta.sync 1, %0;" ::"n"(kMBatchThreads) : "memory");
+			if (threadIdx.x == 0)
+				mbatch_count(A, s.it);
 		}
 		__syncthreads();
-		const int4 it = sh_item;
-		if (it.x >= T)
-			break;
-		const int d = __ldg(A.dim + it.z);
-		if (d == 3)
-			lbatch_item<3, MODE>(L, it.y, it.z, it.w);
-		else if (d == 2)
-			lbatch_item<2, MODE>(L, it.y, it.z, it.w);
-		else
-			lbatch_item<1, MODE>(L, it.y, it.z, it.w);
-		mbatch_done(A, it);
 	}
 	queue_leave(A.queue);
 }
