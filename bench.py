@@ -13,9 +13,10 @@ forces evaluation of one configuration. Synthetic seeded inputs (no dataset exis
           step's positions from pinned host memory to the device and E and F back, inside the timed region, the
           copies overlapped with the evaluations); `e2e.per_call` is one cc_set_positions + cc_energy_grad call per
           configuration (the reference's interface), each waiting for its result.
-  roofline: the dominant kernel's algorithmic FLOPs ((17 + 2d) per particle-k pair and evaluation: 8 in the rho
-          kernel, 9 + 2d in the force kernel) / its CUDA-event duration, against the FP64 FMA peak measured in the
-          same run by an FMA-chain probe kernel (MEASURED_PEAKS.json has no FP64 figure).
+  roofline: the dominant kernel's algorithmic FLOPs (FP64, the line kernels: 12 per particle-k pair and evaluation, 4 in
+          the rho kernel, 8 in the force kernel; mixed, the segment kernels: 17 + 2d, 8 and 9 + 2d) / its CUDA-event
+          duration, against the FP64 FMA peak measured in the same run by an FMA-chain probe kernel
+          (MEASURED_PEAKS.json has no FP64 figure).
   cpu_baseline: the reference's own ShiftedCCPotential (Energy + AllForce, oracle/_ref) on the host cores.
 
 --impl reference times that reference CPU path alone on the same workload and prints its line.
@@ -39,12 +40,14 @@ D, N, CHI = 3, 2000, 0.45
 SIDE = N ** (1.0 / 3.0)
 METRIC = "CC energy+grad evals/s"
 UNIT = "evals/s"
-# DRAM bytes (read + write) per launch of the kernels on this workload, from one ncu capture
-# (profiles/cc_kernels_3d_n2000_ncu.md: dram__bytes_read.sum + dram__bytes_write.sum)
+# Bytes per launch of the kernels on this workload, from ncu captures (profiles/line_kernels_ncu.md; the segment kernels:
+# profiles/cc_kernels_3d_n2000_ncu.md)
 # DRAM bytes (read + write) per launch at this workload from ncu captures with ncu's default cache flush before each
 # pass (cold); with warm caches (--cache-control none) each of the three kernels reads about 256 bytes of DRAM
-NCU_TRAFFIC_BYTES = {"cc_force_kernel": 0.149e6, "cc_rho_kernel": 0.028e6, "cc_reduce_kernel": 1.418e6}
-NCU_L2_BYTES_WARM = {"cc_force_kernel": 5.45e6, "cc_rho_kernel": 3.24e6, "cc_reduce_kernel": 2.23e6}
+NCU_TRAFFIC_BYTES = {"cc_line_force_kernel": 0.203e6, "cc_line_rho_kernel": 0.024e6, "cc_line_reduce_kernel": 5.07e6,
+                     "cc_force_kernel": 0.149e6, "cc_rho_kernel": 0.028e6, "cc_reduce_kernel": 1.418e6}
+NCU_L2_BYTES_WARM = {"cc_line_force_kernel": 9.0e6, "cc_line_rho_kernel": 8.7e6, "cc_line_reduce_kernel": 7.5e6,
+                     "cc_force_kernel": 5.45e6, "cc_rho_kernel": 3.24e6, "cc_reduce_kernel": 2.23e6}
 WORKLOAD = "3D stealthy CC ground-state evaluation: N=2000 uniform in a periodic cube (unit density), chi=0.45, " \
            "M=2724 half-space k (v=1), FP64 energy + Cartesian forces"
 DATA = "synthetic (seeded uniform positions; k-set of the reference CLI's Type 0 rule)"
@@ -192,7 +195,11 @@ def run_reference(args):
     if rank != 0:
         return
     cores = os.cpu_count() or 1
-    ref, M = reference_potential(cores)
+    try:
+        ref, M = reference_potential(cores)
+    except RuntimeError as exc:   # (the reference's sources were absent when this tree was built)
+        print(json.dumps({"impl": "reference", "unavailable": str(exc)}), flush=True)
+        return
     P = args.pool
     pool = pool_positions(P)
     t0 = time.perf_counter()
@@ -588,12 +595,12 @@ def run_ours(args):
     pairs = N * M
     t_rho, t_red, t_force = rho_ms / nt, red_ms / nt, force_ms / nt
     peak = cc.probe_fma_peak(cc.PREC_FP64 if prec == cc.PREC_FP64 else cc.PREC_MIXED)
-    rho_flops, force_flops = 8.0 * pairs, (9.0 + 2 * D) * pairs
-    # the dominant kernel is the force kernel: the largest share of the evaluation's device time in the ncu launch
-    # list (42.8 % against rho 41.9 %) and of its FLOPs; their CUDA-event intervals are within a few percent of
-    # each other and either can come out longer in a given run, so both are reported
-    dom, fl, tk = "cc_force_kernel", force_flops, t_force
-    kernel_ms = {"cc_rho_kernel": t_rho, "cc_reduce_kernel": t_red, "cc_force_kernel": t_force}
+    # the dominant kernel is the force kernel: the larger share of the evaluation's FLOPs; the CUDA-event intervals of the
+    # rho and force kernels are close and either can come out longer in a given run, so both are reported
+    kind = "cc_line_" if prec == cc.PREC_FP64 else "cc_"
+    rho_flops, force_flops = (4.0 * pairs, 8.0 * pairs) if prec == cc.PREC_FP64 else (8.0 * pairs, (9.0 + 2 * D) * pairs)
+    dom, fl, tk = kind + "force_kernel", force_flops, t_force
+    kernel_ms = {kind + "rho_kernel": t_rho, kind + "reduce_kernel": t_red, kind + "force_kernel": t_force}
     launches_per_eval = 3
     achieved = fl / (tk * 1e-3) / 1e12
 

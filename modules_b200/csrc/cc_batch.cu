@@ -1,7 +1,7 @@
 // cc_batch.cu — batches of independent configurations (cc_batch_* in include/cc_gpu.h).
 //
 // A batch evaluates many configurations of uneven size and dimension together: ONE launch of the fused batch kernel
-// (cc_mbatch_kernel, cc_kernels.cuh) per energy + gradient step, whose work queue holds the rho blocks, split-reduction
+// (cc_lbatch_kernel, cc_lines.cuh; cc_mbatch_kernel, cc_kernels.cuh, where no instance has a line plan) per energy + gradient step, whose work queue holds the rho blocks, split-reduction
 // chunks and force blocks of every instance; per-instance completion counts order the three phases of an instance.
 // Its batched L-BFGS (cc_batch_minimize) keeps every instance's positions, gradient and history on the device and
 // enqueues blocks of iterations (one fused evaluation and the L-BFGS kernels each). The reference

@@ -1,10 +1,11 @@
 // cc_capi.cu — the C ABI of libccgpu.so (declared in include/cc_gpu.h): handles, k-set planning, launches.
 //
 // A handle holds the constraint set of one ShiftedCCPotential (potential/CollectiveCoordinatePotential.h:84-117)
-// planned into lattice-line segments (see cc_kernels.cuh), the cell (volume, reciprocal basis) and the device
-// buffers of the bound positions. One evaluation is two kernel launches on the handle's stream:
-//   cc_rho_kernel   -> rho per slot, u = V conj(rho), the energy (and rho in mode order on request);
-//   cc_force_kernel -> Cartesian forces and/or the gradient in fractional coordinates.
+// planned into lattice-line segments (see cc_kernels.cuh) and lines (see cc_lines.cuh), the cell (volume, reciprocal
+// basis) and the device buffers of the bound positions. One evaluation is three kernel launches on the handle's stream
+// (cc_line_* in FP64, cc_* in mixed precision and for sets without a line plan):
+//   rho, reduce -> rho per slot, the force weights, the energy (and rho in mode order on request);
+//   force       -> Cartesian forces and/or the gradient in fractional coordinates.
 // There is no CPU path: without a CUDA device every call that computes returns CC_ERR_NOGPU.
 #include "../../include/cc_gpu.h"
 #include "cc_internal.h"

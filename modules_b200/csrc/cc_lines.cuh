@@ -279,7 +279,7 @@ struct LineReduceArgs {
 	const double2 *cellS0;    // S2 targets, or null
 	double npart;
 	double rho_offset;
-	double2 *rho_slot;            // rho per slot
+	double2 *rho_slot;        // rho per slot
 	double2 *weights;         // force weights in fragment order (may be null)
 	double *eblock;           // [blocks]
 	unsigned *ticket;
