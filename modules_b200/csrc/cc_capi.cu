@@ -1250,12 +1250,12 @@ cudaEvent_t next_event(cc_handle *h)
 // 7.2e-12 s per fine-grid point and transform and 80 us) and, in FP64 on the line kernels, also below the direct path's there.
 // The second condition only takes calls off the NUFFT path: its forces are within 7e-13 of 64-bit sums, the line kernels' within
 // 1e-14 (relative, worst component), so no set goes to it for the few tens of microseconds that it would save between the two.
-// 0.8: calls one after another (not in one graph) overlap on the NUFFT path's streams, 3D N=30000 chi=0.3 347 us against 452.
+// 0.8: calls one after another (not in one graph) overlap on the NUFFT path's streams, 2D N=20000 chi=0.2 28 us.
 // Its estimates are fits to evaluations in CUDA graphs on B200 (27 sets, 2D and 3D, N = 3000 to 100000, chi = 0.05 to 0.49; the
 // direct one within 13 %, mostly 5 %): direct 8.8 us + 59 ps per particle and unit + 39 ps per particle and row of lines in 3D +
-// 0.28 ns per particle; NUFFT 24 us + 0.62 ns per particle + 40 ps per grid point in 2D, 70 us + 9.3 ns + 90 ps in 3D. Measured,
-// direct against NUFFT: 2D N=20000 chi=0.05 42.6 / 39.2 us, chi=0.2 102.9 / 40.2; 3D N=20000 chi=0.49 363 / 348, N=30000 chi=0.2
-// 378 / 384, chi=0.45 698 / 422, N=60000 chi=0.05 379 / 650, N=100000 chi=0.05 963 / 1022.
+// 0.28 ns per particle; NUFFT 24 us + 0.62 ns per particle + 40 ps per grid point in 2D, 70 us + 7.3 ns + 90 ps in 3D. Measured,
+// direct against NUFFT: 2D N=20000 chi=0.05 42.7 / 40.2 us, chi=0.2 102.9 / 40.2; 3D N=20000 chi=0.2 172 / 226, chi=0.49 363 /
+// 293, N=30000 chi=0.2 378 / 316, chi=0.45 699 / 352, N=60000 chi=0.05 379 / 551, N=100000 chi=0.05 964 / 868.
 bool nufft_preferred(cc_handle *h, int64_t N, bool mixed)
 {
 	if (h->main.plan.nslot == 0 || N < 1024 || h->d_slotS0)
@@ -1284,7 +1284,7 @@ bool nufft_preferred(cc_handle *h, int64_t N, bool mixed)
 		return 1.2 * nufft < direct;
 	const double n = (double)N;
 	const double direct_us = 8.8 + 59e-6 * n * L.nunit + (d == 3 ? 39e-6 * n * (double)L.rows.size() : 0.0) + 2.8e-4 * n;
-	const double nufft_us = d == 2 ? 24.0 + 6.2e-4 * n + 4e-5 * grid : 70.0 + 9.3e-3 * n + 9e-5 * grid;
+	const double nufft_us = d == 2 ? 24.0 + 6.2e-4 * n + 4e-5 * grid : 70.0 + 7.3e-3 * n + 9e-5 * grid;
 	return 0.8 * nufft_us < direct_us;
 }
 

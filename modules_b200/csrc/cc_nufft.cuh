@@ -53,12 +53,19 @@ struct NufftDev {
 
 __device__ __forceinline__ double es_kernel(double t, double beta)
 {
-	const double z = 1.0 - (2.0 * t / kNufftW) * (2.0 * t / kNufftW);
+	const double u = t * (2.0 / kNufftW), z = 1.0 - u * u;
 	return z > 0.0 ? exp(beta * (sqrt(z) - 1.0)) : 0.0;
 }
 
+// g modulo n; without a division for g within one period of [0, n), as every index of coordinates in [0, 1) is
 __device__ __forceinline__ int wrap_index(int g, int n)
 {
+	if (g < 0)
+		g += n;
+	else if (g >= n)
+		g -= n;
+	if ((unsigned)g < (unsigned)n)
+		return g;
 	g %= n;
 	return g < 0 ? g + n : g;
 }
@@ -94,7 +101,9 @@ __device__ __forceinline__ bool nufft_weights(const NufftDev &a, const double *f
 
 // Type-1 spread: 16 lanes per particle; lane t adds the particle's weights of last-axis point g_last + t, row by row
 // of the other axes (a particle's 14 lanes hit 14 consecutive grid words), in fixed point (integer atomics: the sum
-// does not depend on their order).
+// does not depend on their order). In 2D it is bound by the atomics (L1 76 % busy; a third fewer instructions changed
+// nothing, nor did particles in tile order: 33 us at N = 1e5); in 3D by instructions, so its rows' addresses are one stride
+// apart except where they wrap (N = 60000, the whole evaluation 694 -> 591 us, with the interpolation).
 template <int D> __global__ void __launch_bounds__(kNufftThreads) nufft_spread_kernel(NufftDev a, const double *frac, int N)
 {
 	__shared__ double sk[kNufftPerBlock][3][kNufftW];
@@ -107,24 +116,31 @@ template <int D> __global__ void __launch_bounds__(kNufftThreads) nufft_spread_k
 		return;
 	constexpr int L = D - 1;
 	const int il = wrap_index(sg0[p][L] + t, a.nf[L]);
-	const double wl = sk[p][L][t];
+	const double wl = sk[p][L][t] * kNufftFix;   // (a power of two: exact)
+	auto add = [](unsigned long long *q, double w) { atomicAdd(q, (unsigned long long)llrint(w)); };
 	if constexpr (D == 1) {
-		atomicAdd(a.gi + il, (unsigned long long)llrint(wl * kNufftFix));
-	} else {
+		add(a.gi + il, wl);
+	} else if constexpr (D == 2) {
 		int i0 = wrap_index(sg0[p][0], a.nf[0]);
 #pragma unroll 2
+		for (int t0 = 0; t0 < kNufftW; t0++, i0 = wrap_next(i0, a.nf[0]))
+			add(a.gi + (size_t)i0 * a.nf[1] + il, sk[p][0][t0] * wl);
+	} else {
+		int i0 = wrap_index(sg0[p][0], a.nf[0]);
+		const int i1s = wrap_index(sg0[p][1], a.nf[1]);
+#pragma unroll 1
 		for (int t0 = 0; t0 < kNufftW; t0++, i0 = wrap_next(i0, a.nf[0])) {
-			const double w0 = sk[p][0][t0];
-			if constexpr (D == 2) {
-				atomicAdd(a.gi + (size_t)i0 * a.nf[1] + il, (unsigned long long)llrint(w0 * wl * kNufftFix));
+			unsigned long long *plane = a.gi + (size_t)i0 * a.nf[1] * a.nf[2] + il;
+			const double w = sk[p][0][t0] * wl;
+			if (i1s + kNufftW <= a.nf[1]) {   // rows one stride apart
+				unsigned long long *q = plane + (size_t)i1s * a.nf[2];
+#pragma unroll
+				for (int t1 = 0; t1 < kNufftW; t1++)
+					add(q + t1 * a.nf[2], sk[p][1][t1] * w);
 			} else {
-				int i1 = wrap_index(sg0[p][1], a.nf[1]);
-#pragma unroll 7
-				for (int t1 = 0; t1 < kNufftW; t1++, i1 = wrap_next(i1, a.nf[1])) {
-					const double w01 = w0 * sk[p][1][t1];
-					atomicAdd(a.gi + ((size_t)i0 * a.nf[1] + i1) * a.nf[2] + il,
-					          (unsigned long long)llrint(w01 * wl * kNufftFix));
-				}
+				int i1 = i1s;
+				for (int t1 = 0; t1 < kNufftW; t1++, i1 = wrap_next(i1, a.nf[1]))
+					add(plane + (size_t)i1 * a.nf[2], sk[p][1][t1] * w);
 			}
 		}
 	}
@@ -303,7 +319,8 @@ struct NufftOut {
 
 // type-2 interpolation: 16 lanes per particle; lane t sums the last-axis point g_last + t over the rows of the other
 // axes (a particle's 14 lanes read 14 consecutive grid words), the lanes' sums are added in a fixed butterfly;
-// g_e = sum_g phi G_e[g] and the forces as the direct force kernel
+// g_e = sum_g phi G_e[g] and the forces as the direct force kernel. Bound by instructions and, in 2D, by the loads in
+// flight (the strided form of 3D takes 70 registers there: 37 -> 40 us at N = 1e5).
 template <int D>
 __global__ void __launch_bounds__(kNufftThreads) nufft_interp_kernel(NufftDev a, const double *frac, int N,
                                                                      int64_t ngrid, NufftOut o)
@@ -347,19 +364,27 @@ __global__ void __launch_bounds__(kNufftThreads) nufft_interp_kernel(NufftDev a,
 			int i0 = wrap_index(sg0[p][0], a.nf[0]);
 			const int i1s = wrap_index(sg0[p][1], a.nf[1]);
 			for (int t0 = 0; t0 < kNufftW; t0++, i0 = wrap_next(i0, a.nf[0])) {
-				const double w0 = sk[p][0][t0];
-				int i1 = i1s;
+				const double *plane = a.gim + (size_t)i0 * a.nf[1] * a.nf[2] + il;
+				const double w0 = sk[p][0][t0] * wl;
 				double v[kNufftW][D];
-#pragma unroll
-				for (int t1 = 0; t1 < kNufftW; t1++, i1 = wrap_next(i1, a.nf[1])) {
-					const size_t idx = ((size_t)i0 * a.nf[1] + i1) * a.nf[2] + il;
+				if (i1s + kNufftW <= a.nf[1]) {   // rows one stride apart
+					const double *q = plane + (size_t)i1s * a.nf[2];
 #pragma unroll
 					for (int e = 0; e < D; e++)
-						v[t1][e] = __ldg(a.gim + (size_t)e * ngrid + idx);
+#pragma unroll
+						for (int t1 = 0; t1 < kNufftW; t1++)
+							v[t1][e] = __ldg(q + (size_t)e * ngrid + t1 * a.nf[2]);
+				} else {
+					int i1 = i1s;
+#pragma unroll
+					for (int t1 = 0; t1 < kNufftW; t1++, i1 = wrap_next(i1, a.nf[1]))
+#pragma unroll
+						for (int e = 0; e < D; e++)
+							v[t1][e] = __ldg(plane + (size_t)e * ngrid + (size_t)i1 * a.nf[2]);
 				}
 #pragma unroll
 				for (int t1 = 0; t1 < kNufftW; t1++) {
-					const double w = w0 * sk[p][1][t1] * wl;
+					const double w = sk[p][1][t1] * w0;
 #pragma unroll
 					for (int e = 0; e < D; e++)
 						acc[e] = fma(w, v[t1][e], acc[e]);
