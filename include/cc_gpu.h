@@ -245,8 +245,8 @@ const char *cc_serve_last_error(void);
  * cc_set_positions + cc_energy_grad (coordinates outside [0,1) are wrapped the same way; a non-finite one fails the
  * call with CC_ERR_ARG). The positions go to the device in chunks of 64 configurations on a second stream while
  * earlier chunks are evaluated, and the evaluations follow one another without host synchronisation (each rho kernel
- * overlaps the previous evaluation's force kernel; three at a time where one does not fill the GPU); pinned host buffers (cudaHostAlloc, cudaHostRegister) let the
- * copies overlap. The call returns when E and F are written. Every configuration of a call is resident on the
+ * overlaps the previous evaluation's force kernel; three at a time where one does not fill the GPU); pinned host
+ * buffers (cudaHostAlloc, cudaHostRegister) let the copies overlap. The call returns when E and F are written. Every configuration of a call is resident on the
  * device at once (2 P N d doubles). Replaces a loop of the reference's SetConfiguration + Energy + AllForce over
  * configurations (potential/CollectiveCoordinatePotential.h:1351-1448). */
 int cc_energy_grad_many(cc_handle *h, int64_t P, int64_t N, const double *frac, double *E, double *F, int precision);
