@@ -376,6 +376,7 @@ int batch_build(cc_batch *b, int per_split, int segs_per_split)
 	    (rc = upload_into(b->d_lrho[0], b->lrho)) || (rc = upload_into(b->d_lred[0], b->lred)) ||
 	    (rc = upload_into(b->d_lforce[0], b->lforce)) || (rc = upload_into(b->d_own, own)))
 		return rc;
+	CC_CUDA(cudaStreamSynchronize(nullptr));   // (with the arena's zeros) the batch's stream does not wait for the legacy one
 	b->per_split = per_split;
 	b->segs_per_split = segs_per_split;
 	return CC_OK;
@@ -846,6 +847,7 @@ int cc_batch_minimize(cc_batch *b, double *const *frac, const cc_lbfgs_opts *opt
 		return rc;
 	if ((rc = upload_into(b->d_start, start)) || (rc = upload_into(b->d_final, final_pos)))
 		return rc;
+	CC_CUDA(cudaStreamSynchronize(nullptr));   // the batch's stream does not wait for the legacy one
 	cudaStream_t st = b->stream;
 	const bool sched = o.precision == CC_PREC_SCHEDULE;
 	CC_CUDA(cudaMemcpyAsync(b->lb_base + ox[0], b->h_pin, b->pos_bytes, cudaMemcpyHostToDevice, st));

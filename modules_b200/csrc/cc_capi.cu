@@ -93,8 +93,8 @@ int cci::get_splits(DevKSet &k, int want, const DevSplits **out)
 	return CC_OK;
 }
 
-
-// The plan's arrays (and the line plan's) go up in one copy into one allocation; what the kernels write starts at zero: slots without a mode are read (with weight 0) but never written on the line path, and the ticket starts at 0.
+// The plan's arrays (and the line plan's) go up in one copy into one allocation; what the kernels write starts at zero:
+// slots without a mode are read (with weight 0) but never written on the line path, and the ticket starts at 0.
 int cci::upload_kset(DevKSet &k, const cc::Plan &plan)
 {
 	k.release();
@@ -145,6 +145,7 @@ int cci::upload_kset(DevKSet &k, const cc::Plan &plan)
 		CC_CUDA(cudaMemcpy(k.blob, up.data(), up.size(), cudaMemcpyHostToDevice));
 	CC_CUDA(cudaMemset(k.blob + up.size(), 0, end - up.size()));
 	CC_CUDA(cudaMemset(k.rho_slot, 0, 2 * nslot * sizeof(double2)));
+	CC_CUDA(cudaStreamSynchronize(nullptr));   // the evaluations' streams do not wait for the legacy one
 	unsigned char *b = k.blob;
 	k.segs = reinterpret_cast<cc::Seg *>(b + o_segs);
 	k.bstart = reinterpret_cast<int *>(b + o_bstart);
@@ -2225,7 +2226,7 @@ int cc_mc_try_move(cc_handle *h, const double *s_prev, const double *s_after, do
 		    (rc = dev_alloc(&h->d_rho_trial, M)) || (rc = dev_alloc(&h->d_rho_cur, M)) ||
 		    (rc = dev_alloc(&h->d_mc_part, nb + 1)))
 			return rc;
-		CC_CUDA(cudaMemset(h->d_mc_part, 0, (nb + 1) * sizeof(double)));   // [nb]: the blocks' ticket
+		CC_CUDA(cudaMemsetAsync(h->d_mc_part, 0, (nb + 1) * sizeof(double), h->stream));   // [nb]: the blocks' ticket
 	}
 	if (!h->mc_valid) {
 		// rho of the bound positions in mode order (FP64), as the cached RhoReal / RhoImag of the reference
