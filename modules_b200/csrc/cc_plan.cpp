@@ -308,9 +308,9 @@ bool line_groups(const LinePlan &L, int d, bool centres, int ntask, int most, Li
 		for (int i = 0, top = shares(r2); i < top; i++) {
 			const int k = (r2 / rstep) % 2 ? top - 1 - i : i;   // back and forth, so that a group across two bands spans few cells
 			for (int r = r2; r < std::min(nrow, r2 + rstep); r++) {
-				const int nj = L.rows[r].nj, nt = shares(r);
+				const int64_t nj = L.rows[r].nj, nt = shares(r);   // (nj * k passes 2^31 on lines of 4e5 cells)
 				if (k < nt)
-					tasks.push_back(T{r, nj * k / nt, nj * (k + 1) / nt - nj * k / nt});
+					tasks.push_back(T{r, (int)(nj * k / nt), (int)(nj * (k + 1) / nt - nj * k / nt)});
 			}
 		}
 	const size_t ngroup = (tasks.size() + most - 1) / most;
