@@ -370,13 +370,14 @@ int batch_build(cc_batch *b, int per_split, int segs_per_split)
 			b->total[mode][ph] = q[ph * (B + 1) + B];
 	}
 	int rc;
-	if ((rc = upload_into(b->d_rho[0], b->rho)) || (rc = upload_into(b->d_red[0], b->red)) ||
-	    (rc = upload_into(b->d_force[0], b->force)) || (rc = upload_into(b->d_pre, pre)) ||
-	    (rc = upload_into(b->d_shape, shape)) || (rc = upload_into(b->d_dim, dim)) ||
-	    (rc = upload_into(b->d_lrho[0], b->lrho)) || (rc = upload_into(b->d_lred[0], b->lred)) ||
-	    (rc = upload_into(b->d_lforce[0], b->lforce)) || (rc = upload_into(b->d_own, own)))
+	cudaStream_t st = b->stream;
+	if ((rc = upload_into(b->d_rho[0], b->rho, st)) || (rc = upload_into(b->d_red[0], b->red, st)) ||
+	    (rc = upload_into(b->d_force[0], b->force, st)) || (rc = upload_into(b->d_pre, pre, st)) ||
+	    (rc = upload_into(b->d_shape, shape, st)) || (rc = upload_into(b->d_dim, dim, st)) ||
+	    (rc = upload_into(b->d_lrho[0], b->lrho, st)) || (rc = upload_into(b->d_lred[0], b->lred, st)) ||
+	    (rc = upload_into(b->d_lforce[0], b->lforce, st)) || (rc = upload_into(b->d_own, own, st)))
 		return rc;
-	CC_CUDA(cudaStreamSynchronize(nullptr));   // (with the arena's zeros) the batch's stream does not wait for the legacy one
+	CC_CUDA(cudaStreamSynchronize(st));   // evaluations may run on a caller's stream
 	b->per_split = per_split;
 	b->segs_per_split = segs_per_split;
 	return CC_OK;
@@ -414,7 +415,9 @@ int batch_eval(cc_batch *b, int set, int precision, cudaStream_t st)
 int batch_check_wait(cc_batch *b, unsigned err)
 {
 	if (err) {
-		CC_CUDA(cudaMemset(b->d_count + 3 * b->order.size(), 0, sizeof(unsigned)));
+		// in place before a launch on any stream: a later clear would erase that launch's error
+		CC_CUDA(cudaMemsetAsync(b->d_count + 3 * b->order.size(), 0, sizeof(unsigned), b->stream));
+		CC_CUDA(cudaStreamSynchronize(b->stream));
 		return fail(CC_ERR_TIMEOUT, "a bounded wait of the fused batch kernel ran out");
 	}
 	return CC_OK;
@@ -568,8 +571,8 @@ int cc_batch_create(int count, cc_handle *const *handles, const int64_t *N, cc_b
 		return rc;
 	}
 	b->arena.cap = b->arena.used;
-	if (cudaMemset(b->arena.base, 0, b->arena.used) != cudaSuccess ||
-	    cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess) {
+	if (cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess ||
+	    cudaMemsetAsync(b->arena.base, 0, b->arena.used, b->stream) != cudaSuccess) {
 		cc_batch_destroy(b);
 		return fail(CC_ERR_CUDA, "batch initialisation failed");
 	}
@@ -608,7 +611,7 @@ int cc_batch_create(int count, cc_handle *const *handles, const int64_t *N, cc_b
 	}
 	for (const auto &p : pieces)
 		*p.first = b->meta + p.second;
-	if (cudaMemset(b->meta, 0, used) != cudaSuccess) {
+	if (cudaMemsetAsync(b->meta, 0, used, b->stream) != cudaSuccess) {
 		cc_batch_destroy(b);
 		return fail(CC_ERR_CUDA, "batch initialisation failed");
 	}
@@ -841,14 +844,13 @@ int cc_batch_minimize(cc_batch *b, double *const *frac, const cc_lbfgs_opts *opt
 		lfa[k].gfrac_out = fa[k].gfrac_out;
 		lfa[k].F_out = nullptr;
 	}
-	if ((rc = upload_into(b->d_lb, lbo)) || (rc = upload_into(b->d_rho[1], ra)) || (rc = upload_into(b->d_red[1], rr)) ||
-	    (rc = upload_into(b->d_force[1], fa)) || (rc = upload_into(b->d_lrho[1], lra)) ||
-	    (rc = upload_into(b->d_lred[1], lrr)) || (rc = upload_into(b->d_lforce[1], lfa)))
-		return rc;
-	if ((rc = upload_into(b->d_start, start)) || (rc = upload_into(b->d_final, final_pos)))
-		return rc;
-	CC_CUDA(cudaStreamSynchronize(nullptr));   // the batch's stream does not wait for the legacy one
 	cudaStream_t st = b->stream;
+	if ((rc = upload_into(b->d_lb, lbo, st)) || (rc = upload_into(b->d_rho[1], ra, st)) ||
+	    (rc = upload_into(b->d_red[1], rr, st)) || (rc = upload_into(b->d_force[1], fa, st)) ||
+	    (rc = upload_into(b->d_lrho[1], lra, st)) || (rc = upload_into(b->d_lred[1], lrr, st)) ||
+	    (rc = upload_into(b->d_lforce[1], lfa, st)) || (rc = upload_into(b->d_start, start, st)) ||
+	    (rc = upload_into(b->d_final, final_pos, st)))
+		return rc;
 	const bool sched = o.precision == CC_PREC_SCHEDULE;
 	CC_CUDA(cudaMemcpyAsync(b->lb_base + ox[0], b->h_pin, b->pos_bytes, cudaMemcpyHostToDevice, st));
 	CC_CUDA(cudaMemsetAsync(b->lb_base + ost[0], 0, st_bytes, st));

@@ -577,6 +577,7 @@ int ensure_particles(cc_handle *h, int64_t N)
 		    (rc = dev_alloc(&h->d_gfrac, need * h->d)) || (rc = dev_alloc(&h->d_fcounters, (need + 31) / 32)))
 			return rc;
 		CC_CUDA(cudaMemset(h->d_fcounters, 0, ((need + 31) / 32) * sizeof(unsigned)));
+		CC_CUDA(cudaStreamSynchronize(nullptr));   // the evaluations' streams do not wait for the legacy one
 		h->ncap = need;
 	}
 	const size_t pin = need * h->d + 2;

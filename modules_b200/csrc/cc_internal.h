@@ -122,19 +122,24 @@ template <class T> int dev_alloc(T **p, size_t n)
 	return CC_OK;
 }
 
+// A new array, in place for every stream when the call returns (a copy from pageable memory may return before it has
+// landed, and the evaluations' streams do not wait for the legacy one).
 template <class T> int upload(T **p, const std::vector<T> &v)
 {
 	if (int rc = dev_alloc(p, v.size()))
 		return rc;
-	if (!v.empty())
-		CC_CUDA(cudaMemcpy(*p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice));
+	if (v.empty())
+		return CC_OK;
+	CC_CUDA(cudaMemcpy(*p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice));
+	CC_CUDA(cudaStreamSynchronize(nullptr));
 	return CC_OK;
 }
 
-template <class T> int upload_into(T *p, const std::vector<T> &v)
+// The same into an array that stream st reads next (or the caller synchronises it).
+template <class T> int upload_into(T *p, const std::vector<T> &v, cudaStream_t st)
 {
 	if (!v.empty())
-		CC_CUDA(cudaMemcpy(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice));
+		CC_CUDA(cudaMemcpyAsync(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, st));
 	return CC_OK;
 }
 

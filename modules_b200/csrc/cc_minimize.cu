@@ -127,10 +127,11 @@ int cc_minimize(cc_handle *h, int64_t N, double *frac, const cc_lbfgs_opts *opts
 		double v = frac[i] - std::floor(frac[i]);
 		x0[i] = v - std::floor(v);
 	}
-	CC_CUDA(cudaMemcpy(b.x, x0.data(), sizeof(double) * n, cudaMemcpyHostToDevice));
-	CC_CUDA(cudaMemcpy(b.xt, x0.data(), sizeof(double) * n, cudaMemcpyHostToDevice));
-	CC_CUDA(cudaMemset(b.g, 0, sizeof(double) * n));
-	CC_CUDA(cudaMemset(b.d, 0, sizeof(double) * n));
+	// the set-up goes through the handle's stream, which reads it
+	CC_CUDA(cudaMemcpyAsync(b.x, x0.data(), sizeof(double) * n, cudaMemcpyHostToDevice, h->stream));
+	CC_CUDA(cudaMemcpyAsync(b.xt, x0.data(), sizeof(double) * n, cudaMemcpyHostToDevice, h->stream));
+	CC_CUDA(cudaMemsetAsync(b.g, 0, sizeof(double) * n, h->stream));
+	CC_CUDA(cudaMemsetAsync(b.d, 0, sizeof(double) * n, h->stream));
 	cc::LbInst inst;
 	inst.n = n;
 	inst.m = m;
@@ -143,7 +144,7 @@ int cc_minimize(cc_handle *h, int64_t N, double *frac, const cc_lbfgs_opts *opts
 	inst.Y = b.Y;
 	inst.part = b.part;
 	inst.st = b.st;
-	CC_CUDA(cudaMemcpy(b.inst, &inst, sizeof(inst), cudaMemcpyHostToDevice));
+	CC_CUDA(cudaMemcpyAsync(b.inst, &inst, sizeof(inst), cudaMemcpyHostToDevice, h->stream));
 	b.host_inst = inst;
 	// warm-up evaluations allocate the evaluation's work buffers before any capture
 	const bool sched = o.precision == CC_PREC_SCHEDULE;
@@ -163,7 +164,7 @@ int cc_minimize(cc_handle *h, int64_t N, double *frac, const cc_lbfgs_opts *opts
 	s0.max_evals = o.max_evals;
 	s0.m = m;
 	s0.newslot = -1;
-	CC_CUDA(cudaMemcpy(b.st, &s0, sizeof(s0), cudaMemcpyHostToDevice));
+	CC_CUDA(cudaMemcpyAsync(b.st, &s0, sizeof(s0), cudaMemcpyHostToDevice, h->stream));
 	h->d_skip = &b.st->status;
 	cudaGraphExec_t gexec[2] = {nullptr, nullptr};
 	auto destroy_graphs = [&]() {

@@ -194,7 +194,7 @@ int fill_slot(const cc_request &r, int idx, int m, const cc::Plan &p, const cc::
 	s0.m = m;
 	s0.newslot = -1;
 	SV_CUDA(cudaMemcpyAsync(b + o_st, &s0, sizeof(s0), cudaMemcpyHostToDevice, st));
-	// host buffers above are pageable: the copies complete before the call returns
+	// s0 and x0 go out of scope: their copies are complete after this
 	SV_CUDA(cudaStreamSynchronize(st));
 	s.req = idx;
 	s.d = d;
@@ -362,10 +362,10 @@ extern "C" int cc_serve(const cc_request *reqs, int count, const cc_serve_opts *
 	SV_CUDA(cudaMalloc(&d_queue, sizeof(unsigned) * 2));
 	SV_CUDA(cudaMalloc(&d_count, sizeof(unsigned) * (3 * o.max_slots + 1)));
 	SV_CUDA(cudaMalloc(&d_brief, sizeof(cc::LbBrief) * o.max_slots));
-	SV_CUDA(cudaMemset(d_queue, 0, sizeof(unsigned) * 2));
+	SV_CUDA(cudaMemsetAsync(d_queue, 0, sizeof(unsigned) * 2, st));
 	// the fused launch's completion counts are zero between launches (its items reset them); the error word after
 	// the counts of the current round's requests must start at zero too
-	SV_CUDA(cudaMemset(d_count, 0, sizeof(unsigned) * (3 * o.max_slots + 1)));
+	SV_CUDA(cudaMemsetAsync(d_count, 0, sizeof(unsigned) * (3 * o.max_slots + 1), st));
 	const auto t0 = std::chrono::steady_clock::now();
 	auto now = [&]() { return std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count(); };
 	int done = 0;
@@ -484,7 +484,7 @@ extern "C" int cc_serve(const cc_request *reqs, int count, const cc_serve_opts *
 		SV_CUDA(cudaMemcpyAsync(d_pre, pre.data(), sizeof(int) * pre.size(), cudaMemcpyHostToDevice, st));
 		SV_CUDA(cudaMemcpyAsync(d_shape, shape.data(), sizeof(int) * shape.size(), cudaMemcpyHostToDevice, st));
 		SV_CUDA(cudaMemcpyAsync(d_dim, dim.data(), sizeof(int) * A, cudaMemcpyHostToDevice, st));
-		// the descriptor vectors are pageable: the copies complete before the iterations read them
+		// the iterations follow the copies on the stream; the pageable vectors are staged when each call returns
 		cc::MBatchArgs ma;
 		ma.rho = d_ra;
 		ma.red = d_rr;
