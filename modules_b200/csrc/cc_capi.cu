@@ -1126,6 +1126,11 @@ int run_nufft_t(cc_handle *h, int64_t N, const double *d_frac, double *d_E, doub
 	cc::NufftDev a = h->nu;
 	a.skip = h->d_skip;
 	const int64_t ngrid = h->nu_ngrid;
+	// An evaluation finds the fixed-point grid zero and its second kernel leaves it so; one that ended between the two left
+	// its particles there.
+	if (h->nu_dirty)
+		CC_CUDA(cudaMemsetAsync(a.gi, 0, sizeof(unsigned long long) * (size_t)ngrid, st));
+	h->nu_dirty = true;
 	if (N > 0) {
 		cc::nufft_spread_kernel<D><<<(unsigned)((N + cc::kNufftPerBlock - 1) / cc::kNufftPerBlock), cc::kNufftThreads,
 		                             0, st>>>(a, d_frac, (int)N);
@@ -1133,6 +1138,7 @@ int run_nufft_t(cc_handle *h, int64_t N, const double *d_frac, double *d_E, doub
 	}
 	cc::nufft_fix_to_double_kernel<<<(unsigned)((ngrid + 255) / 256), 256, 0, st>>>(a, ngrid);
 	CC_CUDA(cudaGetLastError());
+	h->nu_dirty = false;
 	if (cufftSetStream(h->nu_p1, st) != CUFFT_SUCCESS ||
 	    cufftExecD2Z(h->nu_p1, a.gr, reinterpret_cast<cufftDoubleComplex *>(const_cast<double2 *>(a.spec))) !=
 	        CUFFT_SUCCESS)

@@ -298,6 +298,7 @@ struct cc_handle {
 	std::vector<void *> nu_bufs;    // device buffers owned by the NUFFT set-up
 	cufftHandle nu_p1 = 0, nu_p2 = 0;
 	bool nu_p1_ok = false, nu_p2_ok = false;
+	bool nu_dirty = false;          // nu.gi may hold the particles of an evaluation that ended with an error
 	// Monte Carlo: rho in mode order of the bound positions, the trial rho and the device modes
 	int32_t *d_modes = nullptr;
 	double *d_modeV = nullptr;
