@@ -16,7 +16,9 @@
 #include "cc_nufft.cuh"
 #include "cc_plan.h"
 
+#if defined(__x86_64__)
 #include <immintrin.h>
+#endif
 
 #include <algorithm>
 #include <cmath>
@@ -1484,6 +1486,16 @@ int launch_eval_graph(cc_handle *h, int64_t N, int precision, int forces, bool *
 	return CC_OK;
 }
 
+// A pause of a spinning host thread (some 40 ns on x86).
+inline void spin_pause()
+{
+#if defined(__x86_64__)
+	_mm_pause();
+#elif defined(__aarch64__)
+	asm volatile("isb" ::: "memory");
+#endif
+}
+
 // Wait until a kernel has written `number` to mapped host memory: a short look at the word, which the host sees about 4 us
 // before a stream synchronisation returns. False when it does not come soon (a busy GPU, an error): synchronise then.
 bool wait_number(const volatile unsigned long long *word, unsigned long long number)
@@ -1493,7 +1505,7 @@ bool wait_number(const volatile unsigned long long *word, unsigned long long num
 			std::atomic_thread_fence(std::memory_order_acquire);
 			return true;
 		}
-		_mm_pause();
+		spin_pause();
 	}
 	return false;
 }
