@@ -11,7 +11,6 @@ Nothing on the product path imports this package.
 import ctypes
 import os
 import subprocess
-import sys
 
 import numpy as np
 
@@ -27,12 +26,27 @@ _l = ctypes.c_long
 _d = ctypes.c_double
 
 
+# Written by build(): "present" or "absent", whether the reference's sources were there. It travels with the built tree, so
+# that a machine without the sources can tell "not to be had here" from "not built although it should be".
+RECORD = os.path.join(HERE, "_build", "reference_sources")
+
+
+class ReferenceAbsent(RuntimeError):
+    """The reference oracle was asked for where its sources were absent at the build."""
+
+
 def build(ref=True, ref_tree=None):
     """Build the port (always) and the reference oracle (when a reference tree is given, by ref_tree or
     CC_REFERENCE_TREE, and present)."""
     subprocess.run(["make", "-s", "-C", HERE, "port"], check=True)
+    if not ref:
+        return
     tree = ref_tree or REFERENCE_TREE
-    if ref and tree and os.path.isdir(tree):
+    there = bool(tree) and os.path.isdir(os.path.join(tree, "potential"))
+    os.makedirs(os.path.dirname(RECORD), exist_ok=True)
+    with open(RECORD, "w") as f:
+        f.write("present\n" if there else "absent\n")
+    if there:
         subprocess.run(["make", "-s", "-C", HERE, "ref", f"REF={tree}"], check=True)
 
 
@@ -48,11 +62,20 @@ def ref_available():
     return os.path.exists(REF_LIB)
 
 
+def ref_expected():
+    """Whether the reference oracle should be built here: its sources were there at the build (or, before any build, are
+    named by CC_REFERENCE_TREE)."""
+    if os.path.exists(RECORD):
+        with open(RECORD) as f:
+            return f.read().strip() == "present"
+    return bool(REFERENCE_TREE)
+
+
 def ref_lib():
     global _REF
     if _REF is None:
-        if not ref_available() and "pytest" in sys.modules:   # built without the reference's sources
-            sys.modules["pytest"].skip("the reference oracle (oracle/_ref) is not built here")
+        if not ref_available() and not ref_expected():
+            raise ReferenceAbsent("the reference oracle (oracle/_ref) is not built: its sources were absent")
         lib = ctypes.CDLL(REF_LIB)
         lib.ccref_create.restype = _vp
         lib.ccref_create.argtypes = [ctypes.c_int, _vp, _l, _vp, _vp, _vp, _d, ctypes.c_int]
