@@ -330,8 +330,8 @@ Launch find_launch(const DevKSet &k, int64_t N, bool mixed)
 }
 
 // A k-set keeps its last few choices: a program evaluates few particle counts with one handle, and searching the grids
-// takes longer on the host than launching them.
-Launch choose_launch(const DevKSet &k, int64_t N, bool mixed)
+// takes longer on the host than launching them. (A query of a handle that it must not change searches: find_launch.)
+Launch choose_launch(DevKSet &k, int64_t N, bool mixed)
 {
 	for (const DevKSet::Chosen &c : k.chosen)
 		if (c.N == N && c.mixed == mixed)
@@ -2361,7 +2361,7 @@ int cc_plan_info(const cc_handle *h, int64_t N, int *L, int64_t *nseg, int *nspl
 {
 	if (int rc = check_handle(h))
 		return rc;
-	const Launch l = choose_launch(h->main, N, false);
+	const Launch l = find_launch(h->main, N, false);
 	if (L)
 		*L = h->main.plan.L;
 	if (nseg)

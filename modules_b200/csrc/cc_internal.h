@@ -88,7 +88,7 @@ struct DevKSet {
 		bool mixed;
 		Launch l;
 	};
-	mutable std::vector<Chosen> chosen;   // launch configurations of the last few particle counts
+	std::vector<Chosen> chosen;   // launch configurations of the last few particle counts
 
 	void release()
 	{
