@@ -668,17 +668,17 @@ inline bool wrap_unit(double x, double *out)
 	return true;
 }
 
-int ensure_partial(DevKSet &k, size_t elems)
+int ensure_partial(double2 **partial, size_t &cap, size_t elems)
 {
-	if (elems <= k.partial_cap)
+	if (elems <= cap)
 		return CC_OK;
-	cudaFree(k.partial);
-	k.partial = nullptr;
-	k.partial_cap = 0;
-	int rc = dev_alloc(&k.partial, elems);
+	cudaFree(*partial);
+	*partial = nullptr;
+	cap = 0;
+	int rc = dev_alloc(partial, elems);
 	if (rc)
 		return rc;
-	k.partial_cap = elems;
+	cap = elems;
 	return CC_OK;
 }
 
@@ -715,7 +715,7 @@ int run_rho(cc_handle *h, DevKSet &k, int64_t N, const double *d_frac, double *d
 		const cc::LinePlan &L = k.lplan;
 		const LineLane *lane = &k == &h->main ? h->lane : nullptr;
 		if (!lane) {
-			if (int rc = ensure_partial(k, (size_t)nsplit * L.nunit * 128))
+			if (int rc = ensure_partial(&k.line.partial, k.line.partial_cap, (size_t)nsplit * L.nunit * 128))
 				return rc;
 			if (!k.line.weights)
 				if (int rc = dev_alloc(&k.line.weights, (size_t)L.nunit * 256))
@@ -735,7 +735,7 @@ int run_rho(cc_handle *h, DevKSet &k, int64_t N, const double *d_frac, double *d
 		a.groups = dg.groups;
 		a.tasks = dg.tasks;
 		a.tlines = dg.tlines;
-		a.partial = lane ? lane->partial : k.partial;
+		a.partial = lane ? lane->partial : k.line.partial;
 		a.skip = h->d_skip;
 		a.frac_copy = (&k == &h->main) ? h->rho_copy : nullptr;
 		a.early = (h->early_call && &k == &h->main && !a.skip && !a.frac_copy) ? 1 : 0;
@@ -777,7 +777,7 @@ int run_rho(cc_handle *h, DevKSet &k, int64_t N, const double *d_frac, double *d
 	const int nsplit = N > 0 ? l.nsplit : 1;
 	const int csize = N > 0 ? l.csize : 1;
 	const int rows = nsplit / csize;
-	if (int rc = ensure_partial(k, (size_t)rows * p.nslot))
+	if (int rc = ensure_partial(&k.partial, k.partial_cap, (size_t)rows * p.nslot))
 		return rc;
 	cc::RhoArgs a = {};
 	a.frac = d_frac;

@@ -63,6 +63,10 @@ struct DevLines {
 	std::vector<Groups> groups;     // per grouping of the plan
 	double2 *weights = nullptr;     // nunit * 256
 	double *eblock = nullptr;       // one per reduce block
+	// partial rows * nunit * 128, apart from the segment kernels': an evaluation in one precision never moves what a graph
+	// that a program captured in the other one reads
+	double2 *partial = nullptr;
+	size_t partial_cap = 0;         // in double2 elements
 };
 
 struct DevKSet {
@@ -96,6 +100,7 @@ struct DevKSet {
 		cudaFree(rho_slot);   // (and u_slot)
 		cudaFree(rho_mode);
 		cudaFree(line.weights);
+		cudaFree(line.partial);
 		cudaFree(partial);
 		for (DevSplits &f : splits) {
 			cudaFree(f.kstart);
