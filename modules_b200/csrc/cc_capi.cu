@@ -1963,19 +1963,23 @@ static int many_lanes(cc_handle *h, int64_t N, int precision, int *count)
 	             o_t = o_e + room((size_t)L.nunit * (64 / cc::kLineRedCells) * sizeof(double)), bytes = o_t + 256;
 	if (bytes > kManyLaneBytes)
 		return CC_OK;
-	while (h->lanes.size() < kManyLanes - 1) {
-		h->lanes.emplace_back();
-		LineLane &n = h->lanes.back();
-		CC_CUDA(cudaStreamCreateWithFlags(&n.stream, cudaStreamNonBlocking));
-		CC_CUDA(cudaEventCreateWithFlags(&n.ev, cudaEventDisableTiming));
-	}
+	// lanes only make the call faster: where their streams or buffers cannot be had, one lane does the work
+	auto none = [] {
+		cudaGetLastError();
+		return CC_OK;
+	};
+	if (h->lanes.empty())
+		h->lanes.resize(kManyLanes - 1);
 	for (LineLane &n : h->lanes) {
+		if ((!n.stream && cudaStreamCreateWithFlags(&n.stream, cudaStreamNonBlocking) != cudaSuccess) ||
+		    (!n.ev && cudaEventCreateWithFlags(&n.ev, cudaEventDisableTiming) != cudaSuccess))
+			return none();
 		if (bytes > n.cap) {
 			cudaFree(n.blob);
 			n.blob = nullptr;
 			n.cap = 0;
-			if (int rc = dev_alloc(&n.blob, bytes))
-				return rc;
+			if (dev_alloc(&n.blob, bytes))
+				return none();
 			n.cap = bytes;
 		}
 		n.partial = reinterpret_cast<double2 *>(n.blob);
