@@ -223,7 +223,7 @@ Launch choose_line_launch(const cc::LinePlan &p, int d, int64_t N)
 		const cc::LineGroups &g = p.groupings[gi];
 		const int64_t G = std::max<int64_t>(1, (int64_t)g.count());
 		const bool two = g.ntask <= cc::kLineTasks;
-		const int64_t wave = (two ? 2 : 1) * (int64_t)sms, maxns = std::max<int64_t>(1, std::min<int64_t>((N + 7) / 8, 4096));
+		const int64_t wave = (two ? 2 : 1) * (int64_t)sms, maxns = std::max<int64_t>(1, std::min<int64_t>((N + 7) / 8, cc::kLineMaxSplits));
 		for (int64_t ns = 1; ns <= maxns; ns++) {
 			const int64_t per = std::max<int64_t>(8, ((N + ns - 1) / ns + 7) / 8 * 8),
 			              real = std::max<int64_t>(1, (N + per - 1) / per);
@@ -276,7 +276,7 @@ Launch choose_line_launch(const cc::LinePlan &p, int d, int64_t N)
 Launch find_launch(const DevKSet &k, int64_t N, bool mixed)
 {
 	const cc::Plan &p = k.plan;
-	if (!mixed && k.lplan.ok)
+	if (!mixed && k.lplan.ok && N <= cc::kLineMaxParticles)
 		return choose_line_launch(k.lplan, p.d, N);
 	Launch l = {};
 	const size_t esz = mixed ? sizeof(float2) : sizeof(double2);

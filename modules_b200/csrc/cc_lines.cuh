@@ -162,7 +162,6 @@ struct LineRhoArgs {
 	int early;                // as RhoArgs
 };
 
-constexpr int kLineMaxChunk = 128;  // particles per chunk of rho tables (x D at most one coordinate per thread)
 // staged coordinates in front of the tables
 __host__ __device__ constexpr size_t line_pos_bytes(int particles, int d)
 {

@@ -110,6 +110,12 @@ constexpr int kLineTiles = 4;       // column tiles per rho task
 constexpr int kLineTasks = 8;       // warps per rho block, two blocks to an SM
 constexpr int kLineMaxTasks = 16;   // or up to 16, one block to an SM
 constexpr int kLineMaxRow = 160;    // table entries per particle
+constexpr int kLineMaxChunk = 128;  // particles per chunk of rho tables (x d at most one coordinate per thread)
+constexpr int kLineMaxSplits = 4096;   // particle splits of the rho pass, each of a multiple of 8 particles
+// The kernels count particles in 32 bits and look one chunk past the end of a split, which lies at most 8 particles per split
+// behind the last one: more particles than this stay on the segment kernels.
+constexpr int64_t kLineMaxParticles = ((int64_t)1 << 31) - ((int64_t)1 << 16);
+static_assert(kLineMaxParticles + 8 * (int64_t)kLineMaxSplits + kLineMaxChunk < ((int64_t)1 << 31), "32-bit particle indices");
 
 // The rho pass's block groups: blocks of `ntask` warps, each with a task or none.
 struct LineGroups {
