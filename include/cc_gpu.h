@@ -182,8 +182,9 @@ int cc_batch_minimize(cc_batch *b, double *const *frac, const cc_lbfgs_opts *opt
 /* Autotuner of the batch's tile shapes: times `reps` FP64 evaluations of the bound positions for every candidate
  * (particles per rho block 32 / 64 / 128 / 256 / 512 / 1024 x segments per force block 32 / 64 / 128 / 256 / 512 /
  * 1024) with CUDA events and keeps the fastest for the batch's later evaluations and minimisations (default before
- * tuning: 64 x 64). The chosen shape
- * is returned in *per_split and *segs_per_split (either may be NULL). Results of different shapes agree to rounding;
+ * tuning: 64 x 64). Where instances evaluate FP64 on the matrix unit, which has no segments per force block, the particles
+ * are chosen by FP64 evaluations and the segments by mixed ones (and FP64 ones of the other instances). The chosen shape is
+ * returned in *per_split and *segs_per_split (either may be NULL). Results of different shapes agree to rounding;
  * with one shape every instance's result is independent of the rest of the batch. */
 int cc_batch_autotune(cc_batch *b, int reps, int *per_split, int *segs_per_split);
 /* Test hook of the fused batch kernel's bounded waits: every wait gives up after `polls` polls (0: the default, about

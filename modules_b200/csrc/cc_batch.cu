@@ -632,30 +632,55 @@ int cc_batch_autotune(cc_batch *b, int reps, int *per_split, int *segs_per_split
 	CC_CUDA(cudaEventCreate(&e1));
 	float best = 1e30f;
 	int bp = b->per_split, bs = b->segs_per_split, rc = CC_OK;
-	for (int ps : kTuneSplits)
-		for (int sg : kTuneSegs) {
-			if ((rc = batch_build(b, ps, sg)) || (rc = batch_eval(b, 0, CC_PREC_FP64, b->stream)))
-				break;
-			if (cudaEventRecord(e0, b->stream) != cudaSuccess) {
-				rc = fail(CC_ERR_CUDA, "cudaEventRecord failed");
-				break;
+	// `reps` evaluations at a precision, after one that is not timed
+	auto timed = [&](int precision, float *ms) -> int {
+		if (int r2 = batch_eval(b, 0, precision, b->stream))
+			return r2;
+		if (cudaEventRecord(e0, b->stream) != cudaSuccess)
+			return fail(CC_ERR_CUDA, "cudaEventRecord failed");
+		for (int r = 0; r < reps; r++)
+			if (int r2 = batch_eval(b, 0, precision, b->stream))
+				return r2;
+		if (cudaEventRecord(e1, b->stream) != cudaSuccess || cudaEventSynchronize(e1) != cudaSuccess ||
+		    cudaEventElapsedTime(ms, e0, e1) != cudaSuccess)
+			return fail(CC_ERR_CUDA, "autotune timing failed");
+		return CC_OK;
+	};
+	float ms = 0.0f, mixed_ms = 0.0f;
+	if (!b->any_line) {
+		for (int ps : kTuneSplits)
+			for (int sg : kTuneSegs) {
+				if (rc || (rc = batch_build(b, ps, sg)) || (rc = timed(CC_PREC_FP64, &ms)))
+					continue;
+				if (ms < best) {
+					best = ms;
+					bp = ps;
+					bs = sg;
+				}
 			}
-			for (int r = 0; r < reps && rc == CC_OK; r++)
-				rc = batch_eval(b, 0, CC_PREC_FP64, b->stream);
-			if (rc)
-				break;
-			float ms = 0.0f;
-			if (cudaEventRecord(e1, b->stream) != cudaSuccess || cudaEventSynchronize(e1) != cudaSuccess ||
-			    cudaEventElapsedTime(&ms, e0, e1) != cudaSuccess) {
-				rc = fail(CC_ERR_CUDA, "autotune timing failed");
-				break;
-			}
+	} else {
+		// FP64 evaluations of instances with a line plan do not read the segment tile: the particles per rho block are chosen
+		// by FP64, the segments then by FP64 (the other instances) and mixed evaluations (every instance) together
+		for (int ps : kTuneSplits) {
+			if (rc || (rc = batch_build(b, ps, bs)) || (rc = timed(CC_PREC_FP64, &ms)))
+				continue;
 			if (ms < best) {
 				best = ms;
 				bp = ps;
+			}
+		}
+		best = 1e30f;
+		for (int sg : kTuneSegs) {
+			if (rc || (rc = batch_build(b, bp, sg)) || (!b->all_line && (rc = timed(CC_PREC_FP64, &ms))) ||
+			    (rc = timed(CC_PREC_MIXED, &mixed_ms)))
+				continue;
+			const float both = mixed_ms + (b->all_line ? 0.0f : ms);
+			if (both < best) {
+				best = both;
 				bs = sg;
 			}
 		}
+	}
 	cudaEventDestroy(e0);
 	cudaEventDestroy(e1);
 	if (rc)
