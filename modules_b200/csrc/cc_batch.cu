@@ -551,6 +551,11 @@ int cc_batch_create(int count, cc_handle *const *handles, const int64_t *N, cc_b
 		const int max_nsplit = (int)((n + kTuneSplits[0] - 1) / kTuneSplits[0]);
 		const int nchunks = (p.nslot + 31) / 32, pgroups = (int)((n + 31) / 32);
 		const cc::LinePlan &L = h->main.lplan;
+		if (L.ok)
+			if (int rc = ensure_lines(h->main)) {
+				delete b;
+				return rc;
+			}
 		const size_t row = std::max((size_t)p.nslot, L.ok ? (size_t)L.nunit * 128 : 0);   // entries of a partial row
 		b->any_line |= L.ok;
 		q.o_part = b->arena.take(sizeof(double2) * (size_t)max_nsplit * row);

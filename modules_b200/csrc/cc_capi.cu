@@ -27,6 +27,7 @@
 #include <array>
 #include <atomic>
 #include <cstring>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -95,47 +96,55 @@ int cci::get_splits(DevKSet &k, int want, const DevSplits **out)
 	return CC_OK;
 }
 
-// The plan's arrays (and the line plan's) go up in one copy into one allocation; what the kernels write starts at zero:
-// slots without a mode are read (with weight 0) but never written on the line path, and the ticket starts at 0.
+namespace {
+
+// Arrays that go up in one copy to the start of one allocation, each at a multiple of 256 bytes.
+struct Pack {
+	struct Piece {
+		const void *from;
+		size_t at, bytes;
+	};
+	std::vector<Piece> pieces;
+	size_t used = 0;
+
+	template <class T> size_t put(const std::vector<T> &v)
+	{
+		const size_t at = used;
+		pieces.push_back({v.data(), at, v.size() * sizeof(T)});
+		used = (used + v.size() * sizeof(T) + 255) / 256 * 256;
+		return at;
+	}
+	// In place for every stream when the call returns.
+	int upload(unsigned char *to) const
+	{
+		if (used == 0)
+			return CC_OK;
+		std::unique_ptr<unsigned char[]> h(new unsigned char[used]);   // (the gaps are never read)
+		for (const Piece &p : pieces)
+			if (p.bytes)
+				std::memcpy(h.get() + p.at, p.from, p.bytes);
+		CC_CUDA(cudaMemcpy(to, h.get(), used, cudaMemcpyHostToDevice));
+		CC_CUDA(cudaStreamSynchronize(nullptr));
+		return CC_OK;
+	}
+};
+
+}  // namespace
+
+// What the kernels write starts at zero: slots without a mode are read (with weight 0) but never written on the line path,
+// and the ticket starts at 0.
 int cci::upload_kset(DevKSet &k, const cc::Plan &plan)
 {
 	k.release();
 	k.plan = plan;
 	k.lplan = cc::build_line_plan(plan);
-	const cc::LinePlan &L = k.lplan;
-	std::vector<unsigned char> up;
-	auto room = [](size_t bytes) { return (bytes + 255) / 256 * 256; };
-	auto put = [&](const void *p, size_t bytes) {
-		const size_t at = up.size();
-		const unsigned char *s = static_cast<const unsigned char *>(p);
-		up.insert(up.end(), s, s + bytes);
-		up.resize(room(up.size()));
-		return at;
-	};
-#define CC_PUT(v) put((v).data(), (v).size() * sizeof((v)[0]))
-	const size_t o_segs = CC_PUT(plan.segs), o_bstart = CC_PUT(plan.bstart), o_bspec = CC_PUT(plan.bspec),
-	             o_slotV = CC_PUT(plan.slotV), o_mode = CC_PUT(plan.mode_slot);
-	const size_t o_rows = CC_PUT(L.rows), o_lines = CC_PUT(L.lines), o_cells = CC_PUT(L.cells), o_cellV = CC_PUT(L.cellV),
-	             o_phases = CC_PUT(L.phases);
-	struct Offsets {
-		size_t groups, tasks, tlines;
-	};
-	std::vector<Offsets> og;
-	for (const cc::LineGroups &g : L.groupings) {
-		const size_t a = CC_PUT(g.groups), b = CC_PUT(g.tasks), c = CC_PUT(g.tlines);
-		og.push_back({a, b, c});
-	}
-#undef CC_PUT
+	Pack up;
+	const size_t o_segs = up.put(plan.segs), o_bstart = up.put(plan.bstart), o_bspec = up.put(plan.bspec),
+	             o_slotV = up.put(plan.slotV), o_mode = up.put(plan.mode_slot);
 	const size_t nslot = plan.slotV.size(), M = plan.mode_slot.size();
-	const size_t nred = (nslot + 31) / 32, nlred = (size_t)L.nunit * (64 / cc::kLineRedCells);
-	size_t end = up.size();
-	auto take = [&](size_t bytes) {
-		const size_t at = end;
-		end += room(std::max<size_t>(bytes, 1));
-		return at;
-	};
-	const size_t o_ticket = take(sizeof(unsigned)), o_eb = take(nred * sizeof(double)), o_leb = take(nlred * sizeof(double));
-	// (the larger arrays apart: allocations below 2 MB come out of the driver's blocks, larger ones take a millisecond)
+	const size_t o_ticket = up.used, o_eb = o_ticket + 256, end = o_eb + std::max<size_t>(1, (nslot + 31) / 32) * sizeof(double);
+	// (the larger arrays apart: allocations below 1 MB come out of the driver's 2 MB blocks, others are mapped by themselves,
+	// which takes 0.3 ms)
 	if (int rc = dev_alloc(&k.blob, end))
 		return rc;
 	if (int rc = dev_alloc(&k.rho_slot, 2 * nslot))
@@ -143,11 +152,11 @@ int cci::upload_kset(DevKSet &k, const cc::Plan &plan)
 	if (int rc = dev_alloc(&k.rho_mode, M))
 		return rc;
 	k.u_slot = k.rho_slot + nslot;
-	if (!up.empty())
-		CC_CUDA(cudaMemcpy(k.blob, up.data(), up.size(), cudaMemcpyHostToDevice));
-	CC_CUDA(cudaMemset(k.blob + up.size(), 0, end - up.size()));
+	CC_CUDA(cudaMemset(k.blob + o_ticket, 0, end - o_ticket));
 	CC_CUDA(cudaMemset(k.rho_slot, 0, 2 * nslot * sizeof(double2)));
 	CC_CUDA(cudaStreamSynchronize(nullptr));   // the evaluations' streams do not wait for the legacy one
+	if (int rc = up.upload(k.blob))
+		return rc;
 	unsigned char *b = k.blob;
 	k.segs = reinterpret_cast<cc::Seg *>(b + o_segs);
 	k.bstart = reinterpret_cast<int *>(b + o_bstart);
@@ -156,6 +165,36 @@ int cci::upload_kset(DevKSet &k, const cc::Plan &plan)
 	k.mode_slot = reinterpret_cast<int *>(b + o_mode);
 	k.ticket = reinterpret_cast<unsigned *>(b + o_ticket);
 	k.eblock = reinterpret_cast<double *>(b + o_eb);
+	return CC_OK;
+}
+
+// Not with the set: a set that is evaluated in mixed precision alone never needs the line plan's arrays, and with them its
+// first evaluation's buffers no longer found room in the driver's blocks (3D N=3001: 0.57 ms instead of 0.10).
+int cci::ensure_lines(DevKSet &k)
+{
+	if (k.line.blob)
+		return CC_OK;
+	const cc::LinePlan &L = k.lplan;
+	Pack up;
+	const size_t o_rows = up.put(L.rows), o_lines = up.put(L.lines), o_cells = up.put(L.cells), o_cellV = up.put(L.cellV),
+	             o_phases = up.put(L.phases);
+	struct Offsets {
+		size_t groups, tasks, tlines;
+	};
+	std::vector<Offsets> og;
+	for (const cc::LineGroups &g : L.groupings) {
+		const size_t a = up.put(g.groups), b = up.put(g.tasks), c = up.put(g.tlines);
+		og.push_back({a, b, c});
+	}
+	const size_t o_eb = up.used;   // (every energy term is written before it is read)
+	unsigned char *b = nullptr;
+	if (int rc = dev_alloc(&b, o_eb + (size_t)L.nunit * (64 / cc::kLineRedCells) * sizeof(double)))
+		return rc;
+	if (int rc = up.upload(b)) {
+		cudaFree(b);
+		return rc;
+	}
+	k.line.blob = b;
 	k.line.rows = reinterpret_cast<cc::LineRow *>(b + o_rows);
 	k.line.lines = reinterpret_cast<cc::LineIdx *>(b + o_lines);
 	k.line.cells = reinterpret_cast<cc::LineCell *>(b + o_cells);
@@ -164,7 +203,7 @@ int cci::upload_kset(DevKSet &k, const cc::Plan &plan)
 	for (const Offsets &o : og)
 		k.line.groups.push_back({reinterpret_cast<cc::LineTabs *>(b + o.groups), reinterpret_cast<cc::LineTask *>(b + o.tasks),
 		                         reinterpret_cast<cc::LineIdx *>(b + o.tlines)});
-	k.line.eblock = reinterpret_cast<double *>(b + o_leb);
+	k.line.eblock = reinterpret_cast<double *>(b + o_eb);
 	return CC_OK;
 }
 
@@ -714,6 +753,8 @@ int run_rho(cc_handle *h, DevKSet &k, int64_t N, const double *d_frac, double *d
 		const int nsplit = N > 0 ? l.nsplit : 1;
 		const cc::LinePlan &L = k.lplan;
 		const LineLane *lane = &k == &h->main ? h->lane : nullptr;
+		if (int rc = ensure_lines(k))
+			return rc;
 		if (!lane) {
 			if (int rc = ensure_partial(&k.line.partial, k.line.partial_cap, (size_t)nsplit * L.nunit * 128))
 				return rc;

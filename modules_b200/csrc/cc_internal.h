@@ -48,8 +48,9 @@ struct Launch {
 	int mt, fwarps;                       // line force: tiles of 8 particles per block, warps per block
 };
 
-// A line plan (cc_plan.h) on the device.
+// A line plan (cc_plan.h) on the device, from the set's first use on the line kernels on (ensure_lines).
 struct DevLines {
+	unsigned char *blob = nullptr;  // one allocation for the arrays below down to eblock, but for the weights
 	const cc::LineRow *rows = nullptr;
 	const cc::LineIdx *lines = nullptr;
 	const cc::LineCell *cells = nullptr;
@@ -73,7 +74,7 @@ struct DevKSet {
 	cc::Plan plan;
 	cc::LinePlan lplan;
 	DevLines line;
-	unsigned char *blob = nullptr;  // one allocation for the plan's arrays and the line plan's
+	unsigned char *blob = nullptr;  // one allocation for the plan's arrays, ticket and eblock
 	cc::Seg *segs = nullptr;
 	int *bstart = nullptr;
 	cc::TabSpec *bspec = nullptr;
@@ -99,6 +100,7 @@ struct DevKSet {
 		cudaFree(blob);
 		cudaFree(rho_slot);   // (and u_slot)
 		cudaFree(rho_mode);
+		cudaFree(line.blob);
 		cudaFree(line.weights);
 		cudaFree(line.partial);
 		cudaFree(partial);
@@ -151,6 +153,9 @@ template <class T> int upload_into(T *p, const std::vector<T> &v, cudaStream_t s
 
 // Upload a plan into a device k-set (releases what it held).
 int upload_kset(DevKSet &k, const cc::Plan &plan);
+
+// The arrays of the set's line plan (lplan.ok) on the device.
+int ensure_lines(DevKSet &k);
 
 // The device splits of the force pass into about `want` segment ranges (uploaded on first use, kept by the k-set).
 int get_splits(DevKSet &k, int want, const DevSplits **out);
