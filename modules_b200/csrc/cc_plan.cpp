@@ -50,7 +50,8 @@ TabSpec make_spec(int d, const Ranges &r)
 	TabSpec t = {};
 	int off = 0;
 	for (int e = 0; e < d; e++) {
-		const int range = r.hi[e] - r.lo[e] + 1;
+		// (indices of either sign span up to 2^32; what does not fit a table is cut off by the caller, by its row)
+		const int range = (int)std::min<int64_t>((int64_t)r.hi[e] - r.lo[e] + 1, 1 << 28);
 		t.lo[e] = r.lo[e];
 		if (e < d - 1 && range <= kFullMax) {
 			t.full[e] = 1;
