@@ -98,6 +98,21 @@ int cci::get_splits(DevKSet &k, int want, const DevSplits **out)
 
 namespace {
 
+// Grow a device buffer to n elements (contents not kept).
+template <class T> int grow(T **p, size_t &cap, size_t n)
+{
+	n = std::max<size_t>(n, 1);
+	if (n <= cap)
+		return CC_OK;
+	cudaFree(*p);
+	*p = nullptr;
+	cap = 0;
+	if (int rc = dev_alloc(p, n))
+		return rc;
+	cap = n;
+	return CC_OK;
+}
+
 // Arrays that go up in one copy to the start of one allocation, each at a multiple of 256 bytes.
 struct Pack {
 	struct Piece {
@@ -133,10 +148,14 @@ struct Pack {
 
 // What the kernels write starts at zero: slots without a mode are read (with weight 0) but never written on the line path,
 // and the ticket starts at 0.
-int cci::upload_kset(DevKSet &k, const cc::Plan &plan)
+int cci::upload_kset(DevKSet &k, cc::Plan &&plan_in)
 {
-	k.release();
-	k.plan = plan;
+	k.segs = nullptr;   // (until the new plan is in place)
+	k.line.ready = false;
+	k.chosen.clear();
+	k.drop_splits();
+	k.plan = std::move(plan_in);
+	const cc::Plan &plan = k.plan;
 	k.lplan = cc::build_line_plan(plan);
 	Pack up;
 	const size_t o_segs = up.put(plan.segs), o_bstart = up.put(plan.bstart), o_bspec = up.put(plan.bspec),
@@ -145,11 +164,11 @@ int cci::upload_kset(DevKSet &k, const cc::Plan &plan)
 	const size_t o_ticket = up.used, o_eb = o_ticket + 256, end = o_eb + std::max<size_t>(1, (nslot + 31) / 32) * sizeof(double);
 	// (the larger arrays apart: allocations below 1 MB come out of the driver's 2 MB blocks, others are mapped by themselves,
 	// which takes 0.3 ms)
-	if (int rc = dev_alloc(&k.blob, end))
+	if (int rc = grow(&k.blob, k.blob_cap, end))
 		return rc;
-	if (int rc = dev_alloc(&k.rho_slot, 2 * nslot))
+	if (int rc = grow(&k.rho_slot, k.rho_cap, 2 * nslot))
 		return rc;
-	if (int rc = dev_alloc(&k.rho_mode, M))
+	if (int rc = grow(&k.rho_mode, k.mode_cap, M))
 		return rc;
 	k.u_slot = k.rho_slot + nslot;
 	CC_CUDA(cudaMemset(k.blob + o_ticket, 0, end - o_ticket));
@@ -172,7 +191,7 @@ int cci::upload_kset(DevKSet &k, const cc::Plan &plan)
 // first evaluation's buffers no longer found room in the driver's blocks (3D N=3001: 0.57 ms instead of 0.10).
 int cci::ensure_lines(DevKSet &k)
 {
-	if (k.line.blob)
+	if (k.line.ready)
 		return CC_OK;
 	const cc::LinePlan &L = k.lplan;
 	Pack up;
@@ -187,23 +206,22 @@ int cci::ensure_lines(DevKSet &k)
 		og.push_back({a, b, c});
 	}
 	const size_t o_eb = up.used;   // (every energy term is written before it is read)
-	unsigned char *b = nullptr;
-	if (int rc = dev_alloc(&b, o_eb + (size_t)L.nunit * (64 / cc::kLineRedCells) * sizeof(double)))
+	if (int rc = grow(&k.line.blob, k.line.blob_cap, o_eb + (size_t)L.nunit * (64 / cc::kLineRedCells) * sizeof(double)))
 		return rc;
-	if (int rc = up.upload(b)) {
-		cudaFree(b);
+	if (int rc = up.upload(k.line.blob))
 		return rc;
-	}
-	k.line.blob = b;
+	unsigned char *b = k.line.blob;
 	k.line.rows = reinterpret_cast<cc::LineRow *>(b + o_rows);
 	k.line.lines = reinterpret_cast<cc::LineIdx *>(b + o_lines);
 	k.line.cells = reinterpret_cast<cc::LineCell *>(b + o_cells);
 	k.line.cellV = reinterpret_cast<double2 *>(b + o_cellV);
 	k.line.phases = reinterpret_cast<cc::LineTabs *>(b + o_phases);
+	k.line.groups.clear();
 	for (const Offsets &o : og)
 		k.line.groups.push_back({reinterpret_cast<cc::LineTabs *>(b + o.groups), reinterpret_cast<cc::LineTask *>(b + o.tasks),
 		                         reinterpret_cast<cc::LineIdx *>(b + o.tlines)});
 	k.line.eblock = reinterpret_cast<double *>(b + o_eb);
+	k.line.ready = true;
 	return CC_OK;
 }
 
@@ -707,20 +725,6 @@ inline bool wrap_unit(double x, double *out)
 	return true;
 }
 
-int ensure_partial(double2 **partial, size_t &cap, size_t elems)
-{
-	if (elems <= cap)
-		return CC_OK;
-	cudaFree(*partial);
-	*partial = nullptr;
-	cap = 0;
-	int rc = dev_alloc(partial, elems);
-	if (rc)
-		return rc;
-	cap = elems;
-	return CC_OK;
-}
-
 int ensure_partialG(cc_handle *h, size_t elems)
 {
 	if (elems <= h->partialG_cap)
@@ -756,9 +760,9 @@ int run_rho(cc_handle *h, DevKSet &k, int64_t N, const double *d_frac, double *d
 		if (int rc = ensure_lines(k))
 			return rc;
 		if (!lane) {
-			if (int rc = ensure_partial(&k.line.partial, k.line.partial_cap, (size_t)nsplit * L.nunit * 128))
+			if (int rc = grow(&k.line.partial, k.line.partial_cap, (size_t)nsplit * L.nunit * 128))
 				return rc;
-			if (!k.line.weights)
+			if (&k == &h->main && !k.line.weights)   // (S(k) has no force pass)
 				if (int rc = dev_alloc(&k.line.weights, (size_t)L.nunit * 256))
 					return rc;
 		}
@@ -793,7 +797,7 @@ int run_rho(cc_handle *h, DevKSet &k, int64_t N, const double *d_frac, double *d
 		r.cellV = k.line.cellV;
 		r.rho_offset = h->rho_offset;
 		r.rho_slot = rho_out ? rho_out : lane ? lane->rho_slot : k.rho_slot;
-		r.weights = rho_out ? nullptr : lane ? lane->weights : k.line.weights;
+		r.weights = rho_out || &k != &h->main ? nullptr : lane ? lane->weights : k.line.weights;
 		r.eblock = lane ? lane->eblock : k.line.eblock;
 		r.ticket = lane ? lane->ticket : k.ticket;
 		r.inv_vol = 1.0 / h->volume;
@@ -818,7 +822,7 @@ int run_rho(cc_handle *h, DevKSet &k, int64_t N, const double *d_frac, double *d
 	const int nsplit = N > 0 ? l.nsplit : 1;
 	const int csize = N > 0 ? l.csize : 1;
 	const int rows = nsplit / csize;
-	if (int rc = ensure_partial(&k.partial, k.partial_cap, (size_t)rows * p.nslot))
+	if (int rc = grow(&k.partial, k.partial_cap, (size_t)rows * p.nslot))
 		return rc;
 	cc::RhoArgs a = {};
 	a.frac = d_frac;
@@ -957,20 +961,6 @@ int run_force(cc_handle *h, int64_t N, const double *d_frac, double *d_F, double
 		a.fscale = fscale_in;
 	}
 	return launch_force(h->d, a, mixed, N, f->host.max_row, st);
-}
-
-// Grow a device buffer to n elements (contents not kept).
-template <class T> int grow(T **p, size_t &cap, size_t n)
-{
-	if (n <= cap)
-		return CC_OK;
-	cudaFree(*p);
-	*p = nullptr;
-	cap = 0;
-	if (int rc = dev_alloc(p, n))
-		return rc;
-	cap = n;
-	return CC_OK;
 }
 
 // ---------------------------------------------------------------------------------------------------------------
@@ -1276,8 +1266,7 @@ int create_common(int d, const double *basis, int64_t M, const int32_t *modes, c
 		delete h;
 		return fail(CC_ERR_CUDA, std::string("cudaStreamCreate: ") + cudaGetErrorString(e));
 	}
-	cc::Plan plan = cc::build_plan(d, M, modes, V, 8);
-	if ((rc = upload_kset(h->main, plan)) || (rc = dev_alloc(&h->d_E, 2))) {
+	if ((rc = upload_kset(h->main, cc::build_plan(d, M, modes, V, 8))) || (rc = dev_alloc(&h->d_E, 2))) {
 		cc_destroy(h);
 		return rc;
 	}
@@ -2197,9 +2186,9 @@ int cc_structure_factor(cc_handle *h, int64_t K, const int32_t *modes, double *S
 	}
 	if (h->sk.segs == nullptr || (size_t)(K * h->d) != h->sk_modes.size() ||
 	    std::memcmp(modes, h->sk_modes.data(), sizeof(int32_t) * K * h->d) != 0) {
-		std::vector<double> ones((size_t)K, 1.0);
-		cc::Plan plan = cc::build_plan(h->d, K, modes, ones.data(), 8);
-		if (int rc = upload_kset(h->sk, plan))
+		const std::vector<double> ones((size_t)K, 1.0);
+		CC_CUDA(cudaStreamSynchronize(h->stream));   // an earlier call that failed may still read the set
+		if (int rc = upload_kset(h->sk, cc::build_plan(h->d, K, modes, ones.data(), 8)))
 			return rc;
 		h->sk_modes.assign(modes, modes + K * h->d);
 	}

@@ -50,7 +50,9 @@ struct Launch {
 
 // A line plan (cc_plan.h) on the device, from the set's first use on the line kernels on (ensure_lines).
 struct DevLines {
+	bool ready = false;
 	unsigned char *blob = nullptr;  // one allocation for the arrays below down to eblock, but for the weights
+	size_t blob_cap = 0;
 	const cc::LineRow *rows = nullptr;
 	const cc::LineIdx *lines = nullptr;
 	const cc::LineCell *cells = nullptr;
@@ -75,6 +77,7 @@ struct DevKSet {
 	cc::LinePlan lplan;
 	DevLines line;
 	unsigned char *blob = nullptr;  // one allocation for the plan's arrays, ticket and eblock
+	size_t blob_cap = 0;
 	cc::Seg *segs = nullptr;
 	int *bstart = nullptr;
 	cc::TabSpec *bspec = nullptr;
@@ -83,6 +86,7 @@ struct DevKSet {
 	double2 *rho_slot = nullptr;
 	double2 *u_slot = nullptr;
 	double2 *rho_mode = nullptr;
+	size_t rho_cap = 0, mode_cap = 0;   // double2 elements of rho_slot (with u_slot) and of rho_mode
 	double *eblock = nullptr;       // one per reduce block
 	unsigned *ticket = nullptr;
 	double2 *partial = nullptr;     // partial rows * nslot
@@ -104,11 +108,16 @@ struct DevKSet {
 		cudaFree(line.weights);
 		cudaFree(line.partial);
 		cudaFree(partial);
+		drop_splits();
+		*this = DevKSet();
+	}
+	void drop_splits()
+	{
 		for (DevSplits &f : splits) {
 			cudaFree(f.kstart);
 			cudaFree(f.kspec);
 		}
-		*this = DevKSet();
+		splits.clear();
 	}
 };
 
@@ -151,8 +160,9 @@ template <class T> int upload_into(T *p, const std::vector<T> &v, cudaStream_t s
 }
 
 
-// Upload a plan into a device k-set (releases what it held).
-int upload_kset(DevKSet &k, const cc::Plan &plan);
+// Upload a plan into a device k-set, in the place of the one that it held: nothing may still read that one. The buffers stay
+// where the new plan fits them.
+int upload_kset(DevKSet &k, cc::Plan &&plan);
 
 // The arrays of the set's line plan (lplan.ok) on the device.
 int ensure_lines(DevKSet &k);
