@@ -126,6 +126,7 @@ struct cc_batch {
 	int *d_shape = nullptr;                  // 3 x B
 	// instances with a line plan: their FP64 descriptors (set 0 / 1), and the two item counts of every instance
 	bool any_line = false, all_line = false;
+	std::vector<char> line;                  // by instance: FP64 on the line kernels
 	cc::LineRhoArgs *d_lrho[2] = {nullptr, nullptr};
 	cc::LineReduceArgs *d_lred[2] = {nullptr, nullptr};
 	cc::LineForceArgs *d_lforce[2] = {nullptr, nullptr};
@@ -262,7 +263,7 @@ int batch_build(cc_batch *b, int per_split, int segs_per_split)
 		cc::LineForceArgs lf = {};
 		for (int ph = 0; ph < 3; ph++)
 			own[ph * B + k] = c[ph];
-		if (h->main.lplan.ok) {
+		if (b->line[i]) {
 			const cc::LinePlan &L = h->main.lplan;
 			const DevLines &dl = h->main.line;
 			lr.frac = ra.frac;
@@ -338,7 +339,7 @@ int batch_build(cc_batch *b, int per_split, int segs_per_split)
 	for (int k = 0; k < B; k++) {
 		const cc_handle *h = b->h[b->order[k]];
 		const cc::LinePlan &L = h->main.lplan;
-		if (!L.ok)
+		if (!b->line[b->order[k]])
 			continue;
 		const size_t two = cc::line_force_smem(L.phase_row, cc::kLineBatchMT, 8, h->d, 2);
 		if (teams && L.phases.size() == 1 && two <= kBatchLineSmem) {
@@ -523,6 +524,7 @@ int cc_batch_create(int count, cc_handle *const *handles, const int64_t *N, cc_b
 	b->off_F.resize(count);
 	b->off_E.resize(count);
 	b->bufs.resize(count);
+	b->line.assign(count, 0);
 	for (int i = 0; i < count; i++)
 		b->off_frac[i] = b->arena.take(sizeof(double) * N[i] * handles[i]->d);
 	b->pos_bytes = b->arena.used - b->off_frac[0];
@@ -551,13 +553,14 @@ int cc_batch_create(int count, cc_handle *const *handles, const int64_t *N, cc_b
 		const int max_nsplit = (int)((n + kTuneSplits[0] - 1) / kTuneSplits[0]);
 		const int nchunks = (p.nslot + 31) / 32, pgroups = (int)((n + 31) / 32);
 		const cc::LinePlan &L = h->main.lplan;
-		if (L.ok)
+		b->line[i] = uses_lines(h->main, n);   // (a rule on the instance alone)
+		if (b->line[i])
 			if (int rc = ensure_lines(h->main)) {
 				delete b;
 				return rc;
 			}
-		const size_t row = std::max((size_t)p.nslot, L.ok ? (size_t)L.nunit * 128 : 0);   // entries of a partial row
-		b->any_line |= L.ok;
+		const size_t row = std::max((size_t)p.nslot, b->line[i] ? (size_t)L.nunit * 128 : 0);   // entries of a partial row
+		b->any_line |= b->line[i] != 0;
 		q.o_part = b->arena.take(sizeof(double2) * (size_t)max_nsplit * row);
 		q.o_rho = b->arena.take(sizeof(double2) * p.nslot);
 		q.o_u = b->arena.take(sizeof(double2) * p.nslot);
@@ -569,7 +572,7 @@ int cc_batch_create(int count, cc_handle *const *handles, const int64_t *N, cc_b
 	}
 	b->all_line = true;
 	for (int i = 0; i < count; i++)
-		b->all_line &= handles[i]->main.lplan.ok;
+		b->all_line &= b->line[i] != 0;
 	int rc;
 	if ((rc = dev_alloc(&b->arena.base, b->arena.used))) {
 		cc_batch_destroy(b);

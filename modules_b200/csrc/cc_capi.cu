@@ -255,86 +255,26 @@ double grid_cost(int64_t blocks, int wave, double pairs, double fixed_pairs)
 	return (double)waves * (1.0 + pairs / (double)blocks / fixed_pairs);
 }
 
-// The line kernels' grids.
-// rho: the grouping and the particle splits (multiples of 8 particles) with the least estimated time: whole waves of blocks,
-// each with a fixed cost and its FP64 cycles at a rate, plus a cost per partial row (the reduction). The constants are a fit
-// to 490 timings of evaluations on B200 (2D and 3D, N = 300 to 100000, every grouping, 8 to 1024 particles per split);
-// what it picks is within 8 % of the best of them, mostly the best. Two blocks of 8 warps share an SM at 1846 cycles per us
-// (of 1965), one alone reaches 1124, a block of 12 or 16 warps 1726: 3D N=2000 chi=0.45 takes 13.3 us with 3 groups of 4
-// tasks and 24 particles a split, 13.7 with 2 of 8, 14.0 with one of 12; 2D N=1e5 1.95 ms with groups of 8, 2.03 of 16; 2D
-// N=7001 26.7 with one wave of wide blocks, 28.4 with groups of 8.
-// force: tiles of 8 particles per block and warps per block, by whole waves of what one wave measured (3D, 67 units: 9.4,
-// 15.2, 20.6 and 28.7 us for 1 to 4 tiles with 8 warps, two blocks to an SM; 9.0, 11.8 and 16.8 for 2 to 4 tiles with 16).
-constexpr double kLineFixedUs = 1.5, kLineRowUs = 0.012;
-
-Launch choose_line_launch(const cc::LinePlan &p, int d, int64_t N)
-{
-	Launch l = {};
-	l.line = true;
-	l.csize = 1;
-	l.nsplit = 1;
-	l.per_split = 8;
-	const int sms = sm_count();
-	double best = 1e300;
-	for (size_t gi = 0; gi < p.groupings.size(); gi++) {
-		const cc::LineGroups &g = p.groupings[gi];
-		const int64_t G = std::max<int64_t>(1, (int64_t)g.count());
-		const bool two = g.ntask <= cc::kLineTasks;
-		const int64_t wave = (two ? 2 : 1) * (int64_t)sms, maxns = std::max<int64_t>(1, std::min<int64_t>((N + 7) / 8, cc::kLineMaxSplits));
-		for (int64_t ns = 1; ns <= maxns; ns++) {
-			const int64_t per = std::max<int64_t>(8, ((N + ns - 1) / ns + 7) / 8 * 8),
-			              real = std::max<int64_t>(1, (N + per - 1) / per);
-			const int64_t full = G * real / wave, rest = G * real - full * wave;
-			const double cyc = (double)per * g.cycles;
-			const double full_us = two ? 0.55 + 2.0 * cyc / 1846.0 : 0.28 + cyc / 1726.0;
-			const double last_us = rest == 0 ? 0.0 : two && rest <= sms ? 0.72 + cyc / 1124.0 : full_us;
-			const double c = (double)full * full_us + last_us + (double)real * kLineRowUs;
-			if (c < best) {
-				best = c;
-				l.grouping = (int)gi;
-				l.nsplit = (int)real;
-				l.per_split = (int)per;
-			}
-			if (G * real > 8LL * sms)
-				break;
-		}
-	}
-	// chunks: a power of two that holds a split, or as many particles as fit (and have a thread per coordinate)
-	const cc::LineGroups &g = p.groupings[l.grouping];
-	const size_t row = (size_t)g.row * sizeof(double2);
-	const size_t room = (g.ntask <= cc::kLineTasks ? 100 : 204) * 1024;
-	const int most = std::min(cc::kLineMaxChunk, g.ntask * 32 / d);
-	l.chunk = 8;
-	while (l.chunk < l.per_split && 2 * l.chunk <= most && 2 * l.chunk * row <= room)
-		l.chunk *= 2;
-	// force
-	best = 1e300;
-	static const struct {
-		int mt, warps;
-		double unit_us;   // per unit and wave
-	} opt[] = {{1, 8, 0.117}, {2, 8, 0.205}, {3, 8, 0.285}, {4, 8, 0.406}, {2, 16, 0.112}, {3, 16, 0.154}, {4, 16, 0.228}};
-	l.mt = 1;
-	l.fwarps = 8;
-	for (const auto &o : opt) {
-		const double waves = (double)((N + 8 * o.mt - 1) / (8 * o.mt)) / ((o.warps == 8 ? 2.0 : 1.0) * sms);
-		// few waves: whole ones; many: the blocks of a new wave start as those of the last one end
-		const double c = (waves < 4.0 ? std::ceil(waves) : waves + 0.5) * (kLineFixedUs + o.unit_us * p.nunit);
-		if (c < best) {
-			best = c;
-			l.mt = o.mt;
-			l.fwarps = o.warps;
-		}
-	}
-	return l;
-}
-
-// FP64 evaluations take the line kernels where the k-set has a line plan; mixed precision and the other sets (1D, sparse
-// lines) the segment kernels.
+// FP64 evaluations take the line kernels where the k-set has a line plan that is estimated faster; mixed precision and the
+// other sets (1D, sparse lines, few particles with very many modes) the segment kernels.
 Launch find_launch(const DevKSet &k, int64_t N, bool mixed)
 {
 	const cc::Plan &p = k.plan;
-	if (!mixed && k.lplan.ok && N <= cc::kLineMaxParticles)
-		return choose_line_launch(k.lplan, p.d, N);
+	if (!mixed && k.lplan.ok && N <= cc::kLineMaxParticles) {
+		const cc::LineLaunch g = cc::line_launch(k.lplan, p.d, N, sm_count());
+		if (cc::lines_preferred(p, k.lplan, g, N, !k.rho_only)) {
+			Launch l = {};
+			l.line = true;
+			l.csize = 1;
+			l.nsplit = g.nsplit;
+			l.per_split = g.per_split;
+			l.chunk = g.chunk;
+			l.grouping = g.grouping;
+			l.mt = g.mt;
+			l.fwarps = g.fwarps;
+			return l;
+		}
+	}
 	Launch l = {};
 	const size_t esz = mixed ? sizeof(float2) : sizeof(double2);
 	l.chunk = (int)std::max<size_t>(8, std::min<size_t>(64, kRhoTabBudget / (esz * std::max(1, p.block_max_row | 1))));
@@ -398,6 +338,12 @@ Launch choose_launch(DevKSet &k, int64_t N, bool mixed)
 	k.chosen.push_back({N, mixed, find_launch(k, N, mixed)});
 	return k.chosen.back().l;
 }
+
+}  // namespace
+
+bool cci::uses_lines(DevKSet &k, int64_t N) { return choose_launch(k, N, false).line; }
+
+namespace {
 
 // ---------------------------------------------------------------------------------------------------------------
 // kernel dispatch
@@ -1270,6 +1216,7 @@ int create_common(int d, const double *basis, int64_t M, const int32_t *modes, c
 		cc_destroy(h);
 		return rc;
 	}
+	h->sk.rho_only = true;
 	*out = h;
 	return CC_OK;
 }
@@ -1320,7 +1267,7 @@ bool nufft_preferred(cc_handle *h, int64_t N, bool mixed)
 	const double direct = (double)N * (double)h->main.plan.real_segs * h->main.plan.L / 7e11;
 	const double nufft = 3.9e-12 * (double)N * w + 7.2e-12 * grid * (1 + d) + 8e-5;
 	const cc::LinePlan &L = h->main.lplan;
-	if (1.2 * nufft >= direct || mixed || !L.ok)
+	if (1.2 * nufft >= direct || mixed || !uses_lines(h->main, N))
 		return 1.2 * nufft < direct;
 	const double n = (double)N;
 	const double direct_us = 8.8 + 59e-6 * n * L.nunit + (d == 3 ? 39e-6 * n * (double)L.rows.size() : 0.0) + 2.8e-4 * n;

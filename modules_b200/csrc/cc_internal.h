@@ -97,6 +97,7 @@ struct DevKSet {
 		bool mixed;
 		Launch l;
 	};
+	bool rho_only = false;          // no force pass follows its rho passes (S(k))
 	std::vector<Chosen> chosen;   // launch configurations of the last few particle counts
 
 	void release()
@@ -169,6 +170,9 @@ int ensure_lines(DevKSet &k);
 
 // The device splits of the force pass into about `want` segment ranges (uploaded on first use, kept by the k-set).
 int get_splits(DevKSet &k, int want, const DevSplits **out);
+
+// Whether FP64 evaluations of N particles take the line kernels.
+bool uses_lines(DevKSet &k, int64_t N);
 
 // What the line kernels of one evaluation write, for evaluations of one handle that run at the same time: a lane of
 // cc_energy_grad_many (lane 0 uses the k-set's own buffers).

@@ -573,6 +573,103 @@ LinePlan build_line_plan(const Plan &p)
 	return L;
 }
 
+// The line kernels' grids.
+// rho: the grouping and the particle splits (multiples of 8 particles) with the least estimated time: whole waves of blocks,
+// each with a fixed cost and its FP64 cycles at a rate, plus a cost per partial row (the reduction). The constants are a fit
+// to 490 timings of evaluations on B200 (2D and 3D, N = 300 to 100000, every grouping, 8 to 1024 particles per split);
+// what it picks is within 8 % of the best of them, mostly the best. Two blocks of 8 warps share an SM at 1846 cycles per us
+// (of 1965), one alone reaches 1124, a block of 12 or 16 warps 1726: 3D N=2000 chi=0.45 takes 13.3 us with 3 groups of 4
+// tasks and 24 particles a split, 13.7 with 2 of 8, 14.0 with one of 12; 2D N=1e5 1.95 ms with groups of 8, 2.03 of 16; 2D
+// N=7001 26.7 with one wave of wide blocks, 28.4 with groups of 8.
+// force: tiles of 8 particles per block and warps per block, by whole waves of what one wave measured (3D, 67 units: 9.4,
+// 15.2, 20.6 and 28.7 us for 1 to 4 tiles with 8 warps, two blocks to an SM; 9.0, 11.8 and 16.8 for 2 to 4 tiles with 16).
+constexpr double kLineFixedUs = 1.5, kLineRowUs = 0.012;
+
+LineLaunch line_launch(const LinePlan &p, int d, int64_t N, int sms)
+{
+	LineLaunch l;
+	l.nsplit = 1;
+	l.per_split = 8;
+	double best = 1e300;
+	for (size_t gi = 0; gi < p.groupings.size(); gi++) {
+		const LineGroups &g = p.groupings[gi];
+		const int64_t G = std::max<int64_t>(1, (int64_t)g.count());
+		const bool two = g.ntask <= kLineTasks;
+		const int64_t wave = (two ? 2 : 1) * (int64_t)sms, maxns = std::max<int64_t>(1, std::min<int64_t>((N + 7) / 8, kLineMaxSplits));
+		for (int64_t ns = 1; ns <= maxns; ns++) {
+			const int64_t per = std::max<int64_t>(8, ((N + ns - 1) / ns + 7) / 8 * 8),
+			              real = std::max<int64_t>(1, (N + per - 1) / per);
+			const int64_t full = G * real / wave, rest = G * real - full * wave;
+			const double cyc = (double)per * g.cycles;
+			const double full_us = two ? 0.55 + 2.0 * cyc / 1846.0 : 0.28 + cyc / 1726.0;
+			const double last_us = rest == 0 ? 0.0 : two && rest <= sms ? 0.72 + cyc / 1124.0 : full_us;
+			const double c = (double)full * full_us + last_us + (double)real * kLineRowUs;
+			if (c < best) {
+				best = c;
+				l.grouping = (int)gi;
+				l.nsplit = (int)real;
+				l.per_split = (int)per;
+			}
+			if (G * real > 8LL * sms)
+				break;
+		}
+	}
+	l.rho_us = best;
+	// chunks: a power of two that holds a split, or as many particles as fit (and have a thread per coordinate)
+	const LineGroups &g = p.groupings[l.grouping];
+	const size_t row = (size_t)g.row * 2 * sizeof(double);
+	const size_t room = (g.ntask <= kLineTasks ? 100 : 204) * 1024;
+	const int most = std::min(kLineMaxChunk, g.ntask * 32 / d);
+	l.chunk = 8;
+	while (l.chunk < l.per_split && 2 * l.chunk <= most && 2 * l.chunk * row <= room)
+		l.chunk *= 2;
+	// force
+	best = 1e300;
+	static const struct {
+		int mt, warps;
+		double unit_us;   // per unit and wave
+	} opt[] = {{1, 8, 0.117}, {2, 8, 0.205}, {3, 8, 0.285}, {4, 8, 0.406}, {2, 16, 0.112}, {3, 16, 0.154}, {4, 16, 0.228}};
+	l.mt = 1;
+	l.fwarps = 8;
+	for (const auto &o : opt) {
+		const double waves = (double)((N + 8 * o.mt - 1) / (8 * o.mt)) / ((o.warps == 8 ? 2.0 : 1.0) * sms);
+		// few waves: whole ones; many: the blocks of a new wave start as those of the last one end
+		const double whole = waves < 4.0 ? std::ceil(waves) : waves + 0.5;
+		const double c = whole * (kLineFixedUs + o.unit_us * p.nunit);
+		if (c < best) {
+			best = c;
+			l.waves = whole;
+			l.mt = o.mt;
+			l.fwarps = o.warps;
+		}
+	}
+	l.force_us = best;
+	return l;
+}
+
+// Segment or line kernels for N particles. The line kernels do fewer operations per particle and mode, but a block takes all of
+// a set's units (forces) or a share of them (rho) one after another, however few particles there are; the segment kernels
+// split the modes over the SMs too. Both estimates, in us, are fits to 1500 evaluations of sets with a line plan on B200 (lines of
+// 41 to 2001 modes, discs and balls of radius 8 to 250, shells, triangles, boxes of density 0.1 to 1, 2D and 3D, N = 1 to
+// 40000); the choice is within 5 % of the faster one in 97 % of them, and at most 33 % off. Measured, segments against lines: 2D
+// disc of radius 250 (98000 modes) N=100 41 / 108 us, N=1000 147 / 125; 3D ball of radius 30 (57000) N=100 32 / 67, N=1000
+// 105 / 79; 16 lines of 2001 N=100 28 / 62, N=1000 120 / 68; 2D disc of radius 60 N=100 19 / 12; stealthy sets of chi < 0.5 take
+// lines at every N. Without forces: disc of 250, N=100, 26 / 40.
+bool lines_preferred(const Plan &p, const LinePlan &L, const LineLaunch &g, int64_t N, bool forces)
+{
+	const double n = (double)N, segs = (double)std::min<int64_t>(p.real_segs, 2000);
+	const double pairs = n * p.nslot, tables = n * p.nbgroups() * p.block_max_row;
+	if (!forces) {
+		const double seg = 7.76 + 0.58e-6 * pairs + 4.69e-6 * tables + 2.47e-3 * segs + 0.21e-3 * n;
+		return 4.64 + 1.1 * g.rho_us + 0.0476 * L.nunit <= seg;
+	}
+	const double seg = 12.2 + 1.147e-6 * pairs + 8.12e-6 * tables + 7.27e-3 * segs + (N < 64 ? 3.6 : 0.0) + 0.097e-3 * n;
+	const double rows = (p.d == 3 ? 0.19 : 0.026) * (double)L.rows.size();
+	const double line = 4.32 + 1.108 * g.rho_us + 0.879 * g.force_us + g.waves * (2.12 * ((double)L.phases.size() - 1.0) + rows) +
+	                    0.116e-3 * n;
+	return line <= 1.05 * seg;
+}
+
 bool cell_geometry(int d, const double *a, double *volume, double *recip)
 {
 	double inv[9] = {0};

@@ -146,6 +146,19 @@ struct LinePlan {
 // the segment kernels, and for sets whose tables do not fit.
 LinePlan build_line_plan(const Plan &p);
 
+// The line kernels' grids for N particles on `sms` SMs.
+struct LineLaunch {
+	int grouping = 0;                   // of the plan
+	int nsplit = 1, per_split = 8, chunk = 8;   // rho: particle splits, particles each, particles staged at once
+	int mt = 1, fwarps = 8;             // force: tiles of 8 particles per block, warps per block
+	double rho_us = 0.0, force_us = 0.0;   // their estimated times
+	double waves = 1.0;                 // of force blocks
+};
+LineLaunch line_launch(const LinePlan &p, int d, int64_t N, int sms);
+
+// Whether the line kernels are estimated faster than the segment kernels, for energies and forces or (forces false) rho alone.
+bool lines_preferred(const Plan &p, const LinePlan &L, const LineLaunch &g, int64_t N, bool forces);
+
 // |det| of the basis (rows a_i) and the reciprocal basis rows b_e with b_e . a_i = 2 pi delta_ei.
 bool cell_geometry(int d, const double *basis, double *volume, double *recip);
 
