@@ -55,6 +55,7 @@ int batch_line_chunk(const cc::LineGroups &g, int per_split)
 constexpr int kTuneSplits[] = {32, 64, 128, 256, 512, 1024};
 constexpr int kTuneSegs[] = {32, 64, 128, 256, 512, 1024};
 
+constexpr int kApartWaves = 8;   // cc_batch_minimize: launches of their own for the instances of either stage
 constexpr size_t kBatchLineSmem = 104 * 1024;   // line items: two blocks to an SM
 
 // dynamic shared memory the fused kernel is allowed (its largest table rows in FP64, any dimension)
@@ -132,6 +133,7 @@ struct cc_batch {
 	cc::LineForceArgs *d_lforce[2] = {nullptr, nullptr};
 	int *d_own = nullptr;                    // 6 x B
 	size_t line_smem = 0;
+	std::vector<int> seg_force;              // segment force items of every instance (launch order)
 	std::vector<cc::LineRhoArgs> lrho;       // host copies of set 0
 	std::vector<cc::LineReduceArgs> lred;
 	std::vector<cc::LineForceArgs> lforce;
@@ -379,6 +381,7 @@ int batch_build(cc_batch *b, int per_split, int segs_per_split)
 	    (rc = upload_into(b->d_lforce[0], b->lforce, st)) || (rc = upload_into(b->d_own, own, st)))
 		return rc;
 	CC_CUDA(cudaStreamSynchronize(st));   // evaluations may run on a caller's stream
+	b->seg_force.assign(own.begin() + 2 * B, own.begin() + 3 * B);
 	b->per_split = per_split;
 	b->segs_per_split = segs_per_split;
 	return CC_OK;
@@ -893,10 +896,29 @@ int cc_batch_minimize(cc_batch *b, double *const *frac, const cc_lbfgs_opts *opt
 	CC_CUDA(cudaGetLastError());
 	// A block of iterations is enqueued kernel by kernel: an iteration keeps the GPU busy for far longer (40 us and more)
 	// than its four launches take, and capturing a graph of them on every call cost 2 ms. Schedule: each instance at its
-	// stage's precision while some instance is in the mixed stage; then FP64 only.
+	// stage's precision while some instance is in the mixed stage; then FP64 only. The launch that holds both precisions has
+	// the registers of the line items, two blocks to an SM, and mixed items run at two thirds of the speed of the mixed
+	// launch's three: while the running instances' mixed force items fill more than kApartWaves times that, the instances of
+	// either stage have a launch of their own (the other ones' items are skipped, which costs some 25 us; the same items, so the
+	// results are the same). 64 uneven instances, 100 steps in the mixed stage 66 -> 54 ms; with 2 instead of 8, 32 of N <= 1000
+	// to their ground states 93 -> 97.
+	bool apart = false;
+	auto choose_apart = [&](const std::vector<cc::LbBrief> *hs) {
+		int64_t mixed = 0;
+		for (int k = 0; k < count; k++)
+			if (!hs || ((*hs)[k].status == cc::kLbRunning && (*hs)[k].stage == 0))
+				mixed += b->seg_force[k];
+		apart = sched && b->any_line && mixed > (int64_t)kApartWaves * 2 * sm_count();
+	};
+	choose_apart(nullptr);
 	auto iterations = [&](int prec, int count_it) -> int {
 		for (int it = 0; it < count_it; it++) {
-			if (int r2 = batch_eval(b, 1, prec, st))
+			if (prec == CC_PREC_SCHEDULE && apart) {
+				if (int r2 = batch_eval(b, 1, CC_PREC_MIXED, st))
+					return r2;
+				if (int r2 = batch_eval(b, 1, CC_PREC_FP64, st))
+					return r2;
+			} else if (int r2 = batch_eval(b, 1, prec, st))
 				return r2;
 			CC_CUDA(cc::lb_step(b->d_lb, count, nblk, maxn, st, count == 1 ? &lbo[0] : nullptr));
 		}
@@ -943,6 +965,7 @@ int cc_batch_minimize(cc_batch *b, double *const *frac, const cc_lbfgs_opts *opt
 			break;
 		if (sched && stage == 0 && !any_mixed)
 			stage = 1;
+		choose_apart(&hs);
 	}
 	// results: positions wrapped into [0,1) become the bound ones, FP64 energies of the results (one batched evaluation)
 	cc::lb_finish_kernel<<<all, 256, 0, st>>>(b->d_lb, b->d_final);
