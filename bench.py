@@ -15,8 +15,8 @@ forces evaluation of one configuration. Synthetic seeded inputs (no dataset exis
           configuration (the reference's interface), each waiting for its result.
   roofline: the dominant kernel's algorithmic FLOPs (FP64, the line kernels: 12 per particle-k pair and evaluation, 4 in
           the rho kernel, 8 in the force kernel; mixed, the segment kernels: 17 + 2d, 8 and 9 + 2d) / its CUDA-event
-          duration, against the FP64 FMA peak measured in the same run by an FMA-chain probe kernel
-          (MEASURED_PEAKS.json has no FP64 figure).
+          duration, against the FP64 peak measured in the same run by probe kernels (chains of matrix instructions,
+          which the line kernels run on, and of FMAs: the higher; MEASURED_PEAKS.json has no FP64 figure).
   cpu_baseline: the reference's own ShiftedCCPotential (Energy + AllForce, oracle/_ref) on the host cores.
 
 --impl reference times that reference CPU path alone on the same workload and prints its line.
@@ -667,7 +667,7 @@ def run_ours(args):
                 "gpu_launches": launches_per_eval * K * P,
                 "roofline": {"bound": "fp64_fma" if prec == cc.PREC_FP64 else "fp32_fma", "kernel": dom,
                              "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
-                             "peak_source": "measured in this run: FMA-chain probe kernel (cc_probe_fma_peak); "
+                             "peak_source": "measured in this run: FMA and FP64 matrix chains (cc_probe_fma_peak); "
                                             "MEASURED_PEAKS.json has no FP64 figure",
                              "flops_per_launch": fl, "launch_ms": tk, "traffic": NCU_TRAFFIC_BYTES.get(dom),
                              "traffic_unit": "DRAM bytes per launch (ncu capture, cold caches; warm: ~256 B)",

@@ -377,8 +377,9 @@ int cc_get_timing(cc_handle *h, double *rho_ms, double *reduce_ms, double *force
  * splits, the segment length L and the number of segments (for reports). */
 int cc_plan_info(const cc_handle *h, int64_t N, int *L, int64_t *nseg, int *nsplit, int *nksplit);
 
-/* Measure the device's FMA throughput (TFLOP/s, 2 flops per FMA) of independent FMA chains in FP64
- * (precision = CC_PREC_FP64) or FP32 (CC_PREC_MIXED), timed with CUDA events: the roofline peak of this path. */
+/* Measure the device's multiply-add throughput (TFLOP/s, 2 flops each) of independent chains, timed with CUDA events: the
+ * roofline peak of this path. CC_PREC_FP64: the higher one of FP64 FMAs and of FP64 matrix instructions, which share a pipe
+ * (34 and 37 TFLOP/s on B200); CC_PREC_MIXED: FP32 FMAs. */
 int cc_probe_fma_peak(int precision, double *tflops);
 
 #ifdef __cplusplus

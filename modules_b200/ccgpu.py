@@ -271,7 +271,7 @@ class CCMulti:
 
 
 def probe_fma_peak(precision=PREC_FP64):
-    """Measured FMA throughput of the device in TFLOP/s (FP64 or FP32 chains)."""
+    """Measured multiply-add throughput of the device in TFLOP/s (FP64: FMAs or matrix instructions, the higher; else FP32)."""
     t = _d()
     _check(load_library().cc_probe_fma_peak(precision, ctypes.byref(t)))
     return t.value

@@ -1506,19 +1506,37 @@ template <typename T> __global__ void fma_probe_kernel(T *out, int iters, T a, T
 		out[0] = s;
 }
 
-template <typename T> int probe_peak(double *tflops)
+// The same of FP64 matrix instructions: four independent chains of 2048 flops a step and warp.
+__global__ void dmma_probe_kernel(double *out, int iters, double a, double b)
 {
-	T *out = nullptr;
-	if (int rc = dev_alloc(&out, 1))
-		return rc;
-	const int blocks = sm_count() * 8, threads = 256, iters = 1 << 14;
+	double2 c[8];
+#pragma unroll
+	for (int k = 0; k < 8; k++)
+		c[k] = make_double2((double)(threadIdx.x + k) * 1e-3, (double)k);
+	for (int i = 0; i < iters; i++) {
+#pragma unroll
+		for (int k = 0; k < 8; k += 2)
+			cc::dmma16(c[k], c[k + 1], a, b, a, b, a, b);
+	}
+	double s = 0;
+#pragma unroll
+	for (int k = 0; k < 8; k++)
+		s += c[k].x + c[k].y;
+	if (s == -1.2345)
+		out[0] = s;
+}
+
+// Best of five timings of `launch` (after one that is not timed), which does `flops`.
+template <class F> int probe_peak(double flops, double *tflops, F launch)
+{
 	cudaEvent_t a, b;
 	CC_CUDA(cudaEventCreate(&a));
 	CC_CUDA(cudaEventCreate(&b));
 	float best = 1e30f;
 	for (int rep = 0; rep < 6; rep++) {
 		CC_CUDA(cudaEventRecord(a));
-		fma_probe_kernel<T><<<blocks, threads>>>(out, iters, (T)0.9999999, (T)1e-7);
+		launch();
+		CC_CUDA(cudaGetLastError());
 		CC_CUDA(cudaEventRecord(b));
 		CC_CUDA(cudaEventSynchronize(b));
 		float ms = 0;
@@ -1528,9 +1546,34 @@ template <typename T> int probe_peak(double *tflops)
 	}
 	cudaEventDestroy(a);
 	cudaEventDestroy(b);
-	cudaFree(out);
-	*tflops = 2.0 * 8.0 * iters * (double)blocks * threads / (best * 1e-3) / 1e12;
+	*tflops = flops / (best * 1e-3) / 1e12;
 	return CC_OK;
+}
+
+template <typename T> int probe_fma(double *tflops)
+{
+	T *out = nullptr;
+	if (int rc = dev_alloc(&out, 1))
+		return rc;
+	const int blocks = sm_count() * 8, threads = 256, iters = 1 << 14;
+	const int rc = probe_peak(2.0 * 8.0 * iters * (double)blocks * threads, tflops, [&] {
+		fma_probe_kernel<T><<<blocks, threads>>>(out, iters, (T)0.9999999, (T)1e-7);
+	});
+	cudaFree(out);
+	return rc;
+}
+
+int probe_dmma(double *tflops)
+{
+	double *out = nullptr;
+	if (int rc = dev_alloc(&out, 1))
+		return rc;
+	const int blocks = sm_count() * 8, threads = 256, iters = 1 << 12;
+	const int rc = probe_peak(4.0 * 2048.0 * iters * (double)blocks * (threads / 32), tflops, [&] {
+		dmma_probe_kernel<<<blocks, threads>>>(out, iters, 1e-3, 1e-7);
+	});
+	cudaFree(out);
+	return rc;
 }
 
 }  // namespace
@@ -2377,7 +2420,15 @@ int cc_probe_fma_peak(int precision, double *tflops)
 		return fail(CC_ERR_ARG, "tflops is null");
 	if (int rc = device_ok())
 		return rc;
-	return precision == CC_PREC_FP64 ? probe_peak<double>(tflops) : probe_peak<float>(tflops);
+	if (precision != CC_PREC_FP64)
+		return probe_fma<float>(tflops);
+	double fma = 0.0, mma = 0.0;
+	if (int rc = probe_fma<double>(&fma))
+		return rc;
+	if (int rc = probe_dmma(&mma))
+		return rc;
+	*tflops = std::max(fma, mma);
+	return CC_OK;
 }
 
 }  // extern "C"
