@@ -48,8 +48,11 @@ enum {
 };
 
 enum {
-	CC_PREC_FP64 = 0,   /* FP64 seeds, FP64 recurrences, FP64 sums */
-	CC_PREC_MIXED = 1   /* FP64 argument reduction, FP32 seeds and recurrences, FP64 tile partials and sums */
+	CC_PREC_FP64 = 0,   /* FP64 throughout. The faster choice for most sets: its sums run on the FP64 matrix unit */
+	CC_PREC_MIXED = 1   /* FP64 argument reduction, FP32 seeds and recurrences, FP64 tile partials and sums. Faster than FP64
+	                       only for sets of few modes per lattice line, which have no matrix form (3D N=3001, 3000 scattered
+	                       modes: 107 against 159 us an evaluation), and for few particles with very many modes; elsewhere up
+	                       to 2.5 times as slow (3D N=3001, M=2724: 27 against 16 us; 2D N=1e5, M=40002: 3.5 against 1.9 ms) */
 };
 
 typedef struct cc_handle cc_handle;
@@ -118,7 +121,9 @@ int cc_rho(cc_handle *h, double *re, double *im, int precision);
 /* Force on particle i of the bound positions (d doubles), from the last cc_energy_grad. */
 int cc_force_one(cc_handle *h, int64_t i, double *f);
 
-/* S(k) = |rho(k)|^2 / N of the bound positions at K integer modes (K x d), host output S (K). */
+/* S(k) = |rho(k)|^2 / N of the bound positions at K integer modes (K x d), host output S (K). The handle keeps the plan of the
+ * last list: a call with the same list evaluates at once (2D N=1e5, K=40002: 0.8 ms), one with a new list plans it first
+ * (2.3 ms), the first one also allocates (3 to 5 ms). */
 int cc_structure_factor(cc_handle *h, int64_t K, const int32_t *modes, double *S, int precision);
 
 /* The structure optimiser's Switch-0 objective: x = rescale * fractional coordinates (N*d), returns the energy in
@@ -135,7 +140,8 @@ int cc_objective(cc_handle *h, int64_t N, const double *x, double rescale, doubl
  * gradient, the m correction pairs and every dot product stay on the device (FP64). The method is L-BFGS in the compact
  * representation (Byrd, Nocedal & Schnabel 1994) with Armijo backtracking; iterates are not NLopt's bit for bit. */
 enum {
-	CC_PREC_SCHEDULE = 2        /* cc_minimize: mixed precision until E/N <= switch_energy_per_particle, then FP64 */
+	CC_PREC_SCHEDULE = 2        /* mixed precision until E/N <= switch_energy_per_particle, then FP64: for callers whose sets
+	                               are faster in mixed precision; elsewhere plain FP64 is (3D N=2000: 18 against 32 ms) */
 };
 #define CC_STOPVAL_GROUND_STATE (-1.0)
 typedef struct {
@@ -146,7 +152,7 @@ typedef struct {
 	double ftol;                /* stop after 3 accepted steps with E decreasing by <= ftol |E|, default 1e-15 */
 	int precision;              /* CC_PREC_FP64 (default), CC_PREC_MIXED or CC_PREC_SCHEDULE */
 	double switch_energy_per_particle;   /* CC_PREC_SCHEDULE threshold, default 1e-12 */
-	int iters_per_check;        /* iterations per host status check (one CUDA graph replay), default 32 */
+	int iters_per_check;        /* iterations per host status check, default 32 */
 } cc_lbfgs_opts;
 
 typedef struct {
@@ -177,7 +183,7 @@ int cc_batch_set_positions(cc_batch *b, const double *const *frac);
 int cc_batch_energy_grad(cc_batch *b, double *E, double *const *F, int precision);
 /* The same, enqueued on `stream` with results left on the device (no host synchronisation). */
 int cc_batch_eval_device(cc_batch *b, int precision, void *stream);
-/* Minimise every instance from its bound positions; frac[i] (host) receives the results, results[i] the outcomes. */
+/* Minimise every instance from frac[i] (host), which receives the result; results[i] (may be NULL) the outcomes. */
 int cc_batch_minimize(cc_batch *b, double *const *frac, const cc_lbfgs_opts *opts, cc_lbfgs_result *results);
 /* Autotuner of the batch's tile shapes: times `reps` FP64 evaluations of the bound positions for every candidate
  * (particles per rho block 32 / 64 / 128 / 256 / 512 / 1024 x segments per force block 32 / 64 / 128 / 256 / 512 /
