@@ -1,7 +1,7 @@
 // cc_batch.cu — batches of independent configurations (cc_batch_* in include/cc_gpu.h).
 //
 // A batch evaluates many configurations of uneven size and dimension together: ONE launch of the fused batch kernel
-// (cc_lbatch_kernel, cc_lines.cuh; cc_mbatch_kernel, cc_kernels.cuh, where no instance has a line plan) per energy + gradient step, whose work queue holds the rho blocks, split-reduction
+// (cc_lbatch_kernel, cc_lines.cuh; cc_mbatch_kernel, cc_kernels.cuh, where no instance takes the line kernels) per energy + gradient step, whose work queue holds the rho blocks, split-reduction
 // chunks and force blocks of every instance; per-instance completion counts order the three phases of an instance.
 // Its batched L-BFGS (cc_batch_minimize) keeps every instance's positions, gradient and history on the device and
 // enqueues blocks of iterations (one fused evaluation and the L-BFGS kernels each). The reference
@@ -125,7 +125,7 @@ struct cc_batch {
 	int *d_pre = nullptr;                    // 3 queues (one per mode) of 4 x (B + 1): rho, reduce, force, reduce +
 	                                         // force items per instance
 	int *d_shape = nullptr;                  // 3 x B
-	// instances with a line plan: their FP64 descriptors (set 0 / 1), and the two item counts of every instance
+	// instances on the line kernels (uses_lines): their FP64 descriptors (set 0 / 1), and the two item counts of every instance
 	bool any_line = false, all_line = false;
 	std::vector<char> line;                  // by instance: FP64 on the line kernels
 	cc::LineRhoArgs *d_lrho[2] = {nullptr, nullptr};
@@ -356,7 +356,7 @@ int batch_build(cc_batch *b, int per_split, int segs_per_split)
 		b->lforce[k].tiles = per_item;
 		own[5 * B + k] = (own[5 * B + k] + per_item - 1) / per_item;
 	}
-	// the queue of each mode: 0 line items where there is a line plan, 1 segment items, 2 (an instance's stage decides) the
+	// the queue of each mode: 0 line items for instances on the line kernels, 1 segment items, 2 (an instance's stage decides) the
 	// larger of the two counts
 	for (int mode = 0; mode < 3; mode++) {
 		int *q = pre.data() + (size_t)mode * 4 * (B + 1);
@@ -400,7 +400,7 @@ int batch_eval(cc_batch *b, int set, int precision, cudaStream_t st)
 		a.lred = b->d_lred[set];
 		a.lforce = b->d_lforce[set];
 		a.own = b->d_own;
-		// segment items need their own shared memory: mixed ones, and those of instances without a line plan
+		// segment items need their own shared memory: mixed ones, and those of the other instances
 		size_t smem = mode == 1 ? 0 : b->line_smem;
 		if (mode != 0 || !b->all_line)
 			smem = std::max(smem, std::max(rho_smem<double2>(b->rho_row, kBatchChunk, 8),
@@ -670,7 +670,7 @@ int cc_batch_autotune(cc_batch *b, int reps, int *per_split, int *segs_per_split
 				}
 			}
 	} else {
-		// FP64 evaluations of instances with a line plan do not read the segment tile: the particles per rho block are chosen
+		// FP64 evaluations of instances on the line kernels do not read the segment tile: the particles per rho block are chosen
 		// by FP64, the segments then by FP64 (the other instances) and mixed evaluations (every instance) together
 		for (int ps : kTuneSplits) {
 			if (rc || (rc = batch_build(b, ps, bs)) || (rc = timed(CC_PREC_FP64, &ms)))

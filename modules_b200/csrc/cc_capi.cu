@@ -3,7 +3,7 @@
 // A handle holds the constraint set of one ShiftedCCPotential (potential/CollectiveCoordinatePotential.h:84-117)
 // planned into lattice-line segments (see cc_kernels.cuh) and lines (see cc_lines.cuh), the cell (volume, reciprocal
 // basis) and the device buffers of the bound positions. One evaluation is three kernel launches on the handle's stream
-// (cc_line_* in FP64, cc_* in mixed precision and for sets without a line plan):
+// (cc_line_* in FP64, cc_* in mixed precision and where the line kernels are not to be had or not the faster ones):
 //   rho, reduce -> rho per slot, the force weights, the energy (and rho in mode order on request);
 //   force       -> Cartesian forces and/or the gradient in fractional coordinates.
 // There is no CPU path: without a CUDA device every call that computes returns CC_ERR_NOGPU.

@@ -1,5 +1,6 @@
 // cc_kernels.cuh — sm_100a kernels of the collective-coordinate (CC) potential: the segment kernels, which evaluate mixed
-// precision and the constraint sets that have no line plan (FP64 otherwise runs on cc_lines.cuh), and the Monte Carlo move.
+// precision, the constraint sets that have no line plan and few particles with very many modes (FP64 otherwise runs on
+// cc_lines.cuh), and the Monte Carlo move.
 //
 // Work decomposition. The constraint modes n (integer k-lattice indices) are grouped on the host into SEGMENTS of
 // L = 8 modes that share every index but the last and whose last index runs start, start+1, ... (a piece of a lattice

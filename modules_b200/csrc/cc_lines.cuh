@@ -865,7 +865,7 @@ __global__ void __launch_bounds__(32 * W, W == 8 ? 2 : 1) cc_line_force_kernel(L
 // fused batch evaluation with line plans
 // ---------------------------------------------------------------------------------------------------------------
 // The launch of cc_mbatch_kernel (one work queue, phases ordered by completion counts) for batches in which some instance
-// has a line plan: such an instance's FP64 items are line items, its mixed items (and every item of the other instances)
+// takes the line kernels: such an instance's FP64 items are line items, its mixed items (and every item of the other instances)
 // segment items. An instance's phase holds the larger of its two item counts, so that the queue does not depend on the
 // stages; the surplus items do nothing and are counted.
 struct LBatchArgs {
@@ -873,7 +873,7 @@ struct LBatchArgs {
 	const LineRhoArgs *lrho;
 	const LineReduceArgs *lred;
 	const LineForceArgs *lforce;
-	const int *own;       // 6 x B: segment items of the three phases, line items (0: no line plan)
+	const int *own;       // 6 x B: segment items of the three phases, line items (0: on the segment kernels)
 };
 
 union LineItemDesc {
