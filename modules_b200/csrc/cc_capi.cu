@@ -594,8 +594,11 @@ int ensure_particles(cc_handle *h, int64_t N)
 		h->d_pin = nullptr;
 		g_alloc_gen++;
 		cudaError_t e = cudaHostAlloc(reinterpret_cast<void **>(&h->h_pin), pin * sizeof(double), cudaHostAllocMapped);
-		if (e != cudaSuccess)
+		if (e != cudaSuccess) {
+			cudaGetLastError();   // (not for the next launch's check)
+			h->h_pin = nullptr;
 			return fail(CC_ERR_OOM, std::string("cudaHostAlloc: ") + cudaGetErrorString(e));
+		}
 		e = cudaHostGetDevicePointer(reinterpret_cast<void **>(&h->d_pin), h->h_pin, 0);
 		if (e != cudaSuccess)
 			return fail(CC_ERR_CUDA, std::string("cudaHostGetDevicePointer: ") + cudaGetErrorString(e));
@@ -621,8 +624,11 @@ int input_staging(cc_handle *h, size_t n)
 		h->d_in = nullptr;
 		h->in_cap = 0;
 		cudaError_t e = cudaHostAlloc(reinterpret_cast<void **>(&h->h_in), n * sizeof(double), cudaHostAllocMapped);
-		if (e != cudaSuccess)
+		if (e != cudaSuccess) {
+			cudaGetLastError();   // (not for the next launch's check)
+			h->h_in = nullptr;
 			return fail(CC_ERR_OOM, std::string("cudaHostAlloc: ") + cudaGetErrorString(e));
+		}
 		e = cudaHostGetDevicePointer(reinterpret_cast<void **>(&h->d_in), h->h_in, 0);
 		if (e != cudaSuccess) {
 			cudaFreeHost(h->h_in);

@@ -133,9 +133,11 @@ template <class T> int dev_alloc(T **p, size_t n)
 	if (n == 0)
 		n = 1;
 	cudaError_t e = cudaMalloc(reinterpret_cast<void **>(p), n * sizeof(T));
-	if (e != cudaSuccess)
+	if (e != cudaSuccess) {
+		cudaGetLastError();   // (not for the next launch's check)
 		return fail(e == cudaErrorMemoryAllocation ? CC_ERR_OOM : CC_ERR_CUDA,
 		            std::string("cudaMalloc: ") + cudaGetErrorString(e));
+	}
 	return CC_OK;
 }
 

@@ -131,8 +131,11 @@ template <class T> int grow_dev(T **p, size_t &cap, size_t n)
 	*p = nullptr;
 	cap = 0;
 	cudaError_t e = cudaMalloc(reinterpret_cast<void **>(p), n * sizeof(T));
-	if (e != cudaSuccess)
+	if (e != cudaSuccess) {
+		cudaGetLastError();   // (not for the next launch's check)
+		*p = nullptr;
 		return cc::set_error(CC_ERR_OOM, (std::string("cudaMalloc: ") + cudaGetErrorString(e)).c_str());
+	}
 	cap = n;
 	return CC_OK;
 }
