@@ -2269,8 +2269,15 @@ int cc_mc_try_move(cc_handle *h, const double *s_prev, const double *s_after, do
 		return CC_OK;
 	}
 	const int nb = (M + cc::kMcThreads - 1) / cc::kMcThreads;
-	if (!h->d_modes) {
+	if (!h->d_mc_part) {   // the last one of these to be allocated: a call that ran out of memory starts over
 		int rc;
+		cudaFree(h->d_modes);
+		cudaFree(h->d_modeV);
+		cudaFree(h->d_rho_trial);
+		cudaFree(h->d_rho_cur);
+		h->d_modes = nullptr;
+		h->d_modeV = nullptr;
+		h->d_rho_trial = h->d_rho_cur = nullptr;
 		if ((rc = upload(&h->d_modes, h->modes)) || (rc = upload(&h->d_modeV, h->V)) ||
 		    (rc = dev_alloc(&h->d_rho_trial, M)) || (rc = dev_alloc(&h->d_rho_cur, M)) ||
 		    (rc = dev_alloc(&h->d_mc_part, nb + 1)))

@@ -39,14 +39,12 @@ def test_mixed_stage_costs_what_mixed_costs(gpu):
     starts = [rng.random((2000, 3)) for _ in range(count)]
     kw = dict(max_evals=64, stopval=-1e300, ftol=0.0, switch_energy_per_particle=-1.0)
 
-    def ms(precision):
-        best = np.inf
-        for _ in range(4):
+    times = {gpu.PREC_MIXED: [], gpu.PREC_SCHEDULE: []}
+    for _ in range(6):
+        for precision, taken in times.items():
             t = time.perf_counter()
             batch.minimize(starts, precision=precision, **kw)
-            best = min(best, time.perf_counter() - t)
-        return best * 1e3
-
-    mixed, schedule = ms(gpu.PREC_MIXED), ms(gpu.PREC_SCHEDULE)
+            taken.append((time.perf_counter() - t) * 1e3)
+    mixed, schedule = (min(taken) for taken in times.values())
     print(f"mixed {mixed:.2f} ms, schedule {schedule:.2f} ms")
     assert schedule <= 1.25 * mixed
