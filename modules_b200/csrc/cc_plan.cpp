@@ -651,7 +651,7 @@ LineLaunch line_launch(const LinePlan &p, int d, int64_t N, int sms)
 // a set's units (forces) or a share of them (rho) one after another, however few particles there are; the segment kernels
 // split the modes over the SMs too. Both estimates, in us, are fits to 1500 evaluations of sets with a line plan on B200 (lines of
 // 41 to 2001 modes, discs and balls of radius 8 to 250, shells, triangles, boxes of density 0.1 to 1, 2D and 3D, N = 1 to
-// 40000); the choice is within 5 % of the faster one in 97 % of them, and at most 33 % off. Measured, segments against lines: 2D
+// 40000); the choice is within 5 % of the faster one in 96 % of them, and at most a third off. Measured, segments against lines: 2D
 // disc of radius 250 (98000 modes) N=100 41 / 108 us, N=1000 147 / 125; 3D ball of radius 30 (57000) N=100 32 / 67, N=1000
 // 105 / 79; 16 lines of 2001 N=100 28 / 62, N=1000 120 / 68; 2D disc of radius 60 N=100 19 / 12; stealthy sets of chi < 0.5 take
 // lines at every N. Without forces: disc of 250, N=100, 26 / 40.
